@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/d2conv3d.h"
 
 namespace d2c {
@@ -301,6 +303,36 @@ void count_launch();
 void prof_mark(cudaStream_t st, const char* name);
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+
+// Raises a kernel's dynamic shared-memory limit, once per kernel, device and size: the attribute call costs about as
+// much host time as a launch, and a small layer makes a dozen launches per pass.
+template <auto kKernel>
+inline int allow_dynamic_smem(int bytes) {
+  static std::atomic<int> allowed[64];
+  int dev = -1;
+  D2C_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev >= 0 && dev < 64 && allowed[dev].load(std::memory_order_relaxed) >= bytes) return D2C_OK;
+  D2C_CUDA_TRY(cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  if (dev >= 0 && dev < 64) allowed[dev].store(bytes, std::memory_order_relaxed);
+  return D2C_OK;
+}
+
+// A buffer of 4-byte words that a staging kernel clears on the side, for a later kernel that accumulates into it (one
+// launch less than a memset of its own).  `block` of `blocks` clears its share.
+struct ZeroFill {
+  void* ptr;
+  long long bytes;
+};
+__device__ __forceinline__ void zero_fill(const ZeroFill& z, long long block, long long blocks) {
+  const long long first = block * blockDim.x + threadIdx.x, step = blocks * blockDim.x;
+  if (((reinterpret_cast<uintptr_t>(z.ptr) | (uintptr_t)z.bytes) & 15u) == 0) {
+    uint4* p = reinterpret_cast<uint4*>(z.ptr);
+    for (long long i = first; i < (z.bytes >> 4); i += step) p[i] = make_uint4(0u, 0u, 0u, 0u);
+  } else {
+    uint32_t* p = reinterpret_cast<uint32_t*>(z.ptr);
+    for (long long i = first; i < (z.bytes >> 2); i += step) p[i] = 0u;
+  }
+}
 
 // Multiprocessor count of the current device (cached per device).
 int device_sm_count(int* out);

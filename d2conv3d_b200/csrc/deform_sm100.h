@@ -49,8 +49,9 @@ bool sm100_bwd_variant(const Geom& g, int math_mode, unsigned long long cap, boo
 size_t sm100_dw_workspace(const Geom& g, bool x3);
 // grad_bias (nullable, zeroed by the caller) is accumulated by the staging pass over grad_out.
 // sav (nullable): the forward's sample image for this mode; x_cl and recs are not read then.
+// zero_gx: cleared by the staging pass, for the scatter that runs later in the backward.
 int sm100_dw(const Geom& g, bool x3, const float* gy, const void* x_cl, const void* recs, float* grad_w,
-             float* grad_bias, void* ws, cudaStream_t st, const void* sav = nullptr);
+             float* grad_bias, void* ws, cudaStream_t st, const ZeroFill& zero_gx, const void* sav = nullptr);
 
 // `cap` = maximum number of gradient-column elements held at once (clips are processed in chunks).
 bool sm100_bwd_supported(const Geom& g, int dtype, int math_mode, unsigned long long cap);

@@ -489,6 +489,11 @@ dcol_sm100_split_kernel(const DcolParams p) {
   }
 }
 
+// Tap positions per dim of the dilation-field variant, by value (a kernel parameter: no copy to the device).
+struct FieldAxes {
+  float pos[3][kMaxFieldKernelDim];
+};
+
 // ---- (b) sampling gradient + scatter ---------------------------------------------------------------
 
 __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
@@ -509,7 +514,8 @@ __global__ void __launch_bounds__(256, kF32X ? 2 : 3)
 sample_grad_taps_kernel(Geom g, ClStrides cs, int b0, int nh, const float4* __restrict__ recs,
                         const float* __restrict__ dcol, const void* __restrict__ x_cl_v, bool has_mask,
                         float* __restrict__ grad_coord, float* __restrict__ grad_mask, float* __restrict__ gx_cl,
-                        int field_nch, int3 field_ch, const float* __restrict__ field_axes, HeadCfg head) {
+                        int field_nch, int3 field_ch, const __grid_constant__ FieldAxes field_axes, int taps_per_block,
+                        HeadCfg head) {
   const int j = threadIdx.x & 7;
   const int v = blockIdx.x * 32 + (threadIdx.x >> 3);
   const int grp = blockIdx.y % g.G, bl = blockIdx.y / g.G;
@@ -535,13 +541,14 @@ sample_grad_taps_kernel(Geom g, ClStrides cs, int b0, int nh, const float4* __re
     a = __ldg(reinterpret_cast<const float4*>(q));
     b = kNarrow ? zero4 : __ldg(reinterpret_cast<const float4*>(q + 32));
   };
-  float4 rec_n = __ldg(recp);
+  const int tap_beg = blockIdx.z * taps_per_block, tap_end = min(g.K, tap_beg + taps_per_block);
+  float4 rec_n = __ldg(recp + (long long)tap_beg * g.V);
   float4 d0_n, d1_n;
-  ld_cols(dp, d0_n, d1_n);
-  for (int tap = 0; tap < g.K; ++tap) {
+  ld_cols(dp + (long long)tap_beg * nh * slice_stride, d0_n, d1_n);
+  for (int tap = tap_beg; tap < tap_end; ++tap) {
     const float4 rec = rec_n;
     float4 d0 = d0_n, d1 = d1_n;
-    if (tap + 1 < g.K) {
+    if (tap + 1 < tap_end) {
       rec_n = __ldg(recp + (long long)(tap + 1) * g.V);
       ld_cols(dp + (long long)(tap + 1) * nh * slice_stride, d0_n, d1_n);
     }
@@ -643,9 +650,9 @@ sample_grad_taps_kernel(Geom g, ClStrides cs, int b0, int nh, const float4* __re
       } else {
         // the field's gradient sums over taps (and groups): taps are summed here, one atomic per group after
         const int k = tap % g.kw, jj = (tap / g.kw) % g.kh, i = tap / (g.kw * g.kh);
-        fsum[0] += field_axes[i] * (m * wts[0]);
-        fsum[1] += field_axes[kMaxFieldKernelDim + jj] * (m * wts[1]);
-        fsum[2] += field_axes[2 * kMaxFieldKernelDim + k] * (m * wts[2]);
+        fsum[0] += field_axes.pos[0][i] * (m * wts[0]);
+        fsum[1] += field_axes.pos[1][jj] * (m * wts[1]);
+        fsum[2] += field_axes.pos[2][k] * (m * wts[2]);
       }
     }
   }
@@ -696,7 +703,7 @@ struct BwdPlan {
   bool pairg;       // 32 channels per offset group: a 64-channel slice holds two neighbouring groups
   bool split;       // fp32-parity mode with Cout > 256: separate hi / lo operand images, dcol_sm100_split_kernel
   long long gy_lo_off, wt_lo_off;
-  size_t x_cl_bytes, rec_bytes, gat_bytes, gy_img_bytes, wt_img_bytes, dcol_bytes, gx_cl_bytes, axes_bytes;
+  size_t x_cl_bytes, rec_bytes, gat_bytes, gy_img_bytes, wt_img_bytes, dcol_bytes, gx_cl_bytes;
 };
 
 bool make_bwd_plan(const Geom& g, unsigned long long cap, bool x3, BwdPlan* pl) {
@@ -728,7 +735,6 @@ bool make_bwd_plan(const Geom& g, unsigned long long cap, bool x3, BwdPlan* pl) 
   pl->wt_img_bytes = align_up((size_t)pl->wt_lo_off * (pl->split ? 2 : 1), 256);
   pl->dcol_bytes = align_up((size_t)pl->clips_per_chunk * g.V * pl->NT * 4, 256);
   pl->gx_cl_bytes = align_up((size_t)g.B * g.Vin * g.Cin * 4, 256);
-  pl->axes_bytes = 256;
   return true;
 }
 
@@ -747,7 +753,6 @@ int run_bwd(const Geom& g, bool x3, const Coords& coords, unsigned long long cap
   uint8_t* wt_img = wsp; wsp += pl.wt_img_bytes;
   float* dcol = reinterpret_cast<float*>(wsp); wsp += pl.dcol_bytes;
   float* gx_cl = reinterpret_cast<float*>(wsp); wsp += pl.gx_cl_bytes;
-  float* axes_dev = reinterpret_cast<float*>(wsp); wsp += pl.axes_bytes;
   void* dw_ws = wsp;
 
   int sm_count = 0, rc;
@@ -760,15 +765,15 @@ int run_bwd(const Geom& g, bool x3, const Coords& coords, unsigned long long cap
   // dilation-field variant: tap positions per dim, read by the kernel that accumulates grad_size_map
   int field_nch = 0;
   int3 field_ch = make_int3(-1, -1, -1);
+  FieldAxes axes{};
   if constexpr (FieldOut) {
     field_nch = coords.nch;
     field_ch = make_int3(coords.ch[0], coords.ch[1], coords.ch[2]);
-    D2C_CUDA_TRY(cudaMemcpyAsync(axes_dev, &coords.axis[0][0], sizeof(float) * 3 * kMaxFieldKernelDim,
-                                 cudaMemcpyHostToDevice, st));
+    for (int d = 0; d < 3; ++d)
+      for (int i = 0; i < kMaxFieldKernelDim; ++i) axes.pos[d][i] = coords.axis[d][i];
   }
 
   prof_mark(st, "bwd_stage_operands");
-  D2C_CUDA_TRY(cudaMemsetAsync(gx_cl, 0, (size_t)g.B * g.Vin * g.Cin * 4, st));
   if (FieldOut) {
     if (head.geo_bstride)      // the field's gradient channels inside the raw gradient: nch planes per clip
       D2C_CUDA_TRY(cudaMemset2DAsync(grad_coord, sizeof(float) * head.geo_bstride, 0, sizeof(float) * field_nch_of(coords) * g.V,
@@ -791,25 +796,25 @@ int run_bwd(const Geom& g, bool x3, const Coords& coords, unsigned long long cap
   if (!sav) {
     dim3 grid((unsigned)((g.Vin + 31) / 32), (unsigned)((g.Cin + 63) / 64), (unsigned)g.B);
     if (x3)
-      stage_input_cl_f32_kernel<<<grid, 256, 0, st>>>(g.Cin, g.Vin, x, reinterpret_cast<float*>(x_cl));
+      stage_input_cl_f32_kernel<<<grid, 256, 0, st>>>(g.Cin, g.Vin, x, reinterpret_cast<float*>(x_cl), ZeroFill{nullptr, 0});
     else
-      stage_input_cl_f16_kernel<<<grid, 256, 0, st>>>(g.Cin, g.Vin, x, reinterpret_cast<__half*>(x_cl));
+      stage_input_cl_f16_kernel<<<grid, 256, 0, st>>>(g.Cin, g.Vin, x, reinterpret_cast<__half*>(x_cl), ZeroFill{nullptr, 0});
     D2C_LAUNCH_CHECK();
     if (!sav && (rc = launch_sample_records(g, coords, mask, head, recs, gat, st, x3))) return rc;
   }
   // The parameter gradients come first: the weight gradient (tensor-core implicit GEMM over the re-sampled tile)
   // needs only the records and the staged input, and its grad_out staging pass also sums grad_bias.  A caller that
   // reduces them across GPUs can start as soon as `params_ready` fires, under the data-side kernels below.
-  if ((rc = sm100_dw(g, x3, gy, x_cl, gat, grad_w, grad_bias, dw_ws, st, sav))) return rc;
+  if ((rc = sm100_dw(g, x3, gy, x_cl, gat, grad_w, grad_bias, dw_ws, st, ZeroFill{gx_cl, (long long)g.B * g.Vin * g.Cin * 4}, sav))) return rc;
   if (params_ready) D2C_CUDA_TRY(cudaEventRecord(params_ready, st));
   prof_mark(st, "bwd_stage_weights");
   const int img_mode = pl.split ? 2 : (x3 ? 1 : 0);
   stage_wt_img_kernel<<<dim3((unsigned)pl.KBT, (unsigned)g.Cin), 64, 64 * g.K * sizeof(float), st>>>(
       g.Cout, g.Cin, g.K, pl.pairg ? 64 : g.cpg, pl.nh, img_mode, w, wt_img, pl.wt_lo_off);
   D2C_LAUNCH_CHECK();
-  D2C_CUDA_TRY(cudaFuncSetAttribute(dcol_sm100_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem_bytes));
-  D2C_CUDA_TRY(cudaFuncSetAttribute(dcol_sm100_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem_bytes));
-  D2C_CUDA_TRY(cudaFuncSetAttribute(dcol_sm100_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem_bytes));
+  rc = pl.split ? allow_dynamic_smem<dcol_sm100_split_kernel>(pl.smem_bytes)
+                : (x3 ? allow_dynamic_smem<dcol_sm100_kernel<1>>(pl.smem_bytes) : allow_dynamic_smem<dcol_sm100_kernel<0>>(pl.smem_bytes));
+  if (rc) return rc;
 
   for (int b0 = 0; b0 < g.B; b0 += pl.clips_per_chunk) {
     const int nbc = (g.B - b0 < pl.clips_per_chunk) ? g.B - b0 : pl.clips_per_chunk;
@@ -823,7 +828,9 @@ int run_bwd(const Geom& g, bool x3, const Coords& coords, unsigned long long cap
     p.V = g.V; p.NT = pl.NT; p.KB = pl.KB; p.NB = pl.NB;
     p.tiles_per_clip = pl.tiles_per_clip; p.n_tiles = n_tiles; p.n_units = (long long)n_tiles * pl.NB;
     p.tmem_cols = pl.tmem_cols;
-    long long grid = p.n_units / 4;
+    // a unit is 1-3 us of MMAs and stores, the grad_out tile that a CTA loads first less than one: units are spread over
+    // all multiprocessors before any takes a second one
+    long long grid = p.n_units;
     if (grid > sm_count) grid = sm_count;
     if (grid < 1) grid = 1;
     prof_mark(st, "bwd_dcol_sm100");
@@ -837,23 +844,31 @@ int run_bwd(const Geom& g, bool x3, const Coords& coords, unsigned long long cap
       dcol_sm100_kernel<0><<<(unsigned)grid, kDcolThreads, pl.smem_bytes, st>>>(p);
     D2C_LAUNCH_CHECK();
     prof_mark(st, "bwd_sample_grad");
-    dim3 sgrid((unsigned)((g.V + 31) / 32), (unsigned)(nbc * g.G));
+    // A block walks the taps of its 32 voxels one after the other (about 1.7 us per tap while the GPU is not full: two
+    // dependent L2 round trips); small volumes share them out over up to nine blocks so that every multiprocessor has
+    // its two or three blocks.  1024-voxel layer, 27 taps: 46.9 us with one block per 32 voxels, 10.6 us with nine.
+    const long long vblocks = (long long)((g.V + 31) / 32) * nbc * g.G;
+    int tap_split = (int)((3LL * sm_count + vblocks - 1) / vblocks);
+    if (tap_split > 9) tap_split = 9;
+    if (tap_split > g.K) tap_split = g.K;
+    const int taps_per_block = (g.K + tap_split - 1) / tap_split;
+    dim3 sgrid((unsigned)((g.V + 31) / 32), (unsigned)(nbc * g.G), (unsigned)((g.K + taps_per_block - 1) / taps_per_block));
     if (pl.pairg && x3)
       sample_grad_taps_kernel<FieldOut, true, true><<<sgrid, 256, 0, st>>>(g, cs, b0, pl.nh, recs, dcol, x_cl,
                                                                            mask != nullptr, grad_coord, grad_mask,
-                                                                           gx_cl, field_nch, field_ch, axes_dev, head);
+                                                                           gx_cl, field_nch, field_ch, axes, taps_per_block, head);
     else if (pl.pairg)
       sample_grad_taps_kernel<FieldOut, false, true><<<sgrid, 256, 0, st>>>(g, cs, b0, pl.nh, recs, dcol, x_cl,
                                                                             mask != nullptr, grad_coord, grad_mask,
-                                                                            gx_cl, field_nch, field_ch, axes_dev, head);
+                                                                            gx_cl, field_nch, field_ch, axes, taps_per_block, head);
     else if (x3)
       sample_grad_taps_kernel<FieldOut, true><<<sgrid, 256, 0, st>>>(g, cs, b0, pl.nh, recs, dcol, x_cl,
                                                                      mask != nullptr, grad_coord, grad_mask, gx_cl,
-                                                                     field_nch, field_ch, axes_dev, head);
+                                                                     field_nch, field_ch, axes, taps_per_block, head);
     else
       sample_grad_taps_kernel<FieldOut, false><<<sgrid, 256, 0, st>>>(g, cs, b0, pl.nh, recs, dcol, x_cl,
                                                                       mask != nullptr, grad_coord, grad_mask, gx_cl,
-                                                                      field_nch, field_ch, axes_dev, head);
+                                                                      field_nch, field_ch, axes, taps_per_block, head);
     D2C_LAUNCH_CHECK();
   }
   if constexpr (FieldOut) {
@@ -904,7 +919,7 @@ size_t sm100_bwd_workspace(const Geom& g, int dtype, int math_mode, unsigned lon
   BwdPlan pl;
   make_bwd_plan(g, cap, x3, &pl);
   return pl.x_cl_bytes + pl.rec_bytes + pl.gat_bytes + pl.gy_img_bytes + pl.wt_img_bytes + pl.dcol_bytes + pl.gx_cl_bytes +
-         pl.axes_bytes + sm100_dw_workspace(g, x3);
+         sm100_dw_workspace(g, x3);
 }
 
 int sm100_bwd_offsets(const Geom& g, int math_mode, unsigned long long cap, const float* gy, const float* x, const float* offset,

@@ -58,10 +58,12 @@ struct DwParams {
 // lo = bf16(gy - hi), NCH chunks each.
 // grad_bias (nullable) = grad_out summed over clips and voxels (reference dconv3d_gpu.cu:1329): this kernel reads
 // every element of grad_out exactly once, so the 16 threads that share a row add their 128-voxel partial sum with
-// one atomic (grad_bias zeroed before).
+// one atomic (grad_bias zeroed before).  It also clears the two buffers that later kernels of the backward add into.
 __global__ void __launch_bounds__(256)
 stage_gy_kmajor_kernel(int Cout, int V, int tiles_per_clip, int NCH, int x3, const float* __restrict__ gy,
-                       uint8_t* __restrict__ img, float* __restrict__ grad_bias) {
+                       uint8_t* __restrict__ img, float* __restrict__ grad_bias, ZeroFill zero_dws, ZeroFill zero_gx) {
+  zero_fill(zero_dws, blockIdx.x + (long long)gridDim.x * blockIdx.y, (long long)gridDim.x * gridDim.y);
+  zero_fill(zero_gx, blockIdx.x + (long long)gridDim.x * blockIdx.y, (long long)gridDim.x * gridDim.y);
   const int tile = blockIdx.x, coblk = blockIdx.y;        // coblk: 64 rows of co
   const int b = tile / tiles_per_clip, v0 = (tile % tiles_per_clip) * kBM;
   for (int e = threadIdx.x; e < 64 * 16; e += 256) {      // Cout is a multiple of 64: no thread leaves the loop early
@@ -621,9 +623,10 @@ bool make_dw_plan(const Geom& g, int sm_count, bool x3, DwPlan* dp) {
   const int r_stage = ((dp->pairg && !x3) ? 2 : 1) * kRecBytes + 16;
   dp->smem_bytes = kAStages * kAStageBytes + kBStages * dp->b_stage_bytes + kRStages * r_stage + 256 + 1024;
   if (dp->smem_bytes > kSmemLimit) return false;
-  // enough (pair, voxel-range) work items for ~3 waves, but at least 8 tiles per item
+  // enough (pair, voxel-range) work items for ~3 waves, but at least 8 tiles per item -- or, where that would leave
+  // multiprocessors without an item, as many items as there are multiprocessors
   int nsplit = (3 * sm_count + dp->n_pairs - 1) / dp->n_pairs;
-  const int max_split = (dp->n_tiles + 7) / 8;
+  const int max_split = std::max((dp->n_tiles + 7) / 8, std::min(dp->n_tiles, sm_count / dp->n_pairs));
   if (nsplit > max_split) nsplit = max_split;
   if (nsplit < 1) nsplit = 1;
   // The tensor cores add into their fp32 accumulator with truncation (a chain of n accumulating MMAs loses about
@@ -641,12 +644,14 @@ bool make_dw_plan(const Geom& g, int sm_count, bool x3, DwPlan* dp) {
 }
 
 // Work split of the saved-samples kernel: (slice pair, voxel range) items, at least two waves of them, ranges of at
-// least 8 tiles, the smallest count whose last wave is at least 95 % full (else the fullest); the fp32-parity mode ends an
-// accumulation chain after 27 tiles (24 accumulating MMAs per tile and column range -> 648, see make_dw_plan).
+// least 8 tiles (fewer where there would not be an item for every multiprocessor), the smallest count whose last wave is at
+// least 95 % full (else the fullest); the fp32-parity mode ends an accumulation chain after 27 tiles (24 accumulating MMAs
+// per tile and column range -> 648, see make_dw_plan).
 void split_saved(const DwPlan& dp, int sm_count, bool x3, int* tiles_per_split, int* nsplit_out) {
   const int n_pairs = (dp.S + 1) / 2;
   const int chain_min = x3 ? (dp.n_tiles + 26) / 27 : 1;              // fewest ranges the chain cap allows
-  const int size_max = std::max(1, dp.n_tiles / 8);                   // most ranges of at least 8 tiles
+  // most ranges: of at least 8 tiles, or one item per multiprocessor
+  const int size_max = std::max(std::max(1, dp.n_tiles / 8), std::min(dp.n_tiles, sm_count / n_pairs));
   const int lo = std::max(chain_min, std::min(size_max, (2 * sm_count + n_pairs - 1) / n_pairs));
   const int hi = std::max(lo, std::min(size_max, lo + 8));
   int best = lo;
@@ -695,7 +700,7 @@ size_t sm100_dw_workspace(const Geom& g, bool x3) {
 }
 
 int sm100_dw(const Geom& g, bool x3, const float* gy, const void* x_cl, const void* recs, float* grad_w,
-             float* grad_bias, void* ws, cudaStream_t st, const void* sav) {
+             float* grad_bias, void* ws, cudaStream_t st, const ZeroFill& zero_gx, const void* sav) {
   int sm_count = 0;
   {
     const int rc = device_sm_count(&sm_count);
@@ -708,9 +713,9 @@ int sm100_dw(const Geom& g, bool x3, const float* gy, const void* x_cl, const vo
   float* dws = reinterpret_cast<float*>(gyk + dp.gyk_bytes);
 
   prof_mark(st, "bwd_dw_stage");
-  D2C_CUDA_TRY(cudaMemsetAsync(dws, 0, (size_t)dp.S * 64 * g.Cout * 4, st));
   stage_gy_kmajor_kernel<<<dim3((unsigned)dp.n_tiles, (unsigned)((g.Cout + 63) / 64)), 256, 0, st>>>(
-      g.Cout, g.V, dp.tiles_per_clip, dp.NCH, x3 ? 1 : 0, gy, gyk, grad_bias);
+      g.Cout, g.V, dp.tiles_per_clip, dp.NCH, x3 ? 1 : 0, gy, gyk, grad_bias, ZeroFill{dws, (long long)dp.S * 64 * g.Cout * 4},
+      zero_gx);
   D2C_LAUNCH_CHECK();
 
   DwParams p;
@@ -729,14 +734,19 @@ int sm100_dw(const Geom& g, bool x3, const float* gy, const void* x_cl, const vo
     int nsplit = 1;
     split_saved(dp, sm_count, x3, &sp.tiles_per_split, &nsplit);
     prof_mark(st, "bwd_dw_sm100_saved");
+    const int rc = x3 ? allow_dynamic_smem<dw_saved_sm100_kernel<1>>(kSvSmemBytes)
+                      : allow_dynamic_smem<dw_saved_sm100_kernel<0>>(kSvSmemBytes);
+    if (rc) return rc;
     auto kern = x3 ? dw_saved_sm100_kernel<1> : dw_saved_sm100_kernel<0>;
-    D2C_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSvSmemBytes));
     kern<<<sp.n_pairs * nsplit, kSvThreads, kSvSmemBytes, st>>>(sp);
     D2C_LAUNCH_CHECK();
   } else {
     prof_mark(st, "bwd_dw_sm100");
     auto kern = x3 ? dw_sm100_kernel<1, 0> : (dp.pairg ? dw_sm100_kernel<0, 1> : dw_sm100_kernel<0, 0>);
-    D2C_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dp.smem_bytes));
+    const int rc = x3 ? allow_dynamic_smem<dw_sm100_kernel<1, 0>>(dp.smem_bytes)
+                      : (dp.pairg ? allow_dynamic_smem<dw_sm100_kernel<0, 1>>(dp.smem_bytes)
+                                  : allow_dynamic_smem<dw_sm100_kernel<0, 0>>(dp.smem_bytes));
+    if (rc) return rc;
     kern<<<dp.n_pairs * dp.nsplit, kThreads, dp.smem_bytes, st>>>(p);
     D2C_LAUNCH_CHECK();
   }

@@ -59,7 +59,12 @@ constexpr int kRStageBytes = kRecBytes + 16;      // ... + unit header {int64 x_
 constexpr int kRowStride = kGatherWarps * 4;          // 8 threads per row -> rows handled per pass
 constexpr int kRowsPerThread = kBM / kRowStride;
 constexpr int kSmemLimit = 227 * 1024;
-constexpr int kMinUnitsPerCta = 16;
+// Fewest units a CTA is started for.  A unit takes 1.9-2.3 us in its CTA (the producers' gather latency), starting a CTA
+// and adding its partial tile to y about 5 us together: below four units per CTA more CTAs no longer shorten the call.
+// Small layer (432 units): 27 CTAs of 16 units 36.2 us, 108 CTAs of 4 units 17.7 us.
+constexpr int kMinUnitsPerCta = 4;
+// ... and for which the units of a call are cut clip by clip (cta_part_range): every part ends in a partial tile.
+constexpr int kMinUnitsPerPart = 64;
 
 struct FwdParams {
   Geom g;
@@ -223,6 +228,15 @@ bool pick_variant(const Geom& g, int math_mode, bool* x3, Plan* pl) {
   return false;
 }
 
+template <int kX3, int kDual, int kSave>
+int launch_fwd(const FwdParams& p, unsigned grid, int smem_bytes, cudaStream_t st) {
+  const int rc = allow_dynamic_smem<fwd_sm100_kernel<kX3, kDual, kSave>>(smem_bytes);
+  if (rc) return rc;
+  fwd_sm100_kernel<kX3, kDual, kSave><<<grid, kThreadsFwd, smem_bytes, st>>>(p);
+  D2C_LAUNCH_CHECK();
+  return D2C_OK;
+}
+
 template <typename Coords>
 int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& head, const float* x, const float* mask,
             const float* w, const float* bias, float* y, void* ws, cudaStream_t st) {
@@ -268,7 +282,7 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
   // unbalanced.
   const bool rr = grid == sm_count && pl.n_tiles >= 8 * grid;
   const int n_parts = rr ? (int)((pl.n_tiles + grid - 1) / grid)
-                         : ((g.B > 1 && g.B <= 16 && units_per_clip / grid >= 4 * kMinUnitsPerCta) ? g.B : 1);
+                         : ((g.B > 1 && g.B <= 16 && units_per_clip / grid >= kMinUnitsPerPart) ? g.B : 1);
   bool whole_tiles_only = seg_cap >= pl.S && (rr || ((pl.n_tiles % grid == 0) && n_parts == 1));
 
   // CTA pairs (deform_sm100_fwd_pair.cuh) whenever there are at least two tiles and the device can co-schedule
@@ -311,15 +325,16 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
   if (pair_clusters > 0) { sav = nullptr; pos = nullptr; x_cl = ws; }       // the CTA-pair kernel keeps nothing
   prof_mark(st, "fwd_stage_operands");
   {
+    const ZeroFill zero_y{y, whole_tiles_only ? 0 : (long long)sizeof(float) * g.B * g.Cout * g.V};
     dim3 sgrid((unsigned)((g.Vin + 31) / 32), (unsigned)((g.Cin + 63) / 64), (unsigned)g.B);
     if (x3) {
-      stage_input_cl_f32_kernel<<<sgrid, 256, 0, st>>>(g.Cin, g.Vin, x, reinterpret_cast<float*>(x_cl));
+      stage_input_cl_f32_kernel<<<sgrid, 256, 0, st>>>(g.Cin, g.Vin, x, reinterpret_cast<float*>(x_cl), zero_y);
       D2C_LAUNCH_CHECK();
       dim3 wgrid((unsigned)g.Cout, (unsigned)(g.Cin / 32));
       stage_weight_sw128_x3_kernel<<<wgrid, 64, 32 * g.K * sizeof(float), st>>>(g.Cout, g.Cin, g.K, g.cpg, pl.nh, w, w_sw);
       D2C_LAUNCH_CHECK();
     } else {
-      stage_input_cl_f16_kernel<<<sgrid, 256, 0, st>>>(g.Cin, g.Vin, x, reinterpret_cast<__half*>(x_cl));
+      stage_input_cl_f16_kernel<<<sgrid, 256, 0, st>>>(g.Cin, g.Vin, x, reinterpret_cast<__half*>(x_cl), zero_y);
       D2C_LAUNCH_CHECK();
       dim3 wgrid((unsigned)g.Cout, (unsigned)(g.Cin / 64));
       stage_weight_sw128_kernel<<<wgrid, 64, 64 * g.K * sizeof(float), st>>>(g.Cout, g.Cin, g.K,
@@ -327,7 +342,6 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
       D2C_LAUNCH_CHECK();
     }
     if ((rc = launch_sample_records(g, coords, mask, head, pos, recs, st, x3))) return rc;
-    if (!whole_tiles_only) D2C_CUDA_TRY(cudaMemsetAsync(y, 0, sizeof(float) * (size_t)g.B * g.Cout * g.V, st));
   }
 
   FwdParams p;
@@ -368,11 +382,16 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
   }
 #endif
   prof_mark(st, "fwd_sm100_fused");
-  auto kern = sav ? (x3 ? fwd_sm100_kernel<1, 0, 1> : (pl.dual ? fwd_sm100_kernel<0, 1, 1> : fwd_sm100_kernel<0, 0, 1>))
-                  : (x3 ? fwd_sm100_kernel<1, 0, 0> : (pl.dual ? fwd_sm100_kernel<0, 1, 0> : fwd_sm100_kernel<0, 0, 0>));
-  D2C_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem_bytes));
-  kern<<<(unsigned)grid, kThreadsFwd, pl.smem_bytes, st>>>(p);
-  D2C_LAUNCH_CHECK();
+  const int variant = (sav ? 3 : 0) + (x3 ? 0 : (pl.dual ? 1 : 2));
+  switch (variant) {
+    case 0: rc = launch_fwd<1, 0, 0>(p, (unsigned)grid, pl.smem_bytes, st); break;
+    case 1: rc = launch_fwd<0, 1, 0>(p, (unsigned)grid, pl.smem_bytes, st); break;
+    case 2: rc = launch_fwd<0, 0, 0>(p, (unsigned)grid, pl.smem_bytes, st); break;
+    case 3: rc = launch_fwd<1, 0, 1>(p, (unsigned)grid, pl.smem_bytes, st); break;
+    case 4: rc = launch_fwd<0, 1, 1>(p, (unsigned)grid, pl.smem_bytes, st); break;
+    default: rc = launch_fwd<0, 0, 1>(p, (unsigned)grid, pl.smem_bytes, st); break;
+  }
+  if (rc) return rc;
 #ifdef D2C_UNIT_TRACE
   if (p.trace) {
     static long long host[kTraceWords];

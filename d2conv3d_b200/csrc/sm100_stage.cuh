@@ -3,6 +3,7 @@
 
 #include <cuda_fp16.h>
 
+#include "d2c_common.cuh"
 #include "sm100_ptx.cuh"
 
 namespace d2c {
@@ -15,9 +16,12 @@ __device__ __forceinline__ uint32_t pack_f16x2_sat(float lo, float hi) {
   return r;
 }
 
-// x [B][C][Vin] fp32 -> x_cl [B][Vin][C] fp16 (channels-last).  Block: 64 channels x 32 voxels.
+// x [B][C][Vin] fp32 -> x_cl [B][Vin][C] fp16 (channels-last).  Block: 64 channels x 32 voxels.  `zero` is cleared on
+// the side (the output that partial tiles are added to).
 static __global__ void __launch_bounds__(256)
-stage_input_cl_f16_kernel(int C, long long Vin, const float* __restrict__ x, __half* __restrict__ x_cl) {
+stage_input_cl_f16_kernel(int C, long long Vin, const float* __restrict__ x, __half* __restrict__ x_cl, ZeroFill zero) {
+  zero_fill(zero, blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z),
+            (long long)gridDim.x * gridDim.y * gridDim.z);
   __shared__ float tile[64][33];
   const int b = blockIdx.z, c0 = blockIdx.y * 64;
   const long long v0 = (long long)blockIdx.x * 32;
@@ -40,7 +44,9 @@ stage_input_cl_f16_kernel(int C, long long Vin, const float* __restrict__ x, __h
 // replaced by the largest finite float: the gather multiplies stand-in corners by zero weights, which must
 // give zero.
 static __global__ void __launch_bounds__(256)
-stage_input_cl_f32_kernel(int C, long long Vin, const float* __restrict__ x, float* __restrict__ x_cl) {
+stage_input_cl_f32_kernel(int C, long long Vin, const float* __restrict__ x, float* __restrict__ x_cl, ZeroFill zero) {
+  zero_fill(zero, blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z),
+            (long long)gridDim.x * gridDim.y * gridDim.z);
   __shared__ float tile[64][33];
   const int b = blockIdx.z, c0 = blockIdx.y * 64;
   const long long v0 = (long long)blockIdx.x * 32;
