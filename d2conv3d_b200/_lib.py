@@ -1,8 +1,9 @@
-"""ctypes binding of libd2conv3d.so (the C ABI declared in include/d2conv3d.h).
+"""Bindings of libd2conv3d.so (the C ABI declared in include/d2conv3d.h): lib() is the library through ctypes (settings,
+measurements, direct calls), native() the compiled PyTorch front-end over it (csrc/torch_ops.cpp) that the ops run through.
 
-PyTorch is used only for device memory and the current stream: every call passes
+PyTorch is used only for device memory, the current stream and autograd: every call passes
 raw device pointers, sizes and a cudaStream_t across the C boundary.  There is no
-CPU or PyTorch fallback -- if the library is missing or a call fails, an error is
+CPU or PyTorch fallback -- if a library is missing or a call fails, an error is
 raised.
 """
 import ctypes
@@ -118,6 +119,23 @@ def lib():
     return _lib
 
 
+_native = None
+
+
+def native():
+    """The compiled PyTorch front-end; raises if it has not been built."""
+    global _native
+    if _native is None:
+        lib()                    # the same libd2conv3d.so, loaded first
+        try:
+            from . import _C
+        except ImportError as exc:
+            raise RuntimeError("d2conv3d_b200/_C.so is missing or does not load: build it with `python -m "
+                               f"d2conv3d_b200.build` (there is no fallback implementation): {exc}") from exc
+        _native = _C
+    return _native
+
+
 def check(status, what):
     if status == 0:
         return
@@ -164,59 +182,30 @@ def workspace(op, desc, device):
     return ws, n
 
 
-def head_workspace(op, desc, head, field_mode, device):
-    n = lib().d2c_head_workspace_bytes(op, ctypes.byref(desc), ctypes.byref(head), field_mode)
-    if n == 0:
-        return None, 0
-    return torch.empty(n, dtype=torch.uint8, device=device), n
-
-
-_keep_samples = True
-
-
 def set_keep_samples(on):
     """Whether a forward that will be differentiated keeps its blended samples (16-bit, B*Cin*K*V elements) for the
     weight gradient of its backward -- the reference computes them twice.  On by default; switch it off to trade the
     backward's speed for that memory.  Shapes above the intermediate-element cap never keep them."""
-    global _keep_samples
-    _keep_samples = bool(on)
+    native().set_keep_samples(bool(on))
 
 
 def get_keep_samples():
-    return _keep_samples
+    return native().get_keep_samples()
 
 
 class SampleCache:
-    """Buffer + descriptor handed from a forward call to its backward (d2c_sample_cache)."""
+    """Buffer handed from a forward call to its backward (d2c_sample_cache), for the layers with a fused head."""
 
-    def __init__(self, desc, device):
-        n = lib().d2c_sample_cache_bytes(ctypes.byref(desc))
-        self.buf = torch.empty(n, dtype=torch.uint8, device=device) if n else None
-        self.c = SampleCacheStruct(self.buf.data_ptr() if n else None, n, 0, 0)
+    def __init__(self, buf):
+        self.buf = buf
 
     @staticmethod
     def for_forward(desc, device, differentiated):
-        """A bound cache for the forward call that follows, or None (nothing to keep / switched off)."""
-        if not (differentiated and _keep_samples):
+        """The cache of the forward call that follows, or None (nothing to keep / switched off)."""
+        if not (differentiated and get_keep_samples()):
             return None
-        cache = SampleCache(desc, device)
-        if cache.buf is None:
-            return None
-        cache.bind()
-        return cache
-
-    def bind(self):
-        """Applies to the next deformable forward / backward call of this thread."""
-        check(lib().d2c_bind_sample_cache(ctypes.byref(self.c)), "bind_sample_cache")
-
-    @property
-    def kept(self):
-        return self.c.format != 0
-
-
-def finish_forward_cache(cache):
-    """After the forward call: the cache if the kernels filled it, else None (buffer released)."""
-    return cache if cache is not None and cache.kept else None
+        n = lib().d2c_sample_cache_bytes(ctypes.byref(desc))
+        return SampleCache(torch.empty(n, dtype=torch.uint8, device=device)) if n else None
 
 
 def set_math_mode(mode):

@@ -7,7 +7,9 @@ gather rates that bound the sampling kernels) and mma_rate (clocks per tcgen05.m
 on the GPU and are not part of the library.
 
 The library links only the CUDA runtime (statically); it has no dependency on
-torch or Python.  A GPU is not needed to build.
+torch or Python.  _C.so, built beside it, is the PyTorch front-end (csrc/torch_ops.cpp:
+autograd nodes and argument handling over the library's C ABI).  A GPU is not needed
+to build either.
 """
 import os
 import subprocess
@@ -17,6 +19,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB = os.path.join(HERE, "libd2conv3d.so")
+TORCH_SRC = os.path.join(CSRC, "torch_ops.cpp")
+TORCH_LIB = os.path.join(HERE, "_C.so")
 OBJ_DIR = os.path.join(HERE, "build")
 
 SOURCES = ["d2c_api.cu", "depthwise.cu", "deform_sm100_fwd.cu", "deform_sm100_bwd.cu", "deform_sm100_dw.cu",
@@ -34,7 +38,7 @@ def _nvcc():
 def _deps():
     out = [os.path.join(INCLUDE, "d2conv3d.h")]
     for f in os.listdir(CSRC):
-        if os.path.isfile(os.path.join(CSRC, f)):
+        if os.path.isfile(os.path.join(CSRC, f)) and not f.endswith(".cpp"):
             out.append(os.path.join(CSRC, f))
     return out
 
@@ -46,11 +50,45 @@ def needs_build():
     return any(os.path.getmtime(d) > t for d in _deps())
 
 
+def _torch_needs_build():
+    if not os.path.exists(TORCH_LIB):
+        return True
+    t = os.path.getmtime(TORCH_LIB)
+    return any(os.path.getmtime(d) > t for d in (TORCH_SRC, os.path.join(INCLUDE, "d2conv3d.h")))
+
+
+def build_torch(force=False):
+    """The PyTorch front-end _C.so: csrc/torch_ops.cpp against the installed torch, linked to libd2conv3d.so (which it
+    finds beside itself)."""
+    if not force and not _torch_needs_build():
+        return TORCH_LIB
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    inc = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], INCLUDE, "/usr/local/cuda/include"]
+    lib_dir = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_C", "-DTORCH_API_INCLUDE_EXTENSION_H",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+           + [a for i in inc for a in ("-isystem", i)]
+           + [TORCH_SRC, "-o", TORCH_LIB, "-L", lib_dir, "-lc10", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda",
+              "-ltorch_python", "-L", HERE, "-l:libd2conv3d.so", "-L", "/usr/local/cuda/lib64", "-lcudart",
+              "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{lib_dir}"])
+    p = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if p.returncode != 0:
+        sys.stderr.write(p.stdout)
+        raise RuntimeError("building the PyTorch front-end failed")
+    return TORCH_LIB
+
+
 def build(force=False, verbose=False, unit_trace=False):
-    """unit_trace: compile the forward kernel's per-unit timeline instrumentation in (-DD2C_UNIT_TRACE, see
+    """The kernel library, then the PyTorch front-end.
+
+    unit_trace: compile the forward kernel's per-unit timeline instrumentation in (-DD2C_UNIT_TRACE, see
     csrc/deform_sm100_fwd_kernel.cuh and unit_trace.py); always rebuilds.  Build again without it afterwards: the
     instrumented library is for measurements only."""
     if not force and not unit_trace and not needs_build():
+        build_torch()
         return LIB
     os.makedirs(OBJ_DIR, exist_ok=True)
     extra = (["-Xptxas", "-v"] if verbose else []) + (["-DD2C_UNIT_TRACE"] if unit_trace else [])
@@ -71,6 +109,7 @@ def build(force=False, verbose=False, unit_trace=False):
         raise RuntimeError("nvcc failed building libd2conv3d.so")
     cmd = [_nvcc(), "-shared", "-o", LIB] + objs + ["-cudart", "static", "-Xlinker", "-soname=libd2conv3d.so"]
     subprocess.run(cmd, check=True)
+    build_torch(force)
     return LIB
 
 

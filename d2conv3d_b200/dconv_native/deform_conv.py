@@ -9,23 +9,16 @@ import torch
 from torch import nn
 from torch.nn.modules.utils import _single, _triple
 
-from . import _ops
+from .. import _lib
 
 
-def _upcast_if_any_half(tensors):
-    """Reference behaviour (deform_conv.py:15-16,54-59): if any tensor is fp16, every
-    tensor is converted to fp32 and the result stays fp32."""
-    if any(t is not None and t.dtype == torch.half for t in tensors):
-        return [None if t is None else t.float() for t in tensors]
-    return list(tensors)
-
+# If any tensor is fp16, every tensor is converted to fp32 and the result stays fp32 (the last argument of the native
+# calls below); reference behaviour, deform_conv.py:15-16,54-59.
 
 def deform_conv3d(input, offset, alpha, weight, bias=None, stride=(1, 1, 1), padding=(0, 0, 0),
                   dilation=(1, 1, 1), n_weight_groups=1, n_offset_groups=1):
-    input, offset, alpha, weight, bias = _upcast_if_any_half((input, offset, alpha, weight, bias))
-    s, p, d = _triple(stride), _triple(padding), _triple(dilation)
-    return _ops.deform_conv3d(input, offset, alpha, weight, bias, s[0], s[1], s[2], p[0], p[1], p[2],
-                              d[0], d[1], d[2], n_weight_groups, n_offset_groups)
+    return _lib.native().deform_conv3d(input, offset, alpha, weight, bias, _triple(stride), _triple(padding),
+                                       _triple(dilation), n_weight_groups, n_offset_groups, True)
 
 
 def dyn_dilated_conv3d(input, size_map, alpha, weight, bias=None, mode="xyz", stride=(1, 1, 1),
@@ -33,18 +26,17 @@ def dyn_dilated_conv3d(input, size_map, alpha, weight, bias=None, mode="xyz", st
     """deform_conv3d(input, offsets_from_size_map(size_map, mode, k, dilation) repeated per
     offset group, alpha, ...) evaluated without materialising the offsets; also returns the
     gradient w.r.t. size_map directly."""
-    input, size_map, alpha, weight, bias = _upcast_if_any_half((input, size_map, alpha, weight, bias))
-    return _ops.dyn_dilated_conv3d(input, size_map, alpha, weight, bias, mode.lower(), _triple(stride),
-                                   _triple(padding), _triple(dilation), n_weight_groups, n_offset_groups)
+    return _lib.native().dyn_dilated_conv3d(input, size_map, alpha, weight, bias, _lib.FIELD_MODES[mode.lower()],
+                                            _triple(stride), _triple(padding), _triple(dilation), n_weight_groups,
+                                            n_offset_groups, True)
 
 
 def deform_conv1d(input, offset, alpha, weight, bias=None, stride=1, padding=0, dilation=1,
                   n_weight_groups=1, n_offset_groups=1):
     """ops/dconv-native/src/dconv_native/deform_conv.py:19-40: half inputs are up-cast; a missing bias or
     alpha stands for zeros / ones."""
-    input, offset, alpha, weight, bias = _upcast_if_any_half((input, offset, alpha, weight, bias))
-    return _ops.deform_conv1d(input, offset, alpha, weight, bias, stride, padding, dilation,
-                              n_weight_groups, n_offset_groups)
+    return _lib.native().deform_conv1d(input, offset, alpha, weight, bias, _single(stride)[0], _single(padding)[0],
+                                       _single(dilation)[0], n_weight_groups, n_offset_groups, True)
 
 
 class DeformConvNd(nn.Module):
