@@ -24,7 +24,7 @@ TORCH_LIB = os.path.join(HERE, "_C.so")
 OBJ_DIR = os.path.join(HERE, "build")
 
 SOURCES = ["d2c_api.cu", "depthwise.cu", "deform_sm100_fwd.cu", "deform_sm100_bwd.cu", "deform_sm100_dw.cu",
-           "act_norm.cu"]
+           "deform_exact_f32.cu", "deform_exact_f64.cu", "act_norm.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-I", INCLUDE,

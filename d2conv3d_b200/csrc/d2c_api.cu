@@ -1,12 +1,13 @@
 // C ABI of libd2conv3d.so: argument validation, tier selection and launch
 // sequencing.  See include/d2conv3d.h for the contract of every entry point.
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <mutex>
 #include <vector>
 
 #include "d2c_common.cuh"
-#include "deform_generic.cuh"
+#include "deform_exact.h"
 #include "deform_sm100.h"
 
 namespace d2c {
@@ -126,8 +127,6 @@ int depthwise_bwd(const Geom& g, int dtype, const void* gy, const void* x, const
                   void* gw, void* gbias, void* ws, cudaStream_t st);
 size_t depthwise_bwd_workspace(const Geom& g);
 
-static size_t dtype_size(int dtype) { return dtype == D2C_F64 ? 8 : (dtype == D2C_F16 ? 2 : 4); }
-
 // torch.linspace(-dil*(k/2), dil*(k/2), k) as get_kernel_grid of the reference
 // evaluates it (utils/grid.py:21-25): in float32 whatever the field's dtype,
 // ascending from `start` in the first half, descending from `end` in the second.
@@ -180,10 +179,41 @@ static bool ws_ok(const void* ws, size_t have, size_t need) {
   return ws != nullptr && (reinterpret_cast<uintptr_t>(ws) % 256) == 0 && have >= need;
 }
 
-static size_t generic_bwd_workspace(const Geom& g, int dtype, unsigned long long cap) {
-  const int nb = bwd_slice_clips(g, cap);
-  return align_up(dtype_size(dtype) * (size_t)nb * g.Cin * g.K * g.V, 256);
+static size_t exact_fwd_workspace(const Geom& g, int dtype) {
+  return dtype == D2C_F64 ? exact::fwd_workspace<double>(g) : exact::fwd_workspace<float>(g);
 }
+static size_t exact_bwd_workspace(const Geom& g, int dtype, unsigned long long cap) {
+  return dtype == D2C_F64 ? exact::bwd_workspace<double>(g, cap) : exact::bwd_workspace<float>(g, cap);
+}
+
+// ---- integer corner probe -----------------------------------------------------------------------
+template <typename T, typename Coords>
+__global__ void __launch_bounds__(256)
+corners_kernel(Geom g, Coords coords, int32_t* __restrict__ corners) {
+  const long long total = (long long)g.B * g.G * g.K * g.V;
+  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
+       idx += (long long)gridDim.x * blockDim.x) {
+    const int v = (int)(idx % g.V);
+    const int tap = (int)((idx / g.V) % g.K);
+    const int grp = (int)((idx / ((long long)g.V * g.K)) % g.G);
+    const int b = (int)(idx / ((long long)g.V * g.K * g.G));
+    int bz, by, bx;
+    voxel_tap_base(g, v, tap, bz, by, bx);
+    T z, y, xx;
+    coords.get(g, b, grp, tap, v, bz, by, bx, z, y, xx);
+    const Sample<T> s = make_sample(g, z, y, xx);
+    int32_t* o = corners + ((((long long)b * g.G + grp) * g.K + tap) * 3) * g.V + v;
+    o[0] = s.z0; o[g.V] = s.y0; o[2 * (long long)g.V] = s.x0;
+  }
+}
+
+inline unsigned grid_1d(long long total, int block, int max_blocks = 148 * 16) {
+  long long n = (total + block - 1) / block;
+  if (n < 1) n = 1;
+  if (n > max_blocks) n = max_blocks;
+  return (unsigned)n;
+}
+
 
 }  // namespace d2c
 
@@ -229,11 +259,11 @@ size_t d2c_workspace_bytes(int op, const d2c_conv_desc* desc) {
   switch (op) {
     case D2C_OP_DEFORM_FWD:
     case D2C_OP_DYNDIL_FWD:
-      return sm100_fwd_workspace(g, desc->dtype, mode);
+      return std::max(sm100_fwd_workspace(g, desc->dtype, mode), exact_fwd_workspace(g, desc->dtype));
     case D2C_OP_DEFORM_BWD:
     case D2C_OP_DYNDIL_BWD: {
       const size_t fast = sm100_bwd_workspace(g, desc->dtype, mode, cap);
-      const size_t gen = generic_bwd_workspace(g, desc->dtype, cap);
+      const size_t gen = exact_bwd_workspace(g, desc->dtype, cap);
       return fast > gen ? fast : gen;
     }
     case D2C_OP_DEPTHWISE_BWD:
@@ -365,12 +395,14 @@ int d2c_deform_conv3d_fwd(const d2c_conv_desc* desc, const void* x, const void* 
       return sm100_fwd_offsets(g, mode, (const float*)x, (const float*)offset, (const float*)mask,
                                (const float*)w, (const float*)bias, (float*)y, workspace, st);
     }
-    return launch_fwd_generic<float>(g, oc, (const float*)x, (const float*)mask, (const float*)w,
-                                     (const float*)bias, (float*)y, st);
+    if (!ws_ok(workspace, workspace_bytes, exact_fwd_workspace(g, desc->dtype))) return D2C_ERR_WORKSPACE;
+    return exact::launch_fwd<float>(g, oc, (const float*)x, (const float*)mask, (const float*)w,
+                                    (const float*)bias, (float*)y, workspace, st);
   } else if (desc->dtype == D2C_F64) {
     OffsetCoords<double> oc{(const double*)offset};
-    return launch_fwd_generic<double>(g, oc, (const double*)x, (const double*)mask, (const double*)w,
-                                      (const double*)bias, (double*)y, st);
+    if (!ws_ok(workspace, workspace_bytes, exact_fwd_workspace(g, desc->dtype))) return D2C_ERR_WORKSPACE;
+    return exact::launch_fwd<double>(g, oc, (const double*)x, (const double*)mask, (const double*)w,
+                                     (const double*)bias, (double*)y, workspace, st);
   }
   return D2C_ERR_DTYPE;
 }
@@ -407,21 +439,20 @@ int d2c_deform_conv3d_bwd_ev(const d2c_conv_desc* desc, const void* grad_y, cons
                              (float*)grad_mask, (float*)grad_w, (float*)grad_bias, workspace, st,
                              (cudaEvent_t)params_ready);
   }
-  const size_t need = generic_bwd_workspace(g, desc->dtype, cap);
+  const size_t need = exact_bwd_workspace(g, desc->dtype, cap);
   if (!ws_ok(workspace, workspace_bytes, need)) return D2C_ERR_WORKSPACE;
-  const int nb = bwd_slice_clips(g, cap);
   if (desc->dtype == D2C_F32) {
     OffsetCoords<float> oc{(const float*)offset};
-    rc = launch_bwd_generic<float, OffsetCoords<float>, false>(
+    rc = exact::launch_bwd<float, OffsetCoords<float>, false>(
         g, oc, (const float*)grad_y, (const float*)x, (const float*)mask, (const float*)w,
         (float*)grad_x, (float*)grad_offset, 0, (float*)grad_mask, (float*)grad_w, (float*)grad_bias,
-        (float*)workspace, nb, st);
+        workspace, cap, st);
   } else {
     OffsetCoords<double> oc{(const double*)offset};
-    rc = launch_bwd_generic<double, OffsetCoords<double>, false>(
+    rc = exact::launch_bwd<double, OffsetCoords<double>, false>(
         g, oc, (const double*)grad_y, (const double*)x, (const double*)mask, (const double*)w,
         (double*)grad_x, (double*)grad_offset, 0, (double*)grad_mask, (double*)grad_w,
-        (double*)grad_bias, (double*)workspace, nb, st);
+        (double*)grad_bias, workspace, cap, st);
   }
   // the CUDA-core kernels produce the parameter gradients last
   if (rc == D2C_OK && params_ready) D2C_CUDA_TRY(cudaEventRecord((cudaEvent_t)params_ready, st));
@@ -469,12 +500,12 @@ int d2c_deform_conv1d_fwd(const d2c_conv_desc* desc, const void* x, const void* 
   D2C_TAKE_STATUS();
   if (desc->dtype == D2C_F32) {
     Offset1dCoords<float> oc{(const float*)offset};
-    return launch_fwd_generic<float>(g, oc, (const float*)x, (const float*)mask, (const float*)w, (const float*)bias,
-                                     (float*)y, st);
+    return exact::launch_fwd<float>(g, oc, (const float*)x, (const float*)mask, (const float*)w, (const float*)bias,
+                                    (float*)y, nullptr, st);
   } else if (desc->dtype == D2C_F64) {
     Offset1dCoords<double> oc{(const double*)offset};
-    return launch_fwd_generic<double>(g, oc, (const double*)x, (const double*)mask, (const double*)w,
-                                      (const double*)bias, (double*)y, st);
+    return exact::launch_fwd<double>(g, oc, (const double*)x, (const double*)mask, (const double*)w,
+                                     (const double*)bias, (double*)y, nullptr, st);
   }
   return D2C_ERR_DTYPE;
 }
@@ -492,18 +523,17 @@ int d2c_deform_conv1d_bwd(const d2c_conv_desc* desc, const void* grad_y, const v
   cudaStream_t st = (cudaStream_t)stream;
   D2C_TAKE_STATUS();
   const unsigned long long cap = g_max_intermediate.load();
-  if (!ws_ok(workspace, workspace_bytes, generic_bwd_workspace(g, desc->dtype, cap))) return D2C_ERR_WORKSPACE;
-  const int nb = bwd_slice_clips(g, cap);
+  if (!ws_ok(workspace, workspace_bytes, exact_bwd_workspace(g, desc->dtype, cap))) return D2C_ERR_WORKSPACE;
   if (desc->dtype == D2C_F32) {
     Offset1dCoords<float> oc{(const float*)offset};
-    return launch_bwd_generic<float, Offset1dCoords<float>, false>(
+    return exact::launch_bwd<float, Offset1dCoords<float>, false>(
         g, oc, (const float*)grad_y, (const float*)x, (const float*)mask, (const float*)w, (float*)grad_x,
-        (float*)grad_offset, 0, (float*)grad_mask, (float*)grad_w, (float*)grad_bias, (float*)workspace, nb, st);
+        (float*)grad_offset, 0, (float*)grad_mask, (float*)grad_w, (float*)grad_bias, workspace, cap, st);
   }
   Offset1dCoords<double> oc{(const double*)offset};
-  return launch_bwd_generic<double, Offset1dCoords<double>, false>(
+  return exact::launch_bwd<double, Offset1dCoords<double>, false>(
       g, oc, (const double*)grad_y, (const double*)x, (const double*)mask, (const double*)w, (double*)grad_x,
-      (double*)grad_offset, 0, (double*)grad_mask, (double*)grad_w, (double*)grad_bias, (double*)workspace, nb, st);
+      (double*)grad_offset, 0, (double*)grad_mask, (double*)grad_w, (double*)grad_bias, workspace, cap, st);
 }
 
 // ---- dynamic-dilated conv ------------------------------------------------------------------------
@@ -528,13 +558,15 @@ int d2c_dyn_dilated_conv3d_fwd(const d2c_conv_desc* desc, int field_mode, const 
       return sm100_fwd_field(g, mode, fc, (const float*)x, (const float*)mask, (const float*)w,
                              (const float*)bias, (float*)y, workspace, st);
     }
-    return launch_fwd_generic<float>(g, fc, (const float*)x, (const float*)mask, (const float*)w,
-                                     (const float*)bias, (float*)y, st);
+    if (!ws_ok(workspace, workspace_bytes, exact_fwd_workspace(g, desc->dtype))) return D2C_ERR_WORKSPACE;
+    return exact::launch_fwd<float>(g, fc, (const float*)x, (const float*)mask, (const float*)w,
+                                    (const float*)bias, (float*)y, workspace, st);
   } else if (desc->dtype == D2C_F64) {
     FieldCoords<double> fc;
     if ((rc = make_field_coords<double>(g, field_mode, size_map, &fc))) return rc;
-    return launch_fwd_generic<double>(g, fc, (const double*)x, (const double*)mask, (const double*)w,
-                                      (const double*)bias, (double*)y, st);
+    if (!ws_ok(workspace, workspace_bytes, exact_fwd_workspace(g, desc->dtype))) return D2C_ERR_WORKSPACE;
+    return exact::launch_fwd<double>(g, fc, (const double*)x, (const double*)mask, (const double*)w,
+                                     (const double*)bias, (double*)y, workspace, st);
   }
   return D2C_ERR_DTYPE;
 }
@@ -564,9 +596,8 @@ int d2c_dyn_dilated_conv3d_bwd_ev(const d2c_conv_desc* desc, int field_mode, con
   D2C_TAKE_STATUS();
   const unsigned long long cap = g_max_intermediate.load();
   const int mode = g_math_mode.load();
-  const size_t need = generic_bwd_workspace(g, desc->dtype, cap);
+  const size_t need = exact_bwd_workspace(g, desc->dtype, cap);
   if (!ws_ok(workspace, workspace_bytes, need)) return D2C_ERR_WORKSPACE;
-  const int nb = bwd_slice_clips(g, cap);
   const int nch = field_channels(field_mode);
   if (nch < 0) return D2C_ERR_MODE;
   const size_t gs_elems = (size_t)g.B * nch * g.V;
@@ -581,17 +612,17 @@ int d2c_dyn_dilated_conv3d_bwd_ev(const d2c_conv_desc* desc, int field_mode, con
                              (float*)grad_mask, (float*)grad_w, (float*)grad_bias, workspace, st,
                              (cudaEvent_t)params_ready);
     }
-    rc = launch_bwd_generic<float, FieldCoords<float>, true>(
+    rc = exact::launch_bwd<float, FieldCoords<float>, true>(
         g, fc, (const float*)grad_y, (const float*)x, (const float*)mask, (const float*)w,
         (float*)grad_x, (float*)grad_size_map, gs_elems, (float*)grad_mask, (float*)grad_w,
-        (float*)grad_bias, (float*)workspace, nb, st);
+        (float*)grad_bias, workspace, cap, st);
   } else {
     FieldCoords<double> fc;
     if ((rc = make_field_coords<double>(g, field_mode, size_map, &fc))) return rc;
-    rc = launch_bwd_generic<double, FieldCoords<double>, true>(
+    rc = exact::launch_bwd<double, FieldCoords<double>, true>(
         g, fc, (const double*)grad_y, (const double*)x, (const double*)mask, (const double*)w,
         (double*)grad_x, (double*)grad_size_map, gs_elems, (double*)grad_mask, (double*)grad_w,
-        (double*)grad_bias, (double*)workspace, nb, st);
+        (double*)grad_bias, workspace, cap, st);
   }
   if (rc == D2C_OK && params_ready) D2C_CUDA_TRY(cudaEventRecord((cudaEvent_t)params_ready, st));
   return rc;
@@ -698,7 +729,8 @@ int head_fwd_t(const Geom& g, const d2c_head_desc* h, const HeadPlan& hp, int fi
                const T* w, const T* bias, T* y, void* workspace, size_t workspace_bytes, cudaStream_t st) {
   // the CUDA-core route: stage activated dense tensors, then the ordinary kernels
   uint8_t* wsp = reinterpret_cast<uint8_t*>(workspace);
-  if (!ws_ok(workspace, workspace_bytes, hp.geo_bytes + hp.mask_bytes)) return D2C_ERR_WORKSPACE;
+  const size_t stage = hp.geo_bytes + hp.mask_bytes;
+  if (!ws_ok(workspace, workspace_bytes, stage + exact::fwd_workspace<T>(g))) return D2C_ERR_WORKSPACE;
   T* geo = reinterpret_cast<T*>(wsp);
   T* mask = hp.mask_n ? reinterpret_cast<T*>(wsp + hp.geo_bytes) : nullptr;
   head_apply_kernel<T><<<grid_1d((long long)g.B * (hp.geo_n + hp.mask_n) * g.V, 256), 256, 0, st>>>(
@@ -709,10 +741,10 @@ int head_fwd_t(const Geom& g, const d2c_head_desc* h, const HeadPlan& hp, int fi
     FieldCoords<T> fc;
     int rc = make_field_coords<T>(g, field_mode, geo, &fc);
     if (rc) return rc;
-    return launch_fwd_generic<T>(g, fc, x, mask, w, bias, y, st);
+    return exact::launch_fwd<T>(g, fc, x, mask, w, bias, y, wsp + stage, st);
   }
   OffsetCoords<T> oc{geo, 0};
-  return launch_fwd_generic<T>(g, oc, x, mask, w, bias, y, st);
+  return exact::launch_fwd<T>(g, oc, x, mask, w, bias, y, wsp + stage, st);
 }
 
 template <typename T>
@@ -720,28 +752,26 @@ int head_bwd_t(const Geom& g, const d2c_head_desc* h, const HeadPlan& hp, int fi
                const T* gy, const T* x, const T* raw, const T* w, T* gx, T* graw, T* gw, T* gbias, void* workspace,
                size_t workspace_bytes, cudaStream_t st) {
   const size_t stage = 2 * (hp.geo_bytes + hp.mask_bytes);
-  const size_t need = stage + generic_bwd_workspace(g, sizeof(T) == 8 ? D2C_F64 : D2C_F32, cap);
+  const size_t need = stage + exact_bwd_workspace(g, sizeof(T) == 8 ? D2C_F64 : D2C_F32, cap);
   if (!ws_ok(workspace, workspace_bytes, need)) return D2C_ERR_WORKSPACE;
   uint8_t* wsp = reinterpret_cast<uint8_t*>(workspace);
   T* geo = reinterpret_cast<T*>(wsp);
   T* mask = hp.mask_n ? reinterpret_cast<T*>(wsp + hp.geo_bytes) : nullptr;
   T* ggeo = reinterpret_cast<T*>(wsp + hp.geo_bytes + hp.mask_bytes);
   T* gmask = hp.mask_n ? reinterpret_cast<T*>(wsp + 2 * hp.geo_bytes + hp.mask_bytes) : nullptr;
-  T* dcol = reinterpret_cast<T*>(wsp + stage);
   head_apply_kernel<T><<<grid_1d((long long)g.B * (hp.geo_n + hp.mask_n) * g.V, 256), 256, 0, st>>>(
       raw, hp.rstride, g.V, g.B, h->geo_channel0, hp.geo_n, h->mask_channel0, hp.mask_n, is_field ? h->size_act : 0,
       h->mask_act, geo, mask);
   D2C_LAUNCH_CHECK();
-  const int nb = bwd_slice_clips(g, cap);
   int rc;
   if (is_field) {
     FieldCoords<T> fc;
     if ((rc = make_field_coords<T>(g, field_mode, geo, &fc))) return rc;
-    rc = launch_bwd_generic<T, FieldCoords<T>, true>(g, fc, gy, x, mask, w, gx, ggeo, (size_t)g.B * hp.geo_n * g.V, gmask, gw,
-                                                     gbias, dcol, nb, st);
+    rc = exact::launch_bwd<T, FieldCoords<T>, true>(g, fc, gy, x, mask, w, gx, ggeo, (size_t)g.B * hp.geo_n * g.V, gmask, gw,
+                                                    gbias, wsp + stage, cap, st);
   } else {
     OffsetCoords<T> oc{geo, 0};
-    rc = launch_bwd_generic<T, OffsetCoords<T>, false>(g, oc, gy, x, mask, w, gx, ggeo, 0, gmask, gw, gbias, dcol, nb, st);
+    rc = exact::launch_bwd<T, OffsetCoords<T>, false>(g, oc, gy, x, mask, w, gx, ggeo, 0, gmask, gw, gbias, wsp + stage, cap, st);
   }
   if (rc) return rc;
   head_grad_kernel<T><<<grid_1d((long long)g.B * h->raw_channels * g.V, 256), 256, 0, st>>>(
@@ -854,7 +884,7 @@ size_t d2c_head_workspace_bytes(int op, const d2c_conv_desc* desc, const d2c_hea
   const unsigned long long cap = g_max_intermediate.load();
   // whichever route the call takes under the current settings, and never less than the plain op's workspace
   const size_t plain = d2c_workspace_bytes(op, desc);
-  const size_t staged = (bwd ? 2 : 1) * (hp.geo_bytes + hp.mask_bytes) + (bwd ? generic_bwd_workspace(g, desc->dtype, cap) : 0);
+  const size_t staged = (bwd ? 2 : 1) * (hp.geo_bytes + hp.mask_bytes) + (bwd ? exact_bwd_workspace(g, desc->dtype, cap) : exact_fwd_workspace(g, desc->dtype));
   const bool fused = bwd ? head_fused_bwd(g, desc->dtype, mode, cap) : head_fused_fwd(g, desc->dtype, mode);
   return fused ? plain : (staged > plain ? staged : plain);
 }

@@ -135,6 +135,11 @@ template <typename T>
 struct OffsetCoords {
   const T* offset;
   long long bstride;   // elements between clips; 0 = dense [B, G*3K, V]
+  // (i, j, k): the tap's position in the kernel
+  __device__ __forceinline__ void get_at(const Geom& g, int b, int grp, int tap, int, int, int, int v, int bz, int by,
+                                         int bx, T& z, T& y, T& x) const {
+    get(g, b, grp, tap, v, bz, by, bx, z, y, x);
+  }
   __device__ __forceinline__ void get(const Geom& g, int b, int grp, int tap, int v, int bz, int by,
                                       int bx, T& z, T& y, T& x) const {
     const long long bs = bstride ? bstride : (long long)g.G * 3 * g.K * g.V;
@@ -150,6 +155,10 @@ struct OffsetCoords {
 template <typename T>
 struct Offset1dCoords {
   const T* offset;
+  __device__ __forceinline__ void get_at(const Geom& g, int b, int grp, int tap, int, int, int, int v, int bz, int by,
+                                         int bx, T& z, T& y, T& x) const {
+    get(g, b, grp, tap, v, bz, by, bx, z, y, x);
+  }
   __device__ __forceinline__ void get(const Geom& g, int b, int grp, int tap, int v, int bz, int by,
                                       int bx, T& z, T& y, T& x) const {
     z = (T)bz;
@@ -175,9 +184,12 @@ struct FieldCoords {
   T axis[3][kMaxFieldKernelDim];  // linspace(-dil*(k/2), dil*(k/2), k) per dim
   long long bstride;  // elements between clips; 0 = dense [B, nch, V]
   int act;            // d2c_size_act applied to the values read (0: the map holds the scales themselves)
-  __device__ __forceinline__ void get(const Geom& g, int b, int /*grp*/, int tap, int v, int bz,
+  __device__ __forceinline__ void get(const Geom& g, int b, int grp, int tap, int v, int bz,
                                       int by, int bx, T& z, T& y, T& x) const {
-    const int k = tap % g.kw, j = (tap / g.kw) % g.kh, i = tap / (g.kw * g.kh);
+    get_at(g, b, grp, tap, tap / (g.kw * g.kh), (tap / g.kw) % g.kh, tap % g.kw, v, bz, by, bx, z, y, x);
+  }
+  __device__ __forceinline__ void get_at(const Geom& g, int b, int /*grp*/, int /*tap*/, int i, int j, int k, int v, int bz,
+                                         int by, int bx, T& z, T& y, T& x) const {
     const T* p = size_map + (long long)b * (bstride ? bstride : (long long)nch * g.V) + v;
     const T sz = ch[0] < 0 ? (T)1 : size_act_value(act, __ldg(p + (long long)ch[0] * g.V));
     const T sy = ch[1] < 0 ? (T)1 : size_act_value(act, __ldg(p + (long long)ch[1] * g.V));

@@ -13,9 +13,9 @@
 //
 // The weight gradient is in deform_sm100_dw.cu; sampling positions come from the records of
 // sm100_gather.cuh, computed once per backward call.
-#include "deform_generic.cuh"   // grad_bias_kernel, bwd_slice_clips
 #include <type_traits>
 
+#include "deform_exact.h"   // slice_clips
 #include "deform_sm100.h"
 #include "sm100_gather.cuh"
 #include "sm100_ptx.cuh"
@@ -725,7 +725,7 @@ bool make_bwd_plan(const Geom& g, unsigned long long cap, bool x3, BwdPlan* pl) 
   pl->tmem_cols = 512;
   pl->smem_bytes = pl->KB * kABlockBytes + kBStages * kBStageBytes + 256 + 1024;
   if (pl->smem_bytes > kSmemLimit) return false;
-  pl->clips_per_chunk = bwd_slice_clips(g, cap);
+  pl->clips_per_chunk = exact::slice_clips(g, cap);
   pl->x_cl_bytes = align_up((size_t)g.B * g.Vin * g.Cin * (x3 ? 4 : 2), 256);
   pl->rec_bytes = pos_records_bytes(g);
   pl->gat_bytes = gather_records_bytes(g);

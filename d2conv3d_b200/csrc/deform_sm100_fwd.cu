@@ -100,11 +100,6 @@ struct FwdParams {
   int sav_pairg;               // bf16x3: 32 channels per offset group (a 64-channel slice spans two groups)
 };
 
-__device__ __forceinline__ void cta_unit_range(long long n_units, long long& beg, long long& end) {
-  beg = n_units * blockIdx.x / gridDim.x;
-  end = n_units * (blockIdx.x + 1) / gridDim.x;
-}
-
 // Part r of a CTA's work: the units of part r (a clip, FwdParams::units_per_part each) are cut into one contiguous
 // range per CTA, and the CTA takes the range (blockIdx.x + r * part_shift) mod gridDim.x.  All CTAs therefore work
 // inside the SAME clip at the same time -- the staged input they gather from is one clip, not the whole batch, which
