@@ -15,7 +15,8 @@ enum Route { kChannelsLast = 0, kDirect = 1, kAny = 2 };
 
 inline Route route_of(const Geom& g, bool one_d) {
   if (g.cpg % 4 || g.cin_g % 4) return kAny;
-  return !one_d && g.Cin >= kMinChannelsCl ? kChannelsLast : kDirect;
+  // the channels-last kernels address a clip in 31 bits
+  return !one_d && g.Cin >= kMinChannelsCl && g.Vin * g.Cin <= 0x7fffffffLL ? kChannelsLast : kDirect;
 }
 
 // Output channels of a block tile.
@@ -24,14 +25,18 @@ inline int tile_n(const Geom& g) { return g.cout_g <= 32 ? 32 : (g.cout_g <= 64 
 
 template <typename T>
 inline size_t x_cl_bytes(const Geom& g) { return align_up(sizeof(T) * (size_t)g.B * g.Vin * g.Cin, 256); }
+template <int TN> constexpr int kPitchB = TN + 4;     // row pitch of a B tile in elements
+template <typename T> constexpr int kDcolN = sizeof(T) == 4 ? 128 : 64;      // column rows of a gradient-column tile
+
+// Staged weights: B-tile images of 16 x (columns + 4) elements.
 template <typename T>
-inline size_t w_fwd_bytes(const Geom& g) {
-  return align_up(sizeof(T) * (size_t)g.groups * align_up((size_t)g.cin_g * g.K, kTK) * align_up(g.cout_g, tile_n<T>(g)), 256);
+inline size_t w_image_bytes(const Geom& g, int rows, int cols, int tn) {
+  return align_up(sizeof(T) * (size_t)g.groups * ((cols + tn - 1) / tn) * align_up((size_t)rows, kTK) * (tn + 4), 256);
 }
 template <typename T>
-inline size_t w_bwd_bytes(const Geom& g) {
-  return align_up(sizeof(T) * (size_t)g.groups * align_up(g.cout_g, kTK) * align_up((size_t)g.cin_g * g.K, 128), 256);
-}
+inline size_t w_fwd_bytes(const Geom& g) { return w_image_bytes<T>(g, g.cin_g * g.K, g.cout_g, tile_n<T>(g)); }
+template <typename T>
+inline size_t w_bwd_bytes(const Geom& g) { return w_image_bytes<T>(g, g.cout_g, g.cin_g * g.K, kDcolN<T>); }
 
 // Clips per backward slice under the intermediate-element cap.
 inline int slice_clips(const Geom& g, unsigned long long cap) {
