@@ -560,7 +560,15 @@ sample_grad_taps_kernel(Geom g, ClStrides cs, int b0, int nh, const float4* __re
     const float wy[2] = {sub_rn(1.f, s.fy), sub_rn(1.f, s.gy)};
     const float wx[2] = {sub_rn(1.f, s.fx), sub_rn(1.f, s.gx)};
     const bool okz[2] = {true, s.gz < 1.f}, oky[2] = {true, s.gy < 1.f}, okx[2] = {true, s.gx < 1.f};
-    const unsigned valid = active ? s.valid : 0u;
+    unsigned valid = active ? s.valid : 0u;
+    if constexpr (FieldOut) {
+      // A tap at the kernel's centre on an axis does not move along it: the upper corners of that axis weigh nothing and the
+      // axis takes no gradient, so they are not read (4.6 corners a tap instead of 8 with 3 x 3 x 3 taps).
+      const int k = tap % g.kw, jj = (tap / g.kw) % g.kh, i = tap / (g.kw * g.kh);
+      if (field_axes.pos[0][i] == 0.f && !okz[1]) valid &= 0x0fu;
+      if (field_axes.pos[1][jj] == 0.f && !oky[1]) valid &= 0x33u;
+      if (field_axes.pos[2][k] == 0.f && !okx[1]) valid &= 0x55u;
+    }
     const int off0 = ((s.z0 * g.H + s.y0) * g.W + s.x0) * g.Cin + chbase;
     float G[8];
 #pragma unroll

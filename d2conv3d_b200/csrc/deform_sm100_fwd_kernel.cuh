@@ -433,6 +433,8 @@ fwd_sm100_kernel(const FwdParams p) {
     };
 
     uint4 c0[8], c1[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) c0[q] = c1[q] = make_uint4(0u, 0u, 0u, 0u);
     if (n_my_units > 0) {
       ok = ptx::mbar_wait(r_full(0), 0, abort_flag);
       if (ok) issue(0, 0, c0);

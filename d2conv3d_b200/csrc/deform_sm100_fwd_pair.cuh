@@ -243,13 +243,17 @@ fwd_sm100_pair_kernel(const PairParams pp) {
     const uint32_t a_full_leader[kAStages] = {ptx::mapa_shared(a_full(0), 0), ptx::mapa_shared(a_full(1), 0),
                                               ptx::mapa_shared(a_full(2), 0), ptx::mapa_shared(a_full(3), 0)};
     const uint32_t n_my_units = (uint32_t)(u_end - u_beg);
+    uint4 c[kRowsPerThread][8];
+#pragma unroll
+    for (int i = 0; i < kRowsPerThread; ++i)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) c[i][q] = make_uint4(0u, 0u, 0u, 0u);
     for (uint32_t k = 0; k < n_my_units; ++k) {
       const int sr = k % kRStages, sa = k % kAStages;
       if (!ptx::mbar_wait(r_full(sr), (k / kRStages) & 1, abort_flag)) break;
       const uint8_t* rec_stage = base_ptr + rec_off + sr * kRStageBytes;
       const __half* xb = reinterpret_cast<const __half*>(p.x_cl) + *reinterpret_cast<const long long*>(rec_stage + kRecBytes) + j * 8;
       const int rows = *reinterpret_cast<const int*>(rec_stage + kRecBytes + 8);
-      uint4 c[kRowsPerThread][8];
 #pragma unroll
       for (int i = 0; i < kRowsPerThread; ++i) {
         const int r = r0 + kRowStride * i;

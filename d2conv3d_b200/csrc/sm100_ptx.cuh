@@ -318,6 +318,13 @@ __device__ __forceinline__ uint4 ldg_nc_v4(const void* p) {
   asm("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
   return r;
 }
+// The same under a predicate: r keeps its contents where cond is 0.
+__device__ __forceinline__ void ldg_nc_v4_if(uint4& r, const void* p, uint32_t cond) {
+  asm("{\n\t.reg .pred q;\n\t"
+      "setp.ne.u32 q, %5, 0;\n\t"
+      "@q ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+      : "+r"(r.x), "+r"(r.y), "+r"(r.z), "+r"(r.w) : "l"(p), "r"(cond));
+}
 __device__ __forceinline__ void stg_v4_hint(void* p, uint4 v, uint64_t pol) {
   asm volatile("st.global.L2::cache_hint.v4.u32 [%0], {%1, %2, %3, %4}, %5;"
                ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "l"(pol)
