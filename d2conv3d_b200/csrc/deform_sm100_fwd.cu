@@ -59,6 +59,12 @@ constexpr int kRStageBytes = kRecBytes + 16;      // ... + unit header {int64 x_
 constexpr int kRowStride = kGatherWarps * 4;          // 8 threads per row -> rows handled per pass
 constexpr int kRowsPerThread = kBM / kRowStride;
 constexpr int kSmemLimit = 227 * 1024;
+// Shared memory is what the L1 cache does not get, and the gather lives off L1 (the two rows of corners of neighbouring
+// voxels and taps): the weight ring takes no more than leaves the 196 KB split (1 KB of it is the system's), 60 KB of L1.
+// 256 output channels, field layer, 2 x 8 x 60 x 107: 4 stages of 32 KB (28 KB of L1) 2.32 ms, 3 stages 2.15 ms, 2 stages
+// (92 KB of L1, but the ring runs dry) 2.16 ms.  512 output channels with 64 KB stages had no room for that: 1.55 ms at 2 x 8
+// x 30 x 54 where 32 KB stages take 1.31 ms.  Two A stages or two record stages instead cost more than the L1 gives back.
+constexpr int kSmemGather = 195 * 1024;
 // Fewest units a CTA is started for.  A unit takes 1.9-2.3 us in its CTA (the producers' gather latency), starting a CTA
 // and adding its partial tile to y about 5 us together: below four units per CTA more CTAs no longer shorten the call.
 // Small layer (432 units): 27 CTAs of 16 units 36.2 us, 108 CTAs of 4 units 17.7 us.
@@ -84,7 +90,8 @@ struct FwdParams {
   long long units_per_part;
   int seg_cap;                 // at most this many units accumulate in tensor memory before the partial result is
                                // added to y (see run_fwd); S = no limit
-  int b_stages, b_stage_bytes;
+  int b_stages, b_stage_bytes; // weight ring: one stage = one N block (at most 256 rows) of a slice
+  int w_slice_bytes;           // Cout rows x 128 B
   int tmem_cols;
   // Samples kept for the weight gradient (nullable): the blended A tiles, written to global as they are produced,
   // in blocks of 8 KB = one 64-channel slice x 64 voxels (rows of 128 B, 16-byte chunks XOR-swizzled by row & 7):
@@ -178,7 +185,7 @@ stage_weight_sw128_x3_kernel(int Cout, int Cin, int K, int cpg, int nh, const fl
 }
 
 struct Plan {
-  int nh, S, tiles_per_clip, n_tiles, b_stages, b_stage_bytes, tmem_cols, smem_bytes, dual, r_stage_bytes;
+  int nh, S, tiles_per_clip, n_tiles, b_stages, b_stage_bytes, w_slice_bytes, tmem_cols, smem_bytes, dual, r_stage_bytes;
   size_t x_cl_bytes, w_sw_bytes, rec_bytes;
 };
 
@@ -190,6 +197,7 @@ bool make_plan(const Geom& g, bool x3, Plan* pl) {
   pl->dual = dual ? 1 : 0;
   pl->r_stage_bytes = (1 + pl->dual) * kRecBytes + 16;
   if (g.Cout % 64 != 0 || g.Cout > kMaxN) return false;
+  if (dual && g.Cout > 448) return false;      // layers this wide run the (more exact) split kernel
   if (g.Vin * g.Cin > 0x7fffffffLL) return false;                 // 32-bit element offsets within a clip
   if (g.K * 64 * (int)sizeof(float) > 48 * 1024) return false;    // weight staging kernel's smem
   pl->nh = dual ? 1 : g.cpg / (x3 ? 32 : kBK);
@@ -197,10 +205,13 @@ bool make_plan(const Geom& g, bool x3, Plan* pl) {
   pl->tiles_per_clip = (g.V + kBM - 1) / kBM;
   pl->n_tiles = pl->tiles_per_clip * g.B;
   if ((long long)pl->n_tiles * pl->S > 0x7fffffffLL) return false;   // the kernel counts units in 31 bits
-  pl->b_stage_bytes = g.Cout * 128;
+  pl->w_slice_bytes = g.Cout * 128;
+  pl->b_stage_bytes = (g.Cout < 256 ? g.Cout : 256) * 128;
   // 256 bytes of barriers + 272 bytes of part ranges (rounded to 512) + 1 KB of alignment slack
-  int nb = (kSmemLimit - 1024 - 768 - kAStages * kAStageBytes - kRStages * pl->r_stage_bytes) / pl->b_stage_bytes;
+  const int other = 1024 + 768 + kAStages * kAStageBytes + kRStages * pl->r_stage_bytes;
+  int nb = (kSmemGather - other) / pl->b_stage_bytes;
   if (nb > 4) nb = 4;
+  if (nb < 2) nb = (kSmemLimit - other) / pl->b_stage_bytes < 2 ? 0 : 2;
   if (nb < 2) return false;
   pl->b_stages = nb;
   int cols = 32;
@@ -208,7 +219,7 @@ bool make_plan(const Geom& g, bool x3, Plan* pl) {
   pl->tmem_cols = cols;
   pl->smem_bytes = kAStages * kAStageBytes + pl->b_stages * pl->b_stage_bytes + kRStages * pl->r_stage_bytes + 768 + 1024;
   pl->x_cl_bytes = align_up((size_t)g.B * g.Vin * g.Cin * (x3 ? 4 : 2), 256);
-  pl->w_sw_bytes = align_up((size_t)pl->S * pl->b_stage_bytes, 256);
+  pl->w_sw_bytes = align_up((size_t)pl->S * pl->w_slice_bytes, 256);
   pl->rec_bytes = gather_records_bytes(g);
   return true;
 }
@@ -285,9 +296,9 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
   // single-CTA kernel so far.
   const int n_tile_pairs = (pl.n_tiles + 1) / 2;
   const long long n_pair_units = (long long)n_tile_pairs * pl.S;
-  int pair_b_stages = (kSmemLimit - 1024 - 256 - kAStages * kAStageBytes - kRStages * kRStageBytes) / (pl.b_stage_bytes / 2);
+  int pair_b_stages = (kSmemLimit - 1024 - 256 - kAStages * kAStageBytes - kRStages * kRStageBytes) / (pl.w_slice_bytes / 2);
   if (pair_b_stages > 4) pair_b_stages = 4;
-  const int pair_smem = kAStages * kAStageBytes + pair_b_stages * (pl.b_stage_bytes / 2) + kRStages * kRStageBytes + 256 + 1024;
+  const int pair_smem = kAStages * kAStageBytes + pair_b_stages * (pl.w_slice_bytes / 2) + kRStages * kRStageBytes + 256 + 1024;
   long long pair_clusters = 0;
   {
     static int pair_enabled = -1;
@@ -347,7 +358,7 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
   p.n_parts = n_parts; p.rr = rr ? 1 : 0;
   p.units_per_part = rr ? 0 : n_units / n_parts; p.part_shift = rr ? 0 : (int)(grid / n_parts);
   p.seg_cap = seg_cap;
-  p.b_stages = pl.b_stages; p.b_stage_bytes = pl.b_stage_bytes; p.tmem_cols = pl.tmem_cols;
+  p.b_stages = pl.b_stages; p.b_stage_bytes = pl.b_stage_bytes; p.w_slice_bytes = pl.w_slice_bytes; p.tmem_cols = pl.tmem_cols;
   // keep the samples for the weight gradient when the caller bound a cache that is large enough
   p.sav = sav; p.sav_np = sav_np; p.sav_pairg = (g.cpg == 32) ? 1 : 0;
   if (sav) sc->format = x3 ? 2 : 1;
@@ -356,7 +367,7 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
     pair::PairParams pp;
     pp.f = p;
     pp.n_tile_pairs = n_tile_pairs; pp.n_pair_units = n_pair_units;
-    pp.b_stages = pair_b_stages; pp.b_half_bytes = pl.b_stage_bytes / 2;
+    pp.b_stages = pair_b_stages; pp.b_half_bytes = pl.w_slice_bytes / 2;
     prof_mark(st, "fwd_sm100_pair");
     pair::fwd_sm100_pair_kernel<<<(unsigned)(2 * pair_clusters), kThreads, pair_smem, st>>>(pp);
     D2C_LAUNCH_CHECK();

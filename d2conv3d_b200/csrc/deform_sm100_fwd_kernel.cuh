@@ -208,17 +208,17 @@ fwd_sm100_kernel(const FwdParams p) {
       // no integer division or modulo by run-time values in the per-unit path (ring slots and phases are carried as
       // counters), descriptors are built from constants hoisted out of the loops.
       int seg = 0;
-      uint32_t k = 0;           // units consumed so far (A and B rings advance together)
-      int sb = 0;               // weight-ring slot of unit k and its phase
+      uint32_t k = 0;           // units consumed so far
+      int sb = 0;               // weight-ring slot and its phase
       uint32_t phb = 0;
       bool ok = true;
       constexpr int kSteps = kX3 ? 6 : 4;
       // K sub-blocks (16 channels = 32 bytes) of the A and B rows that meet in each MMA
       constexpr int ka_[6] = {0, 1, kX3 ? 2 : 2, kX3 ? 3 : 3, 0, 1};   // bf16: (k,k); x3: hi*hi, lo*hi, hi*lo
       constexpr int kb_[6] = {0, 1, kX3 ? 0 : 2, kX3 ? 1 : 3, 2, 3};
-      const int n_halves = (p.N + 255) / 256;
+      const int n_blocks = (p.N + 255) / 256;      // N blocks of a slice, one weight stage each
       const uint32_t idesc_full = ptx::umma_idesc_bf16_f32(kBM, 256);
-      const uint32_t idesc_last = ptx::umma_idesc_bf16_f32(kBM, p.N - (n_halves - 1) * 256);
+      const uint32_t idesc_last = ptx::umma_idesc_bf16_f32(kBM, p.N - (n_blocks - 1) * 256);
       const uint64_t adesc0 = ptx::umma_desc_kmajor_sw128(a_base), bdesc0 = ptx::umma_desc_kmajor_sw128(b_base);
       const uint64_t a_step = (uint64_t)(kAStageBytes >> 4), b_step = (uint64_t)(p.b_stage_bytes >> 4);
       for (int part = 0; ok && part < p.n_parts; ++part) {
@@ -236,24 +236,25 @@ fwd_sm100_kernel(const FwdParams p) {
           D2C_TR(2, k, 0);
           if (!ptx::mbar_wait(a_full(sa), (k / kAStages) & 1, abort_flag)) { ok = false; break; }
           D2C_TR(2, k, 1);
-          if (!ptx::mbar_wait(b_full(sb), phb, abort_flag)) { ok = false; break; }
-          D2C_TR(2, k, 2);
           ptx::tc_fence_after();
           // descriptor address fields count 16-byte units: a stage further along adds stage_bytes / 16
           const uint64_t adesc = adesc0 + a_step * (uint64_t)sa;
-          const uint64_t bdesc = bdesc0 + b_step * (uint64_t)sb;
+          for (int h = 0; h < n_blocks; ++h) {
+            if (!ptx::mbar_wait(b_full(sb), phb, abort_flag)) { ok = false; break; }
+            D2C_TR(2, k, 2);
+            ptx::tc_fence_after();
+            const uint64_t bdesc = bdesc0 + b_step * (uint64_t)sb;
 #pragma unroll
-          for (int kk = 0; kk < kSteps; ++kk) {
-            for (int h = 0; h < n_halves; ++h)
-              ptx::umma_bf16(tmem_base + (uint32_t)(h * 256), adesc + (uint64_t)(2 * ka_[kk]),
-                             bdesc + (uint64_t)(h * (256 * 128 / 16)) + (uint64_t)(2 * kb_[kk]),
-                             h + 1 < n_halves ? idesc_full : idesc_last, (s > s_beg || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < kSteps; ++kk)
+              ptx::umma_bf16(tmem_base + (uint32_t)(h * 256), adesc + (uint64_t)(2 * ka_[kk]), bdesc + (uint64_t)(2 * kb_[kk]),
+                             h + 1 < n_blocks ? idesc_full : idesc_last, (s > s_beg || kk > 0) ? 1u : 0u);
+            D2C_TR(2, k, 3);
+            ptx::umma_commit(b_empty(sb));
+            if (++sb == p.b_stages) { sb = 0; phb ^= 1u; }
           }
-          D2C_TR(2, k, 3);
+          if (!ok) break;
           ptx::umma_commit(a_empty(sa));
-          ptx::umma_commit(b_empty(sb));
           D2C_TR(2, k, 4);
-          if (++sb == p.b_stages) { sb = 0; phb ^= 1u; }
         }
         if (ok) ptx::umma_commit(acc_full);
         s_beg = s_end == p.S ? 0 : s_end;
@@ -263,7 +264,8 @@ fwd_sm100_kernel(const FwdParams p) {
   } else if (warp == kLoadWarpFwd) {
     // ===================== weight-slice loader =====================
     if (lane == 0) {
-      uint32_t k = 0;
+      [[maybe_unused]] uint32_t k = 0;
+      uint32_t issued = 0;
       int sb = 0;                       // ring slot and phase as counters: no division in the per-unit path
       uint32_t phb = 1;                 // the wait for a FREE slot looks at the previous phase
       for (int part = 0; part < p.n_parts; ++part) {
@@ -271,23 +273,25 @@ fwd_sm100_kernel(const FwdParams p) {
       int u_beg, u_end;
     part_range(part, u_beg, u_end);
       int s = u_beg % p.S;              // once per part
-      const uint8_t* src = p.w_sw + (long long)s * p.b_stage_bytes;
+      const uint8_t* src = p.w_sw + (long long)s * p.w_slice_bytes;
       const int n_part_units = u_end - u_beg;
-      for (int i = 0; i < n_part_units; ++i, ++k) {
+      bool ok = true;
+      for (int i = 0; ok && i < n_part_units; ++i, ++k) {
         D2C_TR(1, k, 0);
-        if (!ptx::mbar_wait(b_empty(sb), phb, abort_flag, 200)) break;
-        D2C_TR(1, k, 1);
-        ptx::mbar_arrive_expect_tx(b_full(sb), (uint32_t)p.b_stage_bytes);
-        const uint32_t dst = b_base + sb * p.b_stage_bytes;
-        for (int off = 0; off < p.b_stage_bytes; off += 32768)
-          ptx::bulk_g2s(dst + off, src + off, (uint32_t)min(32768, p.b_stage_bytes - off), b_full(sb));
-        if (++sb == p.b_stages) { sb = 0; phb ^= 1u; }
-        src += p.b_stage_bytes;
+        for (int off = 0; off < p.w_slice_bytes; off += p.b_stage_bytes) {
+          if (!ptx::mbar_wait(b_empty(sb), phb, abort_flag, 200)) { ok = false; break; }
+          D2C_TR(1, k, 1);
+          const uint32_t bytes = (uint32_t)min(p.b_stage_bytes, p.w_slice_bytes - off);
+          ptx::mbar_arrive_expect_tx(b_full(sb), bytes);
+          ptx::bulk_g2s(b_base + sb * p.b_stage_bytes, src + off, bytes, b_full(sb));
+          ++issued;
+          if (++sb == p.b_stages) { sb = 0; phb ^= 1u; }
+        }
+        src += p.w_slice_bytes;
         if (++s == p.S) { s = 0; src = p.w_sw; }
       }
       }
       // never leave with a bulk copy in flight: wait (bounded) for the last copies issued
-      const uint32_t issued = k;
       for (uint32_t q = (issued > (uint32_t)p.b_stages ? issued - p.b_stages : 0); q < issued; ++q) {
         const long long t0 = clock64();
         while (!ptx::mbar_try_wait(b_full(q % p.b_stages), (q / p.b_stages) & 1))

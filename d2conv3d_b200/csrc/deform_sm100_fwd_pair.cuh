@@ -184,7 +184,7 @@ fwd_sm100_pair_kernel(const PairParams pp) {
         const int s = (int)(u % p.S), sb = k % pp.b_stages;
         if (!ptx::mbar_wait_cluster(b_empty(sb), ((k / pp.b_stages) & 1) ^ 1, abort_flag, 200)) break;
         ptx::mbar_arrive_expect_tx(b_full(sb), (uint32_t)pp.b_half_bytes);
-        const uint8_t* src = p.w_sw + (long long)s * p.b_stage_bytes;
+        const uint8_t* src = p.w_sw + (long long)s * p.w_slice_bytes;
         const uint32_t dst = b_base + sb * pp.b_half_bytes;
         for (int n0 = 0, nb = 0; n0 < p.N; n0 += 256, ++nb) {
           const int rows = min(256, p.N - n0) / 2;
