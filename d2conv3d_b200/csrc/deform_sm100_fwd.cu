@@ -55,6 +55,11 @@ constexpr int kThreads = (6 + 16 + 1) * 32;   // 4 epilogue + MMA + weight loade
 constexpr int kEpiWarps = 4, kMmaWarp = 4, kLoadWarp = 5, kGatherWarp0 = 6, kGatherWarps = 16, kRecWarp = 22;
 constexpr int kRStages = 4;                       // gather-record ring: one stage = the records of a unit's 128 rows
 constexpr int kRecBytes = kBM * 48;               // 6 KB of records ...
+constexpr int kMaskBytes = kBM * 4;               // modulation of 128 rows, where it is not in the records
+// one record set per offset group of the unit, or one set and a modulation row per group; then the unit header
+constexpr int kRStageBytesOf(int dual, int shared) {
+  return (shared ? kRecBytes + (1 + dual) * kMaskBytes : (1 + dual) * kRecBytes) + 16;
+}
 constexpr int kRStageBytes = kRecBytes + 16;      // ... + unit header {int64 x_cl element offset of the slice, int rows}
 constexpr int kRowStride = kGatherWarps * 4;          // 8 threads per row -> rows handled per pass
 constexpr int kRowsPerThread = kBM / kRowStride;
@@ -76,13 +81,15 @@ struct FwdParams {
   Geom g;
   const void* x_cl;            // [B][Vin][Cin] channels-last staging of x: fp16 (bf16 mode) or fp32 (bf16x3 mode)
   const uint8_t* w_sw;         // [S][N rows x 128 B], rows swizzled exactly as the smem B tile
-  const uint4* recs;           // [B][G][K][V] gather records (3 x uint4 each, sm100_gather.cuh)
+  const uint4* recs;           // [B][G][K][V] gather records (3 x uint4 each, sm100_gather.cuh), or
+  const float* masks;          // [B][K][V] records and [B][G][K][V padded] modulation values
   const float* bias;           // [Cout] or nullptr
   float* y;                    // [B, Cout, V]
   ClStrides cs;
   int N;                       // Cout
   int nh;                      // K slices per (group, tap) = cpg / 64
-  int S;                       // slices per tile = G * K * nh
+  int S;                       // slices per tile = G * K * nh, (group, K slice, tap) with the tap fastest: neighbouring taps of
+                               // the same channels sample mostly the same lines, which L1 then still holds
   int tiles_per_clip, n_tiles;
   long long n_units;           // n_tiles * S
   int n_parts, part_shift;     // see cta_part_range
@@ -125,7 +132,7 @@ __device__ __forceinline__ void cta_part_range(const FwdParams& p, int part, lon
 // ---- staging kernels -------------------------------------------------------------------------
 
 // w [Cout][Cin][K] fp32 (weight groups == 1) -> w_sw [S][Cout rows x 128 B] bf16, slice
-// s = (grp*K + tap)*nh + h holding channels grp*cpg + h*64 .. +63, each row's 16-byte
+// s = (grp*nh + h)*K + tap holding channels grp*cpg + h*64 .. +63, each row's 16-byte
 // chunks XOR-swizzled by (row & 7) -- the byte image of the shared-memory B tile.
 __global__ void __launch_bounds__(64)
 stage_weight_sw128_kernel(int Cout, int Cin, int K, int cpg, int nh, const float* __restrict__ w,
@@ -145,14 +152,14 @@ stage_weight_sw128_kernel(int Cout, int Cin, int K, int cpg, int nh, const float
     for (int e = 0; e < 8; ++e) v[e] = wrow[(jj * 8 + e) * K + tap];
     out.x = ptx::pack_bf16x2(v[0], v[1]); out.y = ptx::pack_bf16x2(v[2], v[3]);
     out.z = ptx::pack_bf16x2(v[4], v[5]); out.w = ptx::pack_bf16x2(v[6], v[7]);
-    const long long s = ((long long)grp * K + tap) * nh + h;
+    const long long s = ((long long)grp * nh + h) * K + tap;
     uint8_t* dst = w_sw + s * (long long)Cout * 128 + (long long)(co >> 3) * 1024 + (co & 7) * 128 +
                    ((jj ^ (co & 7)) << 4);
     *reinterpret_cast<uint4*>(dst) = out;
   }
 }
 
-// bf16x3 mode: slice s = (grp*K + tap)*nh + h with nh = cpg/32 holds 32 channels; each row is
+// bf16x3 mode: slice s = (grp*nh + h)*K + tap with nh = cpg/32 holds 32 channels; each row is
 // [hi(32 ch) | lo(32 ch)] where hi = bf16(w), lo = bf16(w - hi); same swizzle.
 __global__ void __launch_bounds__(64)
 stage_weight_sw128_x3_kernel(int Cout, int Cin, int K, int cpg, int nh, const float* __restrict__ w,
@@ -177,7 +184,7 @@ stage_weight_sw128_x3_kernel(int Cout, int Cin, int K, int cpg, int nh, const fl
     uint4 out;
     out.x = ptx::pack_bf16x2(v[0], v[1]); out.y = ptx::pack_bf16x2(v[2], v[3]);
     out.z = ptx::pack_bf16x2(v[4], v[5]); out.w = ptx::pack_bf16x2(v[6], v[7]);
-    const long long s = ((long long)grp * K + tap) * nh + h;
+    const long long s = ((long long)grp * nh + h) * K + tap;
     uint8_t* dst = w_sw + s * (long long)Cout * 128 + (long long)(co >> 3) * 1024 + (co & 7) * 128 +
                    ((jj ^ (co & 7)) << 4);
     *reinterpret_cast<uint4*>(dst) = out;
@@ -189,13 +196,14 @@ struct Plan {
   size_t x_cl_bytes, w_sw_bytes, rec_bytes;
 };
 
-bool make_plan(const Geom& g, bool x3, Plan* pl) {
+// shared: the offset groups share their records (dilation field)
+bool make_plan(const Geom& g, bool x3, Plan* pl, bool shared = false) {
   if (g.groups != 1) return false;
   // a unit must lie inside one offset group -- or, single-pass mode with 32 channels per group, span exactly two
   const bool dual = !x3 && g.cpg == 32 && g.G % 2 == 0;
   if (!dual && g.cpg % (x3 ? 32 : kBK) != 0) return false;
   pl->dual = dual ? 1 : 0;
-  pl->r_stage_bytes = (1 + pl->dual) * kRecBytes + 16;
+  pl->r_stage_bytes = kRStageBytesOf(pl->dual, shared ? 1 : 0);
   if (g.Cout % 64 != 0 || g.Cout > kMaxN) return false;
   if (dual && g.Cout > 448) return false;      // layers this wide run the (more exact) split kernel
   if (g.Vin * g.Cin > 0x7fffffffLL) return false;                 // 32-bit element offsets within a clip
@@ -227,18 +235,27 @@ bool make_plan(const Geom& g, bool x3, Plan* pl) {
 // Which variant serves this shape in this math mode: bf16 mode takes the single-pass kernel where it applies
 // and otherwise the (more exact) split kernel, e.g. for 32 channels per offset group; auto / bf16x3 take the
 // split kernel only.  Returns false when the tensor-core tier does not apply.
-bool pick_variant(const Geom& g, int math_mode, bool* x3, Plan* pl) {
+bool pick_variant(const Geom& g, int math_mode, bool* x3, Plan* pl, bool shared = false) {
   if (math_mode == D2C_MATH_FP32) return false;
-  if (math_mode == D2C_MATH_BF16 && make_plan(g, false, pl)) { *x3 = false; return true; }
-  if (make_plan(g, true, pl)) { *x3 = true; return true; }
+  if (math_mode == D2C_MATH_BF16 && make_plan(g, false, pl, shared)) { *x3 = false; return true; }
+  if (make_plan(g, true, pl, shared)) { *x3 = true; return true; }
   return false;
 }
 
-template <int kX3, int kDual, int kSave>
+template <int kX3, int kDual, int kSave, bool kMayShare>
 int launch_fwd(const FwdParams& p, unsigned grid, int smem_bytes, cudaStream_t st) {
-  const int rc = allow_dynamic_smem<fwd_sm100_kernel<kX3, kDual, kSave>>(smem_bytes);
+  if constexpr (kMayShare) {
+    if (p.masks) {
+      const int rc = allow_dynamic_smem<fwd_sm100_kernel<kX3, kDual, kSave, 1>>(smem_bytes);
+      if (rc) return rc;
+      fwd_sm100_kernel<kX3, kDual, kSave, 1><<<grid, kThreadsFwd, smem_bytes, st>>>(p);
+      D2C_LAUNCH_CHECK();
+      return D2C_OK;
+    }
+  }
+  const int rc = allow_dynamic_smem<fwd_sm100_kernel<kX3, kDual, kSave, 0>>(smem_bytes);
   if (rc) return rc;
-  fwd_sm100_kernel<kX3, kDual, kSave><<<grid, kThreadsFwd, smem_bytes, st>>>(p);
+  fwd_sm100_kernel<kX3, kDual, kSave, 0><<<grid, kThreadsFwd, smem_bytes, st>>>(p);
   D2C_LAUNCH_CHECK();
   return D2C_OK;
 }
@@ -248,7 +265,11 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
             const float* w, const float* bias, float* y, void* ws, cudaStream_t st) {
   bool x3 = false;
   Plan pl;
-  if (!pick_variant(g, math_mode, &x3, &pl)) return D2C_ERR_MODE;
+  // a field's groups share their records where there is more than one (behind them in the same space: 48 bytes per tap and
+  // voxel and 4 more per group, against 48 per group)
+  constexpr bool kField = CoordsSharedAcrossGroups<Coords>::value;
+  const bool shared = kField && g.G > 1;
+  if (!pick_variant(g, math_mode, &x3, &pl, shared)) return D2C_ERR_MODE;
   uint8_t* wsp = reinterpret_cast<uint8_t*>(ws);
   void* x_cl = wsp; wsp += pl.x_cl_bytes;
   uint8_t* w_sw = wsp; wsp += pl.w_sw_bytes;
@@ -328,6 +349,7 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
     }
   }
 
+  float* masks = shared && pair_clusters == 0 ? reinterpret_cast<float*>(recs + 3 * (long long)g.B * g.K * g.V) : nullptr;
   if (pair_clusters > 0) { sav = nullptr; pos = nullptr; x_cl = ws; }       // the CTA-pair kernel keeps nothing
   prof_mark(st, "fwd_stage_operands");
   {
@@ -347,11 +369,11 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
                                                                               pl.dual ? 64 : g.cpg, pl.nh, w, w_sw);
       D2C_LAUNCH_CHECK();
     }
-    if ((rc = launch_sample_records(g, coords, mask, head, pos, recs, st, x3))) return rc;
+    if ((rc = launch_sample_records(g, coords, mask, head, pos, recs, st, x3, masks))) return rc;
   }
 
   FwdParams p;
-  p.g = g; p.x_cl = x_cl; p.w_sw = w_sw; p.recs = recs; p.bias = bias; p.y = y;
+  p.g = g; p.x_cl = x_cl; p.w_sw = w_sw; p.recs = recs; p.masks = masks; p.bias = bias; p.y = y;
   p.cs.dz = g.H * g.W * g.Cin; p.cs.dy = g.W * g.Cin; p.cs.dx = g.Cin;
   p.N = g.Cout; p.nh = pl.nh; p.S = pl.S; p.tiles_per_clip = pl.tiles_per_clip; p.n_tiles = pl.n_tiles;
   p.n_units = n_units;
@@ -390,12 +412,12 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
   prof_mark(st, "fwd_sm100_fused");
   const int variant = (sav ? 3 : 0) + (x3 ? 0 : (pl.dual ? 1 : 2));
   switch (variant) {
-    case 0: rc = launch_fwd<1, 0, 0>(p, (unsigned)grid, pl.smem_bytes, st); break;
-    case 1: rc = launch_fwd<0, 1, 0>(p, (unsigned)grid, pl.smem_bytes, st); break;
-    case 2: rc = launch_fwd<0, 0, 0>(p, (unsigned)grid, pl.smem_bytes, st); break;
-    case 3: rc = launch_fwd<1, 0, 1>(p, (unsigned)grid, pl.smem_bytes, st); break;
-    case 4: rc = launch_fwd<0, 1, 1>(p, (unsigned)grid, pl.smem_bytes, st); break;
-    default: rc = launch_fwd<0, 0, 1>(p, (unsigned)grid, pl.smem_bytes, st); break;
+    case 0: rc = launch_fwd<1, 0, 0, kField>(p, (unsigned)grid, pl.smem_bytes, st); break;
+    case 1: rc = launch_fwd<0, 1, 0, kField>(p, (unsigned)grid, pl.smem_bytes, st); break;
+    case 2: rc = launch_fwd<0, 0, 0, kField>(p, (unsigned)grid, pl.smem_bytes, st); break;
+    case 3: rc = launch_fwd<1, 0, 1, kField>(p, (unsigned)grid, pl.smem_bytes, st); break;
+    case 4: rc = launch_fwd<0, 1, 1, kField>(p, (unsigned)grid, pl.smem_bytes, st); break;
+    default: rc = launch_fwd<0, 0, 1, kField>(p, (unsigned)grid, pl.smem_bytes, st); break;
   }
   if (rc) return rc;
 #ifdef D2C_UNIT_TRACE

@@ -29,12 +29,13 @@ constexpr int kMmaWarpFwd = 4, kLoadWarpFwd = 5, kRecWarpFwd = 6, kGatherWarp0Fw
 // kSave = 1: the blended tiles are also written to FwdParams::sav (a forward whose backward will follow).  A template
 //          parameter, not a run-time test, so that the inference kernel carries neither the stores nor the registers
 //          for their addresses.
-template <int kX3, int kDual, int kSave>
+// kShared = 1: records shared by the offset groups and separate modulation rows (sm100_gather.cuh).
+template <int kX3, int kDual, int kSave, int kShared>
 __global__ void __launch_bounds__(kThreadsFwd, 1)
 fwd_sm100_kernel(const FwdParams p) {
   constexpr int kUnitCh = kX3 ? 32 : 64;
-  constexpr int kRStage = (1 + kDual) * kRecBytes + 16;      // record set(s) + unit header
-  constexpr int hdr_off = (1 + kDual) * kRecBytes;
+  constexpr int kRStage = kRStageBytesOf(kDual, kShared);
+  constexpr int hdr_off = kRStage - 16;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -316,7 +317,7 @@ fwd_sm100_kernel(const FwdParams p) {
       const int tile0 = u_beg / p.S;
       int b = tile0 / p.tiles_per_clip, v0 = (tile0 % p.tiles_per_clip) * kBM;
       int tile = tile0;
-      int h = s % p.nh, tap = (s / p.nh) % g.K, grp = (s / p.nh) / g.K;   // dual: grp is the index of a group PAIR
+      int tap = s % g.K, h = (s / g.K) % p.nh, grp = (s / g.K) / p.nh;   // dual: grp is the index of a group PAIR
       const int n_part_units = u_end - u_beg;
       for (int i = 0; i < n_part_units; ++i, ++k) {
         const int sr = k & (kRStages - 1);
@@ -338,11 +339,21 @@ fwd_sm100_kernel(const FwdParams p) {
             const int half = p.sav_pairg ? (grp & 1) : (h & 1);
             word = (((tile * 2 * p.sav_np + (s64 >> 1)) * 4 + (s64 & 1)) << 1) | half;
           } else {
-            word = tile * 2 * (2 * p.sav_np) + s;
+            word = tile * 2 * (2 * p.sav_np) + (grp * g.K + tap) * p.nh + h;
           }
           *reinterpret_cast<int*>(hdr + 12) = word;
         }
         const uint32_t bytes = (uint32_t)rows * 48u;
+        if constexpr (kShared) {
+          const uint32_t m_bytes = (uint32_t)(rows + 3) / 4 * 16;
+          ptx::mbar_arrive_expect_tx(r_full(sr), bytes + m_bytes * (uint32_t)(1 + kDual));
+          ptx::bulk_g2s(rec_base + sr * kRStage, p.recs + 3 * (((long long)b * g.K + tap) * g.V + v0), bytes, r_full(sr));
+#pragma unroll
+          for (int set = 0; set <= kDual; ++set)
+            ptx::bulk_g2s_hint(rec_base + sr * kRStage + kRecBytes + set * kMaskBytes,
+                               p.masks + (((long long)b * g.G + (kDual ? 2 * grp + set : grp)) * g.K + tap) * mask_row(g.V) + v0, m_bytes,
+                               r_full(sr), pol_stream);
+        } else {
         ptx::mbar_arrive_expect_tx(r_full(sr), bytes * (uint32_t)(1 + kDual));
 #pragma unroll
         for (int set = 0; set <= kDual; ++set) {
@@ -350,10 +361,11 @@ fwd_sm100_kernel(const FwdParams p) {
           ptx::bulk_g2s_hint(rec_base + sr * kRStage + set * kRecBytes,
                              p.recs + 3 * ((((long long)b * g.G + og) * g.K + tap) * g.V + v0), bytes, r_full(sr), pol_stream);
         }
-        // next unit: (h, tap, grp) count through the tile's slices, then the next tile of the clip / next clip
-        if (++h == p.nh) {
-          h = 0;
-          if (++tap == g.K) { tap = 0; ++grp; }
+        }
+        // next unit: (tap, h, grp) count through the tile's slices, then the next tile of the clip / next clip
+        if (++tap == g.K) {
+          tap = 0;
+          if (++h == p.nh) { h = 0; ++grp; }
         }
         if (++s == p.S) {
           s = 0; h = 0; tap = 0; grp = 0;
@@ -392,7 +404,7 @@ fwd_sm100_kernel(const FwdParams p) {
       const long long xoff = *reinterpret_cast<const long long*>(rec_base_ptr + hdr_off);
       const int rows = *reinterpret_cast<const int*>(rec_base_ptr + hdr_off + 8);
       // dual: 16-byte chunks 4-7 of a row (channels 32-63 of the unit) belong to the second offset group
-      const uint8_t* rec_stage = rec_base_ptr + ((kDual && j >= 4) ? kRecBytes : 0);
+      const uint8_t* rec_stage = rec_base_ptr + ((kDual && !kShared && j >= 4) ? kRecBytes : 0);
       const int r = r0 + kRowStride * i;
       uint2 head = make_uint2(0u, 0u);
       if (r < rows) head = *reinterpret_cast<const uint2*>(rec_stage + r * 48);
@@ -406,9 +418,12 @@ fwd_sm100_kernel(const FwdParams p) {
     auto consume = [&](uint32_t k, int i, const uint4 (&c)[8], uint8_t* sd) {
       const uint8_t* rec_base_ptr = base_ptr + rec_off + (k % kRStages) * kRStage;
       const int rows = *reinterpret_cast<const int*>(rec_base_ptr + hdr_off + 8);
-      const uint8_t* rec_stage = rec_base_ptr + ((kDual && j >= 4) ? kRecBytes : 0);
+      const uint8_t* rec_stage = rec_base_ptr + ((kDual && !kShared && j >= 4) ? kRecBytes : 0);
       const uint32_t stage = a_base + (k % kAStages) * kAStageBytes;
       const int r = r0 + kRowStride * i;
+      float m = 1.f;
+      if constexpr (kShared)
+        m = r < rows ? *reinterpret_cast<const float*>(rec_base_ptr + kRecBytes + ((kDual && j >= 4) ? kMaskBytes : 0) + r * 4) : 0.f;
       if constexpr (kX3) {
         float w[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // rows past the clip end: stage bytes are stale
         if (r < rows) {
@@ -423,7 +438,7 @@ fwd_sm100_kernel(const FwdParams p) {
         // item j = channels 4j..4j+3: hi in 16-byte chunk j/2 (half j&1), lo in chunk 4 + j/2; the lane pair (j, j^1)
         // shares both chunks: the even lane writes the hi chunk, the odd lane the lo chunk
         const uint32_t row_base = stage + (uint32_t)((r >> 3) * 1024 + (r & 7) * 128);
-        const uint4 o = blend_split_store16(c, w, row_base + ((((j & 1) * 4 + (j >> 1)) ^ (r & 7)) << 4), (j & 1) != 0);
+        const uint4 o = blend_split_store16<kShared != 0>(c, w, row_base + ((((j & 1) * 4 + (j >> 1)) ^ (r & 7)) << 4), (j & 1) != 0, m);
         if constexpr (kSave) ptx::stg_v4_hint(sd, o, pol_stream);
       } else {
         uint4 w03 = make_uint4(0u, 0u, 0u, 0u), w47 = w03;       // rows past the clip end: stage bytes are stale
@@ -431,7 +446,7 @@ fwd_sm100_kernel(const FwdParams p) {
           w03 = *reinterpret_cast<const uint4*>(rec_stage + r * 48 + 16);
           w47 = *reinterpret_cast<const uint4*>(rec_stage + r * 48 + 32);
         }
-        const uint4 o = blend_store(c, w03, w47, stage + (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((j ^ (r & 7)) << 4)));
+        const uint4 o = blend_store<kShared != 0>(c, w03, w47, stage + (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((j ^ (r & 7)) << 4)), m);
         if constexpr (kSave) ptx::stg_v4_hint(sd, o, pol_stream);
       }
     };

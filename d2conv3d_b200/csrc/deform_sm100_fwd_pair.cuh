@@ -206,12 +206,12 @@ fwd_sm100_pair_kernel(const PairParams pp) {
       for (long long u = u_beg; u < u_end; ++u, ++k) {
         int s, b, v0; bool tile_ok;
         unit_tile(u, s, b, v0, tile_ok);
-        const int gt = s / p.nh, tap = gt % g.K, grp = gt / g.K;
+        const int gh = s / g.K, tap = s % g.K, grp = gh / p.nh;
         const int sr = k % kRStages;
         if (!ptx::mbar_wait(r_empty(sr), ((k / kRStages) & 1) ^ 1, abort_flag, 200)) break;
         const int rows = tile_ok ? min(kBM, g.V - v0) : 0;
         uint8_t* hdr = base_ptr + rec_off + sr * kRStageBytes + kRecBytes;
-        *reinterpret_cast<long long*>(hdr) = (long long)b * g.Vin * g.Cin + grp * g.cpg + (s % p.nh) * kBK;
+        *reinterpret_cast<long long*>(hdr) = (long long)b * g.Vin * g.Cin + grp * g.cpg + (gh % p.nh) * kBK;
         *reinterpret_cast<int*>(hdr + 8) = rows;
         if (tile_ok) {
           const uint32_t bytes = (uint32_t)rows * 48u;

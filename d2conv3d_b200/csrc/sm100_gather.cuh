@@ -21,6 +21,9 @@
 //        wj    = half2 {a_j*mask, a_j*mask}: trilinear weight x modulation, rounded to fp16, duplicated; ZERO
 //                for every corner that does not contribute to the forward sample.  In the fp32-parity mode
 //                the same 48 bytes hold {voff, steps, w0, w1}, w2..w5, {w6, w7, -, -} with fp32 weights.
+// A dilation field gives all offset groups the same positions: with more than one group its forward takes the record once per
+// (clip, tap, voxel), with the plain weights, and the activated modulation separately (fp32 [B][G][K][V padded to 4]), which the
+// producer multiplies the blended sample by.  Eight groups: 80 instead of 384 bytes written and read per tap and voxel.
 //   so a producer reads only the corners that weigh anything and blends all eight: what it holds for a corner it did not
 //   read is finite (zero, or a voxel of an earlier item -- the staging is kept finite), and its weight is zero.
 // Corners of zero weight are those outside the volume and, for a dilation field, the upper neighbour along every axis on which
@@ -39,12 +42,15 @@ namespace {
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ __half2 bits_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 
+// Row of the separate modulation values: 16-byte copies of any tile start on a boundary.
+__host__ __device__ inline int mask_row(int V) { return (V + 3) / 4 * 4; }
+
 // kShared: the coordinates do not depend on the offset group (dilation field): a thread serves one (voxel, tap)
 // and all groups, computing the position, corners and weights once and applying each group's modulation.
 template <typename Coords, bool kShared>
 static __global__ void __launch_bounds__(256)
 sample_records_kernel(Geom g, Coords coords, const float* __restrict__ mask, long long mask_bstride, int mask_act,
-                      float4* __restrict__ pos, uint4* __restrict__ gat, int f32_weights) {
+                      float4* __restrict__ pos, uint4* __restrict__ gat, int f32_weights, float* __restrict__ masks) {
   const int v = blockIdx.x * 256 + threadIdx.x;
   if (v >= g.V) return;
   const int tap = kShared ? blockIdx.y : blockIdx.y % g.K, b = blockIdx.z;
@@ -76,13 +82,15 @@ sample_records_kernel(Geom g, Coords coords, const float* __restrict__ mask, lon
                                                           ((long long)grp * g.K + tap) * g.V + v : i)))
                          : 1.f;
     if (pos) pos[i] = make_float4(z, y, x, m);
-    if (gat) {
-      uint4* o = gat + 3 * i;
+    if (masks) masks[(((long long)b * g.G + grp) * g.K + tap) * mask_row(g.V) + v] = m;
+    if (gat && (!masks || grp == grp_beg)) {
+      uint4* o = gat + 3 * (masks ? ((long long)b * g.K + tap) * g.V + v : i);
+      const float m_w = masks ? 1.f : m;
       if (f32_weights) {
         // fp32-parity mode: the 48 bytes hold the eight products a_j*mask in fp32
         uint32_t f[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] = ((valid >> j) & 1u) ? __float_as_uint(a[j] * m) : 0u;
+        for (int j = 0; j < 8; ++j) f[j] = ((valid >> j) & 1u) ? __float_as_uint(a[j] * m_w) : 0u;
         uint32_t weighs = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) weighs |= (f[j] << 1) ? 8u << j : 0u;      // +-0 alike
@@ -92,7 +100,7 @@ sample_records_kernel(Geom g, Coords coords, const float* __restrict__ mask, lon
       } else {
         uint32_t w[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) w[j] = ((valid >> j) & 1u) ? h2_bits(__float2half2_rn(a[j] * m)) : 0u;
+        for (int j = 0; j < 8; ++j) w[j] = ((valid >> j) & 1u) ? h2_bits(__float2half2_rn(a[j] * m_w)) : 0u;
         uint32_t weighs = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) weighs |= (w[j] & 0x7fffu) ? 8u << j : 0u;
@@ -111,12 +119,12 @@ struct CoordsSharedAcrossGroups<FieldCoords<T>> { static constexpr bool value = 
 
 template <typename Coords>
 static int launch_sample_records(const Geom& g, const Coords& coords, const float* mask, const HeadCfg& head, float4* pos,
-                                 uint4* gat, cudaStream_t st, bool f32_weights = false) {
+                                 uint4* gat, cudaStream_t st, bool f32_weights = false, float* masks = nullptr) {
   constexpr bool kShared = CoordsSharedAcrossGroups<Coords>::value;
   dim3 grid((unsigned)((g.V + 255) / 256), (unsigned)(kShared ? g.K : g.G * g.K), (unsigned)g.B);
   if (grid.y > 65535 || grid.z > 65535) return D2C_ERR_TOO_LARGE;
   sample_records_kernel<Coords, kShared><<<grid, 256, 0, st>>>(g, coords, mask, head.mask_bstride, head.mask_act, pos, gat,
-                                                              f32_weights ? 1 : 0);
+                                                              f32_weights ? 1 : 0, masks);
   D2C_LAUNCH_CHECK();
   return D2C_OK;
 }
@@ -154,7 +162,9 @@ __device__ __forceinline__ void load_corners(const __half* __restrict__ xb_ch, C
 }
 
 // Returns the 16 bytes it stored (a caller that also keeps the samples for the backward writes them to global).
-__device__ __forceinline__ uint4 blend_store(const uint4 (&c)[8], uint4 w03, uint4 w47, uint32_t dst) {
+// kScaled: the weights are plain, the sample is multiplied by m.
+template <bool kScaled = false>
+__device__ __forceinline__ uint4 blend_store(const uint4 (&c)[8], uint4 w03, uint4 w47, uint32_t dst, float m = 1.f) {
   const uint32_t w[8] = {w03.x, w03.y, w03.z, w03.w, w47.x, w47.y, w47.z, w47.w};
   __half2 acc[4];
 #pragma unroll
@@ -167,12 +177,14 @@ __device__ __forceinline__ uint4 blend_store(const uint4 (&c)[8], uint4 w03, uin
     acc[2] = __hfma2(bits_h2(c[j].z), wj, acc[2]);
     acc[3] = __hfma2(bits_h2(c[j].w), wj, acc[3]);
   }
-  uint4 out;
-  float2 f;
-  f = __half22float2(acc[0]); out.x = ptx::pack_bf16x2(f.x, f.y);
-  f = __half22float2(acc[1]); out.y = ptx::pack_bf16x2(f.x, f.y);
-  f = __half22float2(acc[2]); out.z = ptx::pack_bf16x2(f.x, f.y);
-  f = __half22float2(acc[3]); out.w = ptx::pack_bf16x2(f.x, f.y);
+  uint32_t o[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float2 f = __half22float2(acc[e]);
+    if constexpr (kScaled) { f.x *= m; f.y *= m; }
+    o[e] = ptx::pack_bf16x2(f.x, f.y);
+  }
+  const uint4 out = make_uint4(o[0], o[1], o[2], o[3]);
   ptx::sts_v4(dst, out);
   return out;
 }
@@ -222,8 +234,9 @@ __device__ __forceinline__ uint4 blend_split_store(const uint4 (&c)[8], const fl
 // lane both lo halves.  dst_chunk: shared-memory address of the 16-byte chunk THIS lane writes (hi chunk for an even
 // lane, lo chunk for an odd one).  Returns the 16 bytes stored.  Two 8-byte stores per lane cost 2.6x the
 // shared-memory wavefronts of this form (bank conflicts between the half-chunks of different rows).
+template <bool kScaled = false>
 __device__ __forceinline__ uint4 blend_split_store16(const uint4 (&c)[8], const float (&w)[8], uint32_t dst_chunk,
-                                                     bool odd_lane) {
+                                                     bool odd_lane, float m = 1.f) {
   float v[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
@@ -231,6 +244,10 @@ __device__ __forceinline__ uint4 blend_split_store16(const uint4 (&c)[8], const 
     v[1] = __fmaf_rn(__uint_as_float(c[j].y), w[j], v[1]);
     v[2] = __fmaf_rn(__uint_as_float(c[j].z), w[j], v[2]);
     v[3] = __fmaf_rn(__uint_as_float(c[j].w), w[j], v[3]);
+  }
+  if constexpr (kScaled) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] *= m;
   }
   const uint32_t h01 = ptx::pack_bf16x2(v[0], v[1]), h23 = ptx::pack_bf16x2(v[2], v[3]);
   const uint32_t l01 = ptx::pack_bf16x2(v[0] - ptx::bf16_lo(h01), v[1] - ptx::bf16_hi(h01));
