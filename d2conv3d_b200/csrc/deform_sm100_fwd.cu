@@ -26,10 +26,9 @@
 //   warp  6     one thread bulk-copies each unit's gather records into the record ring and writes the unit
 //               header (staging offset of the slice, valid rows), so the producers do no index arithmetic
 //   warp  7     idle (completes the warpgroup)
-//   warps 8-23  gather producers: unit header + gather record from the shared-memory record ring, 8
-//               unconditional corner loads (16 B) per row, the next row's loads issued before the current row is
-//               blended (setmaxnreg moves registers from warps 0-7 to these), blend with pre-modulated weights,
-//               bf16 pack, swizzled st.shared of the A tile
+//   warps 8-23  gather producers: unit header + gather record from the shared-memory record ring, 32 bytes of every corner
+//               that weighs anything, the next unit's loads issued half by half as the current unit's corners are blended
+//               (setmaxnreg moves registers from warps 0-7 to these), blend, bf16 pack, swizzled st.shared of the A tile
 // Stage hand-off is by mbarriers; every wait in the kernel's own code is bounded (sm100_ptx.cuh).
 //
 // Two math modes share the kernel (template parameter): single-pass bf16 (64-channel units, fp16 staging) and

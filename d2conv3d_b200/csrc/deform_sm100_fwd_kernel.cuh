@@ -386,124 +386,179 @@ fwd_sm100_kernel(const FwdParams p) {
   } else {
     // ===================== gather producers (software-pipelined) =====================
     asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
-    // A thread owns rows r0 and r0 + 64 of every unit, chunk j (16 B of the 128-byte A row).  Items are taken in
-    // the order (unit k, row 0), (unit k, row 1), (unit k+1, row 0) ...; the 8 corner loads of item t+1 are
-    // issued before item t is blended, so 8 loads are always in flight under the blend and 16 while it waits.
+    // A thread owns 32 bytes (a quarter) of one row's 128: 8 fp32 or 16 fp16 channels, so that one record, one header and
+    // eight addresses serve 32 bytes of every corner and a row's 16-byte chunks of the A tile need no exchange between lanes.
+    // The corners of unit k+1 are requested half by half (z floor, z ceil) as soon as the same half of unit k is blended:
+    // 64 registers of corners are all in flight while the thread waits, half of them under each blend.
+    // Bound by the load pipe (73 % busy at 512 channels, 8 x 30 x 54).  With 16 bytes of two rows per thread and unit, twice the
+    // records, addresses and waits, it took 1.40 ms at 512 channels, 2 x 8 x 30 x 54, now 1.33; 256-channel field layer, 2 x 8 x
+    // 60 x 107: 2.20 ms, now 1.88.
     const int t = threadIdx.x - kGatherWarp0Fwd * 32;
-    const int j = t & 7;             // 16-byte chunk (8 channels) of the 128-byte row
-    const int r0 = t >> 3;           // rows r0, r0 + kRowStride
+    const int j = t & 3;             // 32-byte quarter of the row
+    // the two rows of a quarter warp (one shared-memory store phase) differ in the bit that keeps their chunks apart:
+    // fp32-parity stores chunk j, then 4 + j (rows r and r + 4); single pass stores chunks 2j and 2j + 1 (rows r and r + 1)
+    const int rr = (t >> 2) & 7;
+    const int r = (t >> 5) * 8 + (kX3 ? (rr >> 1) | ((rr & 1) << 2) : rr);
     const uint32_t n_my_units = (uint32_t)part_tab[32];
-    bool ok = true;
-    // Samples kept for the weight gradient (p.sav != nullptr): the thread's two rows r0 and r0 + 64 are the same row
-    // of the two 64-voxel blocks of the tile, so its byte offset inside an 8 KB block is fixed.
-    const uint32_t sav_row = (uint32_t)((r0 >> 3) * 1024 + (r0 & 7) * 128);
+    const uint32_t row_off = (uint32_t)((r >> 3) * 1024 + (r & 7) * 128);
+    const uint32_t chunk0 = (uint32_t)(((kX3 ? j : 2 * j) ^ (r & 7)) << 4), chunk1 = (uint32_t)(((kX3 ? 4 + j : 2 * j + 1) ^ (r & 7)) << 4);
     const uint64_t pol_stream = ptx::l2_evict_first();
+    using XT = typename std::conditional<kX3 != 0, float, __half>::type;
+    // dual: the second half of a row (channels 32-63 of the unit) belongs to the second offset group
+    const int rec_row = r * 48 + ((kDual && !kShared && j >= 2) ? kRecBytes : 0);
 
-    auto issue = [&](uint32_t k, int i, uint4 (&c)[8]) {
-      const uint8_t* rec_base_ptr = base_ptr + rec_off + (k % kRStages) * kRStage;
-      const long long xoff = *reinterpret_cast<const long long*>(rec_base_ptr + hdr_off);
-      const int rows = *reinterpret_cast<const int*>(rec_base_ptr + hdr_off + 8);
-      // dual: 16-byte chunks 4-7 of a row (channels 32-63 of the unit) belong to the second offset group
-      const uint8_t* rec_stage = rec_base_ptr + ((kDual && !kShared && j >= 4) ? kRecBytes : 0);
-      const int r = r0 + kRowStride * i;
+    // unit k + 1: base address of the thread's corners, steps along the axes, corner bits, whether the row exists, image word
+    const XT* p0 = reinterpret_cast<const XT*>(p.x_cl);
+    int dx = 0, dy = 0, dz = 0, word_n = 0;
+    uint32_t bits = 0;
+    bool live_n = false;
+    auto locate = [&](uint32_t k) {
+      const uint8_t* st = base_ptr + rec_off + (k % kRStages) * kRStage;
+      const uint4 hdr = *reinterpret_cast<const uint4*>(st + hdr_off);         // {staging offset, rows, image word}
+      live_n = r < (int)hdr.z;
+      word_n = (int)hdr.w;
       uint2 head = make_uint2(0u, 0u);
-      if (r < rows) head = *reinterpret_cast<const uint2*>(rec_stage + r * 48);
-      if constexpr (kX3)
-        load_corners_f32(reinterpret_cast<const float*>(p.x_cl) + xoff + j * 4, p.cs, head.x, head.y, c);
-      else
-        load_corners(reinterpret_cast<const __half*>(p.x_cl) + xoff + j * 8, p.cs, head.x, head.y, c);
+      if (live_n) head = *reinterpret_cast<const uint2*>(st + rec_row);
+      bits = head.y;
+      dx = (bits & 1u) ? p.cs.dx : 0; dy = (bits & 2u) ? p.cs.dy : 0; dz = (bits & 4u) ? p.cs.dz : 0;
+      p0 = reinterpret_cast<const XT*>(p.x_cl) + (long long)(((uint64_t)hdr.y << 32) | hdr.x) + j * (kX3 ? 8 : 16) + head.x;
     };
-    // sd (kSave): where the 16 bytes this lane writes to the A tile (bf16x3: the lane pair's hi chunk or lo chunk) go
-    // in the kept image
-    auto consume = [&](uint32_t k, int i, const uint4 (&c)[8], uint8_t* sd) {
-      const uint8_t* rec_base_ptr = base_ptr + rec_off + (k % kRStages) * kRStage;
-      const int rows = *reinterpret_cast<const int*>(rec_base_ptr + hdr_off + 8);
-      const uint8_t* rec_stage = rec_base_ptr + ((kDual && !kShared && j >= 4) ? kRecBytes : 0);
-      const uint32_t stage = a_base + (k % kAStages) * kAStageBytes;
-      const int r = r0 + kRowStride * i;
-      float m = 1.f;
-      if constexpr (kShared)
-        m = r < rows ? *reinterpret_cast<const float*>(rec_base_ptr + kRecBytes + ((kDual && j >= 4) ? kMaskBytes : 0) + r * 4) : 0.f;
+    auto issue_half = [&](int z, uint32_t (&c)[4][8]) {
+      const XT* q = z ? p0 + dz : p0;
+      ptx::ldg_nc_v8_if(c[0], q, bits & (z ? 128u : 8u));
+      ptx::ldg_nc_v8_if(c[1], q + dx, bits & (z ? 256u : 16u));
+      ptx::ldg_nc_v8_if(c[2], q + dy, bits & (z ? 512u : 32u));
+      ptx::ldg_nc_v8_if(c[3], q + dy + dx, bits & (z ? 1024u : 64u));
+    };
+    // corner order 000..111, as the reference's interpolation chain; rows past the clip end have weight zero (their records
+    // are stale bytes)
+    uint64_t acc2[4];                // fp32-parity: 8 channels
+    __half2 acch[8];                 // single pass: 16 channels
+    auto blend_half = [&](int z, const uint8_t* rec, bool live, const uint32_t (&c)[4][8]) {
       if constexpr (kX3) {
-        float w[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // rows past the clip end: stage bytes are stale
-        if (r < rows) {
-          const uint2 w01 = *reinterpret_cast<const uint2*>(rec_stage + r * 48 + 8);
-          const uint4 w25 = *reinterpret_cast<const uint4*>(rec_stage + r * 48 + 16);
-          const uint2 w67 = *reinterpret_cast<const uint2*>(rec_stage + r * 48 + 32);
-          w[0] = __uint_as_float(w01.x); w[1] = __uint_as_float(w01.y);
-          w[2] = __uint_as_float(w25.x); w[3] = __uint_as_float(w25.y);
-          w[4] = __uint_as_float(w25.z); w[5] = __uint_as_float(w25.w);
-          w[6] = __uint_as_float(w67.x); w[7] = __uint_as_float(w67.y);
+        float w[4] = {0.f, 0.f, 0.f, 0.f};
+        if (live) {
+          const float2 a = *reinterpret_cast<const float2*>(rec + (z ? 24 : 8)), b = *reinterpret_cast<const float2*>(rec + (z ? 32 : 16));
+          w[0] = a.x; w[1] = a.y; w[2] = b.x; w[3] = b.y;
         }
-        // item j = channels 4j..4j+3: hi in 16-byte chunk j/2 (half j&1), lo in chunk 4 + j/2; the lane pair (j, j^1)
-        // shares both chunks: the even lane writes the hi chunk, the odd lane the lo chunk
-        const uint32_t row_base = stage + (uint32_t)((r >> 3) * 1024 + (r & 7) * 128);
-        const uint4 o = blend_split_store16<kShared != 0>(c, w, row_base + ((((j & 1) * 4 + (j >> 1)) ^ (r & 7)) << 4), (j & 1) != 0, m);
-        if constexpr (kSave) ptx::stg_v4_hint(sd, o, pol_stream);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint64_t w2;
+          asm("mov.b64 %0, {%1, %1};" : "=l"(w2) : "f"(w[q]));
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            uint64_t c2;
+            asm("mov.b64 %0, {%1, %2};" : "=l"(c2) : "r"(c[q][2 * e]), "r"(c[q][2 * e + 1]));
+            if (z == 0 && q == 0) acc2[e] = 0ull;
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc2[e]) : "l"(c2), "l"(w2));
+          }
+        }
       } else {
-        uint4 w03 = make_uint4(0u, 0u, 0u, 0u), w47 = w03;       // rows past the clip end: stage bytes are stale
-        if (r < rows) {
-          w03 = *reinterpret_cast<const uint4*>(rec_stage + r * 48 + 16);
-          w47 = *reinterpret_cast<const uint4*>(rec_stage + r * 48 + 32);
-        }
-        const uint4 o = blend_store<kShared != 0>(c, w03, w47, stage + (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((j ^ (r & 7)) << 4)), m);
-        if constexpr (kSave) ptx::stg_v4_hint(sd, o, pol_stream);
+        uint4 w = make_uint4(0u, 0u, 0u, 0u);
+        if (live) w = *reinterpret_cast<const uint4*>(rec + (z ? 32 : 16));
+        const uint32_t wq[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            if (z == 0 && q == 0) acch[e] = __float2half2_rn(0.f);
+            acch[e] = __hfma2(bits_h2(c[q][e]), bits_h2(wq[q]), acch[e]);
+          }
       }
     };
-
-    uint4 c0[8], c1[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) c0[q] = c1[q] = make_uint4(0u, 0u, 0u, 0u);
-    if (n_my_units > 0) {
-      ok = ptx::mbar_wait(r_full(0), 0, abort_flag);
-      if (ok) issue(0, 0, c0);
-    }
-    for (uint32_t k = 0; ok && k < n_my_units; ++k) {
-      const int sr = k % kRStages, sa = k % kAStages;
-      // where this lane's bytes of the unit go in the kept image: block = (tile, 64-voxel block, slice) in the
-      // single-pass mode; (tile, 64-voxel block, slice pair, {hi, lo}, slice of the pair) in the hi/lo mode, where a
-      // 64-channel row holds this unit's 32 channels in its half `half`, an even lane holds the hi chunk of the lane
-      // pair's 8 channels and an odd lane the lo chunk two blocks further.  The tile's second 64-voxel block (row 1 of
-      // this thread) lies sav_blk1 bytes further.
-      uint8_t* sav_dst = nullptr;
-      long long sav_blk1 = 0;
-      if constexpr (kSave) {
-        const int word = *reinterpret_cast<const int*>(base_ptr + rec_off + sr * kRStage + hdr_off + 12);
-        if constexpr (kX3) {
-          sav_dst = p.sav + ((long long)((word >> 1) + (j & 1) * 2) << 13) + sav_row +
-                    (uint32_t)(((4 * (word & 1) + (j >> 1)) ^ (r0 & 7)) << 4);
-          sav_blk1 = (long long)(p.sav_np * 4) << 13;
-        } else {
-          sav_dst = p.sav + ((long long)word << 13) + sav_row + (uint32_t)((j ^ (r0 & 7)) << 4);
-          sav_blk1 = (long long)(2 * p.sav_np) << 13;
-        }
-      }
 #ifdef D2C_UNIT_TRACE
-      const int trole = lane != 0 ? -1 : (warp == kGatherWarp0Fwd ? 3 : (warp == kGatherWarp0Fwd + 15 ? 4 : -1));
+    const int trole = lane != 0 ? -1 : (warp == kGatherWarp0Fwd ? 3 : (warp == kGatherWarp0Fwd + 15 ? 4 : -1));
 #define D2C_TG(e) do { if (trole >= 0) D2C_TR(trole, k, e); } while (0)
 #else
 #define D2C_TG(e) ((void)0)
 #endif
-      D2C_TG(0);
-      issue(k, 1, c1);
-      D2C_TG(1);
-      if (!ptx::mbar_wait(a_empty(sa), ((k / kAStages) & 1) ^ 1, abort_flag)) break;
-      D2C_TG(2);
-      consume(k, 0, c0, sav_dst);
-      D2C_TG(3);
-      if (k + 1 < n_my_units) {
-        if (!ptx::mbar_wait(r_full((k + 1) % kRStages), ((k + 1) / kRStages) & 1, abort_flag)) break;
-        D2C_TG(4);
-        issue(k + 1, 0, c0);
+
+    uint32_t c0[4][8], c1[4][8];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) c0[q][e] = c1[q][e] = 0u;
+    bool ok = true;
+    if (n_my_units > 0) {
+      ok = ptx::mbar_wait(r_full(0), 0, abort_flag);
+      if (ok) {
+        locate(0);
+        issue_half(0, c0);
+        issue_half(1, c1);
       }
+    }
+    for (uint32_t k = 0; ok && k < n_my_units; ++k) {
+      const int sr = k % kRStages, sa = k % kAStages;
+      const uint8_t* st = base_ptr + rec_off + sr * kRStage;
+      const uint8_t* rec = st + rec_row;
+      const bool live = live_n, more = k + 1 < n_my_units;
+      [[maybe_unused]] const int word = word_n;
+      D2C_TG(0);
+      blend_half(0, rec, live, c0);
+      D2C_TG(1);
+      if (more) {
+        if (!ptx::mbar_wait(r_full((k + 1) % kRStages), ((k + 1) / kRStages) & 1, abort_flag)) break;
+        D2C_TG(2);
+        locate(k + 1);
+        issue_half(0, c0);
+      }
+      D2C_TG(3);
+      blend_half(1, rec, live, c1);
+      if (more) issue_half(1, c1);
+      D2C_TG(4);
+      float m = 1.f;
+      if constexpr (kShared) m = live ? *reinterpret_cast<const float*>(st + kRecBytes + ((kDual && j >= 2) ? kMaskBytes : 0) + r * 4) : 0.f;
+      uint4 o0, o1;                  // chunk0, chunk1
+      if constexpr (kX3) {
+        uint32_t h[4], l[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float v0, v1;
+          asm("mov.b64 {%0, %1}, %2;" : "=f"(v0), "=f"(v1) : "l"(acc2[e]));
+          if constexpr (kShared) { v0 *= m; v1 *= m; }
+          h[e] = ptx::pack_bf16x2(v0, v1);
+          l[e] = ptx::pack_bf16x2(v0 - ptx::bf16_lo(h[e]), v1 - ptx::bf16_hi(h[e]));
+        }
+        o0 = make_uint4(h[0], h[1], h[2], h[3]);
+        o1 = make_uint4(l[0], l[1], l[2], l[3]);
+      } else {
+        uint32_t o[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          float2 f = __half22float2(acch[e]);
+          if constexpr (kShared) { f.x *= m; f.y *= m; }
+          o[e] = ptx::pack_bf16x2(f.x, f.y);
+        }
+        o0 = make_uint4(o[0], o[1], o[2], o[3]);
+        o1 = make_uint4(o[4], o[5], o[6], o[7]);
+      }
+      if (!ptx::mbar_wait(a_empty(sa), ((k / kAStages) & 1) ^ 1, abort_flag)) break;
       D2C_TG(5);
-      consume(k, 1, c1, sav_dst + sav_blk1);
+      const uint32_t row = a_base + sa * kAStageBytes + row_off;
+      ptx::sts_v4(row + chunk0, o0);
+      ptx::sts_v4(row + chunk1, o1);
       D2C_TG(6);
       ptx::fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
         ptx::mbar_arrive(a_full(sa));
         ptx::mbar_arrive(r_empty(sr));
+      }
+      if constexpr (kSave) {
+        // where the thread's bytes go in the kept image: block = (tile, 64-voxel block, slice) in the single-pass mode;
+        // (tile, 64-voxel block, slice pair, {hi, lo}, slice of the pair) in the hi/lo mode, where a 64-channel row holds this
+        // unit's 32 channels in its half `word & 1`, and the lo block lies two blocks further
+        const uint32_t in_blk = row_off & 8191u;
+        if constexpr (kX3) {
+          uint8_t* sd = p.sav + ((long long)((word >> 1) + (r >> 6) * p.sav_np * 4) << 13) + in_blk +
+                        (uint32_t)(((4 * (word & 1) + j) ^ (r & 7)) << 4);
+          ptx::stg_v4_hint(sd, o0, pol_stream);
+          ptx::stg_v4_hint(sd + (2 << 13), o1, pol_stream);
+        } else {
+          uint8_t* sd = p.sav + ((long long)(word + (r >> 6) * 2 * p.sav_np) << 13) + in_blk;
+          ptx::stg_v4_hint(sd + chunk0, o0, pol_stream);
+          ptx::stg_v4_hint(sd + chunk1, o1, pol_stream);
+        }
       }
       D2C_TG(7);
     }

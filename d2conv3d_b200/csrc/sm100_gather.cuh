@@ -162,9 +162,7 @@ __device__ __forceinline__ void load_corners(const __half* __restrict__ xb_ch, C
 }
 
 // Returns the 16 bytes it stored (a caller that also keeps the samples for the backward writes them to global).
-// kScaled: the weights are plain, the sample is multiplied by m.
-template <bool kScaled = false>
-__device__ __forceinline__ uint4 blend_store(const uint4 (&c)[8], uint4 w03, uint4 w47, uint32_t dst, float m = 1.f) {
+__device__ __forceinline__ uint4 blend_store(const uint4 (&c)[8], uint4 w03, uint4 w47, uint32_t dst) {
   const uint32_t w[8] = {w03.x, w03.y, w03.z, w03.w, w47.x, w47.y, w47.z, w47.w};
   __half2 acc[4];
 #pragma unroll
@@ -180,8 +178,7 @@ __device__ __forceinline__ uint4 blend_store(const uint4 (&c)[8], uint4 w03, uin
   uint32_t o[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    float2 f = __half22float2(acc[e]);
-    if constexpr (kScaled) { f.x *= m; f.y *= m; }
+    const float2 f = __half22float2(acc[e]);
     o[e] = ptx::pack_bf16x2(f.x, f.y);
   }
   const uint4 out = make_uint4(o[0], o[1], o[2], o[3]);
@@ -227,37 +224,6 @@ __device__ __forceinline__ uint4 blend_split_store(const uint4 (&c)[8], const fl
   ptx::sts_v2(dst_hi, make_uint2(h01, h23));
   ptx::sts_v2(dst_lo, make_uint2(l01, l23));
   return make_uint4(h01, h23, l01, l23);
-}
-
-// The same item written with ONE 16-byte store per lane: lanes 2i and 2i+1 of a warp hold neighbouring 4-channel
-// items of the same row, so the even lane takes both hi halves (one 16-byte chunk of the row's hi part) and the odd
-// lane both lo halves.  dst_chunk: shared-memory address of the 16-byte chunk THIS lane writes (hi chunk for an even
-// lane, lo chunk for an odd one).  Returns the 16 bytes stored.  Two 8-byte stores per lane cost 2.6x the
-// shared-memory wavefronts of this form (bank conflicts between the half-chunks of different rows).
-template <bool kScaled = false>
-__device__ __forceinline__ uint4 blend_split_store16(const uint4 (&c)[8], const float (&w)[8], uint32_t dst_chunk,
-                                                     bool odd_lane, float m = 1.f) {
-  float v[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    v[0] = __fmaf_rn(__uint_as_float(c[j].x), w[j], v[0]);
-    v[1] = __fmaf_rn(__uint_as_float(c[j].y), w[j], v[1]);
-    v[2] = __fmaf_rn(__uint_as_float(c[j].z), w[j], v[2]);
-    v[3] = __fmaf_rn(__uint_as_float(c[j].w), w[j], v[3]);
-  }
-  if constexpr (kScaled) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] *= m;
-  }
-  const uint32_t h01 = ptx::pack_bf16x2(v[0], v[1]), h23 = ptx::pack_bf16x2(v[2], v[3]);
-  const uint32_t l01 = ptx::pack_bf16x2(v[0] - ptx::bf16_lo(h01), v[1] - ptx::bf16_hi(h01));
-  const uint32_t l23 = ptx::pack_bf16x2(v[2] - ptx::bf16_lo(h23), v[3] - ptx::bf16_hi(h23));
-  // even lane gives its lo and receives the odd lane's hi; the odd lane the other way round
-  const uint32_t t0 = __shfl_xor_sync(0xffffffffu, odd_lane ? h01 : l01, 1);
-  const uint32_t t1 = __shfl_xor_sync(0xffffffffu, odd_lane ? h23 : l23, 1);
-  const uint4 out = odd_lane ? make_uint4(t0, t1, l01, l23) : make_uint4(h01, h23, t0, t1);
-  ptx::sts_v4(dst_chunk, out);
-  return out;
 }
 
 }  // namespace
