@@ -244,7 +244,7 @@ PHASE_WORK = {
     "bwd_dcol_sm100": ("tensor", "F"), "bwd_dcol_generic": ("tensor", "F"),
     "bwd_dw_sm100": ("tensor", "F"), "bwd_dw_sm100_saved": ("tensor", "F"), "bwd_dw_generic": ("tensor", "F"),
     "bwd_sample_grad": ("hbm", "sample_grad_bytes"),
-    "bwd_coord_grad_generic": ("hbm", "coord_bytes"), "bwd_col2im_generic": ("hbm", "col2im_bytes"),
+    "bwd_sample_grad_generic": ("hbm", "coord_bytes"),
 }
 
 
@@ -367,10 +367,9 @@ def run_gpu_arm(args, impl="ours"):
     F = fwd_flops(wl["B"], wl["Cin"], wl["Cout"], V, 27)
     s = 4
     coord_bytes = s * (wl["B"] * wl["Cin"] * 27 * V + wl["B"] * wl["Cin"] * V + 2 * wl["B"] * wl["G"] * 4 * 27 * V)
-    col2im_bytes = s * (wl["B"] * wl["Cin"] * 27 * V + wl["B"] * wl["G"] * 4 * 27 * V + wl["B"] * wl["Cin"] * V)
     # fused offset/mask-gradient + scatter: dcol read once, x read, offsets+mask read, their gradients and grad_x written
     sample_grad_bytes = s * (wl["B"] * wl["Cin"] * 27 * V + 2 * wl["B"] * wl["Cin"] * V + 2 * wl["B"] * wl["G"] * 4 * 27 * V)
-    work = {"F": F, "coord_bytes": coord_bytes, "col2im_bytes": col2im_bytes, "sample_grad_bytes": sample_grad_bytes}
+    work = {"F": F, "coord_bytes": coord_bytes, "sample_grad_bytes": sample_grad_bytes}
 
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)      # 256 MB > 126 MB L2
     s_main = torch.cuda.current_stream()
