@@ -582,24 +582,26 @@ dw_saved_sm100_kernel(const DwSavedParams p) {
 }
 
 // dws [(slice, c)][co] -> grad_w [co][cin][tap]   (cin = grp*cpg + h*64 + c)
+// Block: nc channels of one (group, 64-channel slice) with all their taps (at most 256 rows), 32 output channels, so that it
+// writes runs of nc * K floats.  32 x 32 tiles wrote single floats K apart: 512 x 512 channels, 27 taps, 44 us, now 25.
+constexpr int kUnstageRows = 256;
 __global__ void __launch_bounds__(256)
-unstage_dw_kernel(int Cout, int Cin, int K, int cpg, int nh, int S, const float* __restrict__ dws,
-                  float* __restrict__ grad_w) {
-  __shared__ float tile[32][33];
-  const int r0 = blockIdx.x * 32, co0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int rr = ty; rr < 32; rr += 8) {
-    const int r = r0 + rr;
-    tile[rr][tx] = (r < S * 64 && co0 + tx < Cout) ? __ldg(dws + (long long)r * Cout + co0 + tx) : 0.f;
+unstage_dw_kernel(int Cout, int Cin, int K, int cpg, int nh, int log_nc, const float* __restrict__ dws, float* __restrict__ grad_w) {
+  __shared__ float tile[kUnstageRows][33];
+  const int nc = 1 << log_nc, blocks_c = 64 >> log_nc, cb = blockIdx.x % blocks_c * nc, gh = blockIdx.x / blocks_c, h = gh % nh, grp = gh / nh;
+  const int co0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5, rows = nc * K;
+#pragma unroll 8
+  for (int i = ty; i < rows; i += 8) {             // i = tap * nc + c: neighbouring rows of dws
+    const int tap = i >> log_nc, c = i & (nc - 1);
+    const long long r = ((long long)(grp * K + tap) * nh + h) * 64 + cb + c;
+    if (co0 + tx < Cout) tile[c * K + tap][tx] = __ldg(dws + r * Cout + co0 + tx);
   }
   __syncthreads();
   for (int cc = ty; cc < 32; cc += 8) {
-    const int r = r0 + tx, co = co0 + cc;
-    if (r < S * 64 && co < Cout) {
-      const int c = r & 63, s = r >> 6;
-      const int h = s % nh, gt = s / nh, tap = gt % K, grp = gt / K;
-      grad_w[((long long)co * Cin + grp * cpg + h * 64 + c) * K + tap] = tile[tx][cc];
-    }
+    const int co = co0 + cc;
+    if (co >= Cout) break;
+    float* dst = grad_w + ((long long)co * Cin + grp * cpg + h * 64 + cb) * K;
+    for (int i = tx; i < rows; i += 32) dst[i] = tile[i][cc];
   }
 }
 
@@ -755,8 +757,12 @@ int sm100_dw(const Geom& g, bool x3, const float* gy, const void* x_cl, const vo
     D2C_LAUNCH_CHECK();
   }
   prof_mark(st, "bwd_dw_unstage");
-  unstage_dw_kernel<<<dim3((unsigned)((dp.S * 64 + 31) / 32), (unsigned)((g.Cout + 31) / 32)), 256, 0, st>>>(
-      g.Cout, g.Cin, g.K, dp.pairg ? kBK : g.cpg, dp.nh, dp.S, dws, grad_w);
+  // K <= 192 (make_bwd_plan): at least one channel; fewer than fit where multiprocessors would be left without a block
+  int log_nc = 6;
+  while (log_nc > 0 && ((g.K << log_nc) > kUnstageRows ||
+                        (long long)(dp.S / g.K) * (64 >> log_nc) * ((g.Cout + 31) / 32) < 2LL * sm_count)) --log_nc;
+  unstage_dw_kernel<<<dim3((unsigned)(dp.S / g.K * (64 >> log_nc)), (unsigned)((g.Cout + 31) / 32)), 256, 0, st>>>(
+      g.Cout, g.Cin, g.K, dp.pairg ? kBK : g.cpg, dp.nh, log_nc, dws, grad_w);
   D2C_LAUNCH_CHECK();
   return D2C_OK;
 }

@@ -353,16 +353,13 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
   prof_mark(st, "fwd_stage_operands");
   {
     const ZeroFill zero_y{y, whole_tiles_only ? 0 : (long long)sizeof(float) * g.B * g.Cout * g.V};
-    dim3 sgrid((unsigned)((g.Vin + 31) / 32), (unsigned)((g.Cin + 63) / 64), (unsigned)g.B);
     if (x3) {
-      stage_input_cl_f32_kernel<<<sgrid, 256, 0, st>>>(g.Cin, g.Vin, x, reinterpret_cast<float*>(x_cl), zero_y);
-      D2C_LAUNCH_CHECK();
+      if ((rc = launch_stage_input(g, x, reinterpret_cast<float*>(x_cl), zero_y, sm_count, st))) return rc;
       dim3 wgrid((unsigned)g.Cout, (unsigned)(g.Cin / 32));
       stage_weight_sw128_x3_kernel<<<wgrid, 64, 32 * g.K * sizeof(float), st>>>(g.Cout, g.Cin, g.K, g.cpg, pl.nh, w, w_sw);
       D2C_LAUNCH_CHECK();
     } else {
-      stage_input_cl_f16_kernel<<<sgrid, 256, 0, st>>>(g.Cin, g.Vin, x, reinterpret_cast<__half*>(x_cl), zero_y);
-      D2C_LAUNCH_CHECK();
+      if ((rc = launch_stage_input(g, x, reinterpret_cast<__half*>(x_cl), zero_y, sm_count, st))) return rc;
       dim3 wgrid((unsigned)g.Cout, (unsigned)(g.Cin / 64));
       stage_weight_sw128_kernel<<<wgrid, 64, 64 * g.K * sizeof(float), st>>>(g.Cout, g.Cin, g.K,
                                                                               pl.dual ? 64 : g.cpg, pl.nh, w, w_sw);
