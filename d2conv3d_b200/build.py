@@ -12,6 +12,7 @@ autograd nodes and argument handling over the library's C ABI).  A GPU is not ne
 to build either.
 """
 import os
+import re
 import subprocess
 import sys
 
@@ -91,7 +92,7 @@ def build(force=False, verbose=False, unit_trace=False):
         build_torch()
         return LIB
     os.makedirs(OBJ_DIR, exist_ok=True)
-    extra = (["-Xptxas", "-v"] if verbose else []) + (["-DD2C_UNIT_TRACE"] if unit_trace else [])
+    extra = ["-Xptxas", "-v"] + (["-DD2C_UNIT_TRACE"] if unit_trace else [])
     procs = []
     objs = []
     for src in SOURCES:
@@ -102,6 +103,8 @@ def build(force=False, verbose=False, unit_trace=False):
     failed = False
     for src, p in procs:
         out, _ = p.communicate()
+        with open(os.path.join(OBJ_DIR, src.replace(".cu", ".ptxas")), "w") as f:
+            f.write(out)
         if p.returncode != 0 or verbose:
             sys.stderr.write(f"--- {src} ---\n{out}\n")
         failed |= p.returncode != 0
@@ -111,6 +114,23 @@ def build(force=False, verbose=False, unit_trace=False):
     subprocess.run(cmd, check=True)
     build_torch(force)
     return LIB
+
+
+def ptxas_report():
+    """{mangled kernel name: (registers, bytes of stack, of spill stores, of spill loads)} of the last build here; kernels of
+    sources whose report is missing are absent."""
+    out = {}
+    for src in SOURCES:
+        path = os.path.join(OBJ_DIR, src.replace(".cu", ".ptxas"))
+        if not os.path.exists(path):
+            continue
+        with open(path) as f:
+            text = f.read()
+        for name, stack, stores, loads, regs in re.findall(
+                r"Compiling entry function '(\w+)'.*?(\d+) bytes stack frame, (\d+) bytes spill stores, (\d+) bytes spill loads"
+                r".*?Used (\d+) registers", text, re.S):
+            out[name] = (int(regs), int(stack), int(stores), int(loads))
+    return out
 
 
 def build_microbench():

@@ -561,9 +561,12 @@ sample_grad_taps_kernel(Geom g, ClStrides cs, int b0, int nh, const float4* __re
     const float wx[2] = {sub_rn(1.f, s.fx), sub_rn(1.f, s.gx)};
     const bool okz[2] = {true, s.gz < 1.f}, oky[2] = {true, s.gy < 1.f}, okx[2] = {true, s.gx < 1.f};
     unsigned valid = active ? s.valid : 0u;
-    if constexpr (FieldOut) {
+    if constexpr (FieldOut && (kF32X || !kNarrow)) {
       // A tap at the kernel's centre on an axis does not move along it: the upper corners of that axis weigh nothing and the
-      // axis takes no gradient, so they are not read (4.6 corners a tap instead of 8 with 3 x 3 x 3 taps).
+      // axis takes no gradient, so they are not read (4.6 corners a tap instead of 8 with 3 x 3 x 3 taps).  Not where a thread
+      // has 4 channels of fp16: it issues its loads either way (a corner left out reads the stand-in below), and finding out
+      // which to leave out costs it more than the cache hits give back and its registers spill.  256 channels, bf16 mode: 8
+      // groups on 8 x 120 x 214 9.13 ms with the skip, 8.15 without; one group (8 channels a thread) on 2 x 8 x 60 x 107 2.03 and 2.07.
       const int k = tap % g.kw, jj = (tap / g.kw) % g.kh, i = tap / (g.kw * g.kh);
       if (field_axes.pos[0][i] == 0.f && !okz[1]) valid &= 0x0fu;
       if (field_axes.pos[1][jj] == 0.f && !oky[1]) valid &= 0x33u;
