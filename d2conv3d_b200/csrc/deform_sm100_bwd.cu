@@ -817,8 +817,8 @@ int run_bwd(const Geom& g, bool x3, const Coords& coords, unsigned long long cap
     }
   }
   if (!sav) {
-    rc = x3 ? launch_stage_input(g, x, reinterpret_cast<float*>(x_cl), ZeroFill{nullptr, 0}, sm_count, st)
-            : launch_stage_input(g, x, reinterpret_cast<__half*>(x_cl), ZeroFill{nullptr, 0}, sm_count, st);
+    rc = x3 ? launch_stage_input(g, x, reinterpret_cast<float*>(x_cl), ZeroFill{nullptr, 0}, nullptr, sm_count, st)
+            : launch_stage_input(g, x, reinterpret_cast<__half*>(x_cl), ZeroFill{nullptr, 0}, nullptr, sm_count, st);
     if (rc) return rc;
     if (!sav && (rc = launch_sample_records(g, coords, mask, head, recs, gat, st, x3))) return rc;
   }

@@ -302,10 +302,6 @@ dw_sm100_kernel(const DwParams p) {
         row_dst[i] = (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((j ^ (r & 7)) << 4));
       }
       uint4 c[kRowsPerThread][8];
-#pragma unroll
-      for (int i = 0; i < kRowsPerThread; ++i)
-#pragma unroll
-        for (int e = 0; e < 8; ++e) c[i][e] = make_uint4(0u, 0u, 0u, 0u);
       const int nq = 2 * n_my_tiles;
       for (int q = 0; q < nq; ++q) {
         const int t = q >> 1, sl = q & 1, sa = t % kAStages, sr = q % kRStages;

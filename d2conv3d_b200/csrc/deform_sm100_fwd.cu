@@ -76,12 +76,15 @@ constexpr int kMinUnitsPerCta = 4;
 // ... and for which the units of a call are cut clip by clip (cta_part_range): every part ends in a partial tile.
 constexpr int kMinUnitsPerPart = 64;
 
+constexpr size_t kFlagBytes = 256;                // workspace of the NaN flag, a whole alignment unit
+
 struct FwdParams {
   Geom g;
   const void* x_cl;            // [B][Vin][Cin] channels-last staging of x: fp16 (bf16 mode) or fp32 (bf16x3 mode)
   const uint8_t* w_sw;         // [S][N rows x 128 B], rows swizzled exactly as the smem B tile
   const uint4* recs;           // [B][G][K][V] gather records (3 x uint4 each, sm100_gather.cuh), or
   const float* masks;          // [B][K][V] records and [B][G][K][V padded] modulation values
+  const int* nan_flag;         // whether x holds a NaN (sm100_stage.cuh)
   const float* bias;           // [Cout] or nullptr
   float* y;                    // [B, Cout, V]
   ClStrides cs;
@@ -214,7 +217,7 @@ bool make_plan(const Geom& g, bool x3, Plan* pl, bool shared = false) {
   if ((long long)pl->n_tiles * pl->S > 0x7fffffffLL) return false;   // the kernel counts units in 31 bits
   pl->w_slice_bytes = g.Cout * 128;
   pl->b_stage_bytes = (g.Cout < 256 ? g.Cout : 256) * 128;
-  // 256 bytes of barriers + 272 bytes of part ranges (rounded to 512) + 1 KB of alignment slack
+  // 256 bytes of barriers + 132 bytes of part ranges (rounded to 512) + 1 KB of alignment slack
   const int other = 1024 + 768 + kAStages * kAStageBytes + kRStages * pl->r_stage_bytes;
   int nb = (kSmemGather - other) / pl->b_stage_bytes;
   if (nb > 4) nb = 4;
@@ -272,6 +275,7 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
   uint8_t* wsp = reinterpret_cast<uint8_t*>(ws);
   void* x_cl = wsp; wsp += pl.x_cl_bytes;
   uint8_t* w_sw = wsp; wsp += pl.w_sw_bytes;
+  int* nan_flag = reinterpret_cast<int*>(wsp); wsp += kFlagBytes;
   uint4* recs = reinterpret_cast<uint4*>(wsp);
   // A bound sample cache that is large enough takes the operand tiles (written by the kernel), and the staged input
   // and the position records move into it, so that the backward of this call stages nothing a second time.
@@ -352,24 +356,24 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
   if (pair_clusters > 0) { sav = nullptr; pos = nullptr; x_cl = ws; }       // the CTA-pair kernel keeps nothing
   prof_mark(st, "fwd_stage_operands");
   {
+    if ((rc = launch_sample_records(g, coords, mask, head, pos, recs, st, x3, masks, nan_flag))) return rc;
     const ZeroFill zero_y{y, whole_tiles_only ? 0 : (long long)sizeof(float) * g.B * g.Cout * g.V};
     if (x3) {
-      if ((rc = launch_stage_input(g, x, reinterpret_cast<float*>(x_cl), zero_y, sm_count, st))) return rc;
+      if ((rc = launch_stage_input(g, x, reinterpret_cast<float*>(x_cl), zero_y, nan_flag, sm_count, st))) return rc;
       dim3 wgrid((unsigned)g.Cout, (unsigned)(g.Cin / 32));
       stage_weight_sw128_x3_kernel<<<wgrid, 64, 32 * g.K * sizeof(float), st>>>(g.Cout, g.Cin, g.K, g.cpg, pl.nh, w, w_sw);
       D2C_LAUNCH_CHECK();
     } else {
-      if ((rc = launch_stage_input(g, x, reinterpret_cast<__half*>(x_cl), zero_y, sm_count, st))) return rc;
+      if ((rc = launch_stage_input(g, x, reinterpret_cast<__half*>(x_cl), zero_y, nan_flag, sm_count, st))) return rc;
       dim3 wgrid((unsigned)g.Cout, (unsigned)(g.Cin / 64));
       stage_weight_sw128_kernel<<<wgrid, 64, 64 * g.K * sizeof(float), st>>>(g.Cout, g.Cin, g.K,
                                                                               pl.dual ? 64 : g.cpg, pl.nh, w, w_sw);
       D2C_LAUNCH_CHECK();
     }
-    if ((rc = launch_sample_records(g, coords, mask, head, pos, recs, st, x3, masks))) return rc;
   }
 
   FwdParams p;
-  p.g = g; p.x_cl = x_cl; p.w_sw = w_sw; p.recs = recs; p.masks = masks; p.bias = bias; p.y = y;
+  p.g = g; p.x_cl = x_cl; p.w_sw = w_sw; p.recs = recs; p.masks = masks; p.nan_flag = nan_flag; p.bias = bias; p.y = y;
   p.cs.dz = g.H * g.W * g.Cin; p.cs.dy = g.W * g.Cin; p.cs.dx = g.Cin;
   p.N = g.Cout; p.nh = pl.nh; p.S = pl.S; p.tiles_per_clip = pl.tiles_per_clip; p.n_tiles = pl.n_tiles;
   p.n_units = n_units;
@@ -454,7 +458,7 @@ size_t sm100_fwd_workspace(const Geom& g, int dtype, int math_mode) {
   bool x3;
   Plan pl;
   pick_variant(g, math_mode, &x3, &pl);
-  return pl.x_cl_bytes + pl.w_sw_bytes + pl.rec_bytes;
+  return pl.x_cl_bytes + pl.w_sw_bytes + kFlagBytes + pl.rec_bytes;
 }
 
 int sm100_fwd_offsets(const Geom& g, int math_mode, const float* x, const float* offset, const float* mask,

@@ -487,6 +487,11 @@ fwd_sm100_kernel(const FwdParams p) {
         issue_half(1, c1);
       }
     }
+    // Corners that weigh nothing are not read, and blended with weight zero: their registers hold zero or a corner of an earlier
+    // unit, of which only a NaN would show.  Where x holds a NaN they are cleared, in a loop of its own.  256 channels, field
+    // layer of one group, 2 x 8 x 60 x 107, inference, without / with that / always cleared / cleared where a blended sample is
+    // NaN: 1.371 / 1.377 / 1.495 / 1.404 ms; as a branch in one loop 1.383.
+    auto work = [&](auto clear) {
     for (uint32_t k = 0; ok && k < n_my_units; ++k) {
       const int sr = k % kRStages, sa = k % kAStages;
       const uint8_t* st = base_ptr + rec_off + sr * kRStage;
@@ -506,6 +511,13 @@ fwd_sm100_kernel(const FwdParams p) {
       blend_half(1, rec, live, c1);
       if (more) issue_half(1, c1);
       D2C_TG(4);
+      if constexpr (clear) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (!(bits & (8u << q))) ptx::clear_v8(c0[q]);
+          if (!(bits & (128u << q))) ptx::clear_v8(c1[q]);
+        }
+      }
       float m = 1.f;
       if constexpr (kShared) m = live ? *reinterpret_cast<const float*>(st + kRecBytes + ((kDual && j >= 2) ? kMaskBytes : 0) + r * 4) : 0.f;
       uint4 o0, o1;                  // chunk0, chunk1
@@ -562,6 +574,9 @@ fwd_sm100_kernel(const FwdParams p) {
       }
       D2C_TG(7);
     }
+    };
+    if (__ldg(p.nan_flag)) work(std::true_type{});
+    else work(std::false_type{});
   }
 
   // ---- teardown ----

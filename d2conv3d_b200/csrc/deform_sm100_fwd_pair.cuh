@@ -244,10 +244,6 @@ fwd_sm100_pair_kernel(const PairParams pp) {
                                               ptx::mapa_shared(a_full(2), 0), ptx::mapa_shared(a_full(3), 0)};
     const uint32_t n_my_units = (uint32_t)(u_end - u_beg);
     uint4 c[kRowsPerThread][8];
-#pragma unroll
-    for (int i = 0; i < kRowsPerThread; ++i)
-#pragma unroll
-      for (int q = 0; q < 8; ++q) c[i][q] = make_uint4(0u, 0u, 0u, 0u);
     for (uint32_t k = 0; k < n_my_units; ++k) {
       const int sr = k % kRStages, sa = k % kAStages;
       if (!ptx::mbar_wait(r_full(sr), (k / kRStages) & 1, abort_flag)) break;

@@ -24,8 +24,11 @@
 // A dilation field gives all offset groups the same positions: with more than one group its forward takes the record once per
 // (clip, tap, voxel), with the plain weights, and the activated modulation separately (fp32 [B][G][K][V padded to 4]), which the
 // producer multiplies the blended sample by.  Eight groups: 80 instead of 384 bytes written and read per tap and voxel.
-//   so a producer reads only the corners that weigh anything and blends all eight: what it holds for a corner it did not
-//   read is finite (zero, or a voxel of an earlier item -- the staging is kept finite), and its weight is zero.
+// A producer reads only the corners that weigh anything and blends all eight, the others as zero: zero times their weight, where
+// what a register held before may be a NaN of another voxel, tile or clip.  The 16-byte gathers clear a register before each
+// load (256 channels in 8 groups on 2 x 8 x 60 x 107, bf16: weight gradient that gathers 0.97 ms; 1.19 with registers that kept
+// their contents from item to item, which spilled).  The forward, whose 32-byte gathers have a register file's worth in flight,
+// clears them only where the staged input holds a NaN (deform_sm100_fwd_kernel.cuh).
 // Corners of zero weight are those outside the volume and, for a dilation field, the upper neighbour along every axis on which
 // the tap sits at the kernel's centre: 4.6 corners a tap instead of 8 with 3 x 3 x 3 taps.  The forward of such a layer, 256
 // channels on 2 x 8 x 60 x 107, takes 2.27 ms instead of 2.71; with free offsets the corners outside the volume give 512 channels on 2 x 8 x 30 x 54 1.55 instead of 1.68.
@@ -47,11 +50,14 @@ __host__ __device__ inline int mask_row(int V) { return (V + 3) / 4 * 4; }
 
 // kShared: the coordinates do not depend on the offset group (dilation field): a thread serves one (voxel, tap)
 // and all groups, computing the position, corners and weights once and applying each group's modulation.
+// nan_flag (nullable): cleared on the side for the staging kernel that follows.
 template <typename Coords, bool kShared>
 static __global__ void __launch_bounds__(256)
 sample_records_kernel(Geom g, Coords coords, const float* __restrict__ mask, long long mask_bstride, int mask_act,
-                      float4* __restrict__ pos, uint4* __restrict__ gat, int f32_weights, float* __restrict__ masks) {
+                      float4* __restrict__ pos, uint4* __restrict__ gat, int f32_weights, float* __restrict__ masks,
+                      int* __restrict__ nan_flag) {
   const int v = blockIdx.x * 256 + threadIdx.x;
+  if (nan_flag && v == 0 && blockIdx.y == 0 && blockIdx.z == 0) *nan_flag = 0;
   if (v >= g.V) return;
   const int tap = kShared ? blockIdx.y : blockIdx.y % g.K, b = blockIdx.z;
   const int grp_beg = kShared ? 0 : blockIdx.y / g.K, grp_end = kShared ? g.G : grp_beg + 1;
@@ -119,12 +125,13 @@ struct CoordsSharedAcrossGroups<FieldCoords<T>> { static constexpr bool value = 
 
 template <typename Coords>
 static int launch_sample_records(const Geom& g, const Coords& coords, const float* mask, const HeadCfg& head, float4* pos,
-                                 uint4* gat, cudaStream_t st, bool f32_weights = false, float* masks = nullptr) {
+                                 uint4* gat, cudaStream_t st, bool f32_weights = false, float* masks = nullptr,
+                                 int* nan_flag = nullptr) {
   constexpr bool kShared = CoordsSharedAcrossGroups<Coords>::value;
   dim3 grid((unsigned)((g.V + 255) / 256), (unsigned)(kShared ? g.K : g.G * g.K), (unsigned)g.B);
   if (grid.y > 65535 || grid.z > 65535) return D2C_ERR_TOO_LARGE;
   sample_records_kernel<Coords, kShared><<<grid, 256, 0, st>>>(g, coords, mask, head.mask_bstride, head.mask_act, pos, gat,
-                                                              f32_weights ? 1 : 0, masks);
+                                                              f32_weights ? 1 : 0, masks, nan_flag);
   D2C_LAUNCH_CHECK();
   return D2C_OK;
 }
@@ -144,21 +151,21 @@ struct ClStrides {
 // One A-tile item = the 8 channels [ch0, ch0+8) of one modulated trilinear sample, blended in packed fp16
 // (the weights already carry the modulation), converted to bf16 and stored (16 bytes) in the swizzled A tile.
 // The work is split in two so that a producer can put the corners of several items in flight before the first
-// blend: load_corners issues the corner loads of one item (those that weigh anything, see the record format above; c is
-// finite before), blend_store consumes them.   xb_ch: channels-last fp16 staging of the clip, advanced to the item's channel.
+// blend: load_corners issues the corner loads of one item (those that weigh anything, see the record format above),
+// blend_store consumes them.   xb_ch: channels-last fp16 staging of the clip, advanced to the item's channel.
 __device__ __forceinline__ void load_corners(const __half* __restrict__ xb_ch, ClStrides cs, uint32_t voff,
                                              uint32_t steps, uint4 (&c)[8]) {
   const int dx = (steps & 1u) ? cs.dx : 0, dy = (steps & 2u) ? cs.dy : 0, dz = (steps & 4u) ? cs.dz : 0;
   const __half* p0 = xb_ch + voff;
   const __half* p1 = p0 + dz;
-  ptx::ldg_nc_v4_if(c[0], p0, steps & 8u);
-  ptx::ldg_nc_v4_if(c[1], p0 + dx, steps & 16u);
-  ptx::ldg_nc_v4_if(c[2], p0 + dy, steps & 32u);
-  ptx::ldg_nc_v4_if(c[3], p0 + dy + dx, steps & 64u);
-  ptx::ldg_nc_v4_if(c[4], p1, steps & 128u);
-  ptx::ldg_nc_v4_if(c[5], p1 + dx, steps & 256u);
-  ptx::ldg_nc_v4_if(c[6], p1 + dy, steps & 512u);
-  ptx::ldg_nc_v4_if(c[7], p1 + dy + dx, steps & 1024u);
+  ptx::ldg_nc_v4_or_zero(c[0], p0, steps & 8u);
+  ptx::ldg_nc_v4_or_zero(c[1], p0 + dx, steps & 16u);
+  ptx::ldg_nc_v4_or_zero(c[2], p0 + dy, steps & 32u);
+  ptx::ldg_nc_v4_or_zero(c[3], p0 + dy + dx, steps & 64u);
+  ptx::ldg_nc_v4_or_zero(c[4], p1, steps & 128u);
+  ptx::ldg_nc_v4_or_zero(c[5], p1 + dx, steps & 256u);
+  ptx::ldg_nc_v4_or_zero(c[6], p1 + dy, steps & 512u);
+  ptx::ldg_nc_v4_or_zero(c[7], p1 + dy + dx, steps & 1024u);
 }
 
 // Returns the 16 bytes it stored (a caller that also keeps the samples for the backward writes them to global).
@@ -195,14 +202,14 @@ __device__ __forceinline__ void load_corners_f32(const float* __restrict__ xb_ch
   const int dx = (steps & 1u) ? cs.dx : 0, dy = (steps & 2u) ? cs.dy : 0, dz = (steps & 4u) ? cs.dz : 0;
   const float* p0 = xb_ch + voff;
   const float* p1 = p0 + dz;
-  ptx::ldg_nc_v4_if(c[0], p0, steps & 8u);
-  ptx::ldg_nc_v4_if(c[1], p0 + dx, steps & 16u);
-  ptx::ldg_nc_v4_if(c[2], p0 + dy, steps & 32u);
-  ptx::ldg_nc_v4_if(c[3], p0 + dy + dx, steps & 64u);
-  ptx::ldg_nc_v4_if(c[4], p1, steps & 128u);
-  ptx::ldg_nc_v4_if(c[5], p1 + dx, steps & 256u);
-  ptx::ldg_nc_v4_if(c[6], p1 + dy, steps & 512u);
-  ptx::ldg_nc_v4_if(c[7], p1 + dy + dx, steps & 1024u);
+  ptx::ldg_nc_v4_or_zero(c[0], p0, steps & 8u);
+  ptx::ldg_nc_v4_or_zero(c[1], p0 + dx, steps & 16u);
+  ptx::ldg_nc_v4_or_zero(c[2], p0 + dy, steps & 32u);
+  ptx::ldg_nc_v4_or_zero(c[3], p0 + dy + dx, steps & 64u);
+  ptx::ldg_nc_v4_or_zero(c[4], p1, steps & 128u);
+  ptx::ldg_nc_v4_or_zero(c[5], p1 + dx, steps & 256u);
+  ptx::ldg_nc_v4_or_zero(c[6], p1 + dy, steps & 512u);
+  ptx::ldg_nc_v4_or_zero(c[7], p1 + dy + dx, steps & 1024u);
 }
 
 // w: the eight fp32 products a_j*mask (corner order 000..111, the reference's interpolation chain).

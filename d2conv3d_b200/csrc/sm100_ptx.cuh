@@ -318,20 +318,26 @@ __device__ __forceinline__ uint4 ldg_nc_v4(const void* p) {
   asm("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
   return r;
 }
-// The same under a predicate: r keeps its contents where cond is 0.
-__device__ __forceinline__ void ldg_nc_v4_if(uint4& r, const void* p, uint32_t cond) {
+// The same under a predicate: zero where cond is 0.
+__device__ __forceinline__ void ldg_nc_v4_or_zero(uint4& r, const void* p, uint32_t cond) {
   asm("{\n\t.reg .pred q;\n\t"
       "setp.ne.u32 q, %5, 0;\n\t"
+      "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
       "@q ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
-      : "+r"(r.x), "+r"(r.y), "+r"(r.z), "+r"(r.w) : "l"(p), "r"(cond));
+      : "=&r"(r.x), "=&r"(r.y), "=&r"(r.z), "=&r"(r.w) : "l"(p), "r"(cond));
 }
-// 32 bytes (32-byte aligned) under a predicate.
+// 32 bytes (32-byte aligned) under a predicate: r keeps its contents where cond is 0.
 __device__ __forceinline__ void ldg_nc_v8_if(uint32_t (&r)[8], const void* p, uint32_t cond) {
   asm("{\n\t.reg .pred q;\n\t"
       "setp.ne.u32 q, %9, 0;\n\t"
       "@q ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
       : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
       : "l"(p), "r"(cond));
+}
+// Clears r in the branch that it is written in (volatile: as a select it would wait for loads in flight).
+__device__ __forceinline__ void clear_v8(uint32_t (&r)[8]) {
+#pragma unroll
+  for (int e = 0; e < 8; ++e) asm volatile("mov.b32 %0, 0;" : "=r"(r[e]));
 }
 __device__ __forceinline__ void stg_v4_hint(void* p, uint4 v, uint64_t pol) {
   asm volatile("st.global.L2::cache_hint.v4.u32 [%0], {%1, %2, %3, %4}, %5;"
