@@ -9,15 +9,19 @@
 // Interfaces it stands in for: csrc/ops/dconv3d.h:70-226 (DeformConv3dFunction, deform_conv3d), csrc/ops/dconv1d.h:69-186,
 // fast-depthwise-conv3d/csrc/grouped_conv3d.h:29-106, and the half-precision up-cast of deform_conv.py:54-59.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/cuda/Event.h>
 #include <torch/extension.h>
 
 #include <array>
 #include <atomic>
+#include <mutex>
 #include <optional>
+#include <vector>
 
 #include "d2conv3d.h"
 
@@ -86,22 +90,37 @@ d2c_conv_desc make_desc(const Tensor& x, const Tensor& w, int dtype, const Tripl
 // Whether a forward that will be differentiated keeps its blended samples for the weight gradient.
 std::atomic<bool> g_keep_samples{true};
 
-// Event that every deformable backward records as soon as its parameter gradients are final, one per device.
-constexpr int kMaxDevices = 64;
-std::atomic<cudaEvent_t> g_params_ready[kMaxDevices];
-std::atomic<int> g_params_ready_device{-1};
+// Events that deformable backwards record as soon as their parameter gradients are final.  A backward records one that nobody
+// else holds; the last one recorded waits here until params_ready_event() hands it out for good (a later backward then records
+// another), the one before it is recorded again.
+struct ReadyEvents {
+  std::mutex mutex;
+  std::optional<at::cuda::CUDAEvent> latest;
+  std::vector<at::cuda::CUDAEvent> spare;      // as many as backwards ran at the same time
 
-cudaEvent_t params_ready_event(int device) {
-  if (device < 0 || device >= kMaxDevices) return nullptr;
-  cudaEvent_t ev = g_params_ready[device].load(std::memory_order_acquire);
-  if (ev) return ev;
-  C10_CUDA_CHECK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-  cudaEvent_t none = nullptr;
-  if (!g_params_ready[device].compare_exchange_strong(none, ev)) {
-    (void)cudaEventDestroy(ev);
-    ev = none;
+  at::cuda::CUDAEvent borrow(const at::cuda::CUDAStream& stream) {
+    {
+      const std::lock_guard<std::mutex> lock(mutex);
+      for (auto it = spare.begin(); it != spare.end(); ++it)
+        if (it->device_index() == stream.device_index()) {
+          at::cuda::CUDAEvent ev = std::move(*it);
+          spare.erase(it);
+          return ev;
+        }
+    }
+    at::cuda::CUDAEvent ev;
+    ev.record(stream);                          // creates it
+    return ev;
   }
-  return ev;
+  void publish(at::cuda::CUDAEvent&& ev) {
+    const std::lock_guard<std::mutex> lock(mutex);
+    if (latest) spare.push_back(std::move(*latest));
+    latest = std::move(ev);
+  }
+};
+ReadyEvents& ready_events() {
+  static auto* const events = new ReadyEvents();     // outlives the CUDA context
+  return *events;
 }
 
 // Results of a backward node: gradients are computed outside the graph, so a second derivative has to fail loudly.
@@ -152,9 +171,11 @@ struct DeformNode : public Node {
       const int op = (kind == Kind::field || kind == Kind::head_field) ? D2C_OP_DYNDIL_BWD : D2C_OP_DEFORM_BWD;
       const size_t n = is_head ? d2c_head_workspace_bytes(op, &desc, &head, field_mode) : d2c_workspace_bytes(op, &desc);
       const Tensor ws = bytes_on(n, xv);
-      void* st = stream_of(xv);
-      const int device = xv.device().index();
-      cudaEvent_t ev = kind == Kind::conv1d ? nullptr : params_ready_event(device);
+      const at::cuda::CUDAStream stream = at::cuda::getCurrentCUDAStream(xv.device().index());
+      void* st = stream.stream();
+      std::optional<at::cuda::CUDAEvent> ready;
+      if (kind != Kind::conv1d) ready = ready_events().borrow(stream);
+      cudaEvent_t ev = ready ? ready->event() : nullptr;
       if (cache.format) check(d2c_bind_sample_cache(&cache), "bind_sample_cache");
       int rc = 0;
       switch (kind) {
@@ -180,7 +201,7 @@ struct DeformNode : public Node {
           break;
       }
       check(rc, "deformable convolution backward");
-      if (ev) g_params_ready_device.store(device, std::memory_order_release);
+      if (ready) ready_events().publish(std::move(*ready));
     }
     if (is_head) return once_differentiable({gx, ggeo, gw, gbias});
     return once_differentiable({gx, ggeo, gmask, gw, gbias});
@@ -483,10 +504,20 @@ Tensor depthwise_conv3d(const Tensor& input, const Tensor& weight, const OptTens
 
 void set_keep_samples(bool on) { g_keep_samples.store(on); }
 bool get_keep_samples() { return g_keep_samples.load(); }
-int64_t params_ready_device() { return g_params_ready_device.load(std::memory_order_acquire); }
-void wait_params_ready(int64_t device, int64_t stream) {
-  cudaEvent_t ev = params_ready_event((int)device);
-  if (ev) C10_CUDA_CHECK(cudaStreamWaitEvent(reinterpret_cast<cudaStream_t>(stream), ev, 0));
+
+// The event of the most recent backward as a torch.cuda.Event, once; None where there is none that was not handed out.
+py::object take_params_ready_event() {
+  ReadyEvents& events = ready_events();
+  {
+    const std::lock_guard<std::mutex> lock(events.mutex);
+    if (!events.latest) return py::none();
+  }
+  py::object event = py::module_::import("torch.cuda").attr("Event")();
+  const std::lock_guard<std::mutex> lock(events.mutex);
+  if (!events.latest) return py::none();
+  reinterpret_cast<THCPEvent*>(event.ptr())->cuda_event = std::move(*events.latest);
+  events.latest.reset();
+  return event;
 }
 
 }  // namespace
@@ -500,6 +531,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("depthwise_conv3d", torch::wrap_pybind_function_no_gil(depthwise_conv3d));
   m.def("set_keep_samples", set_keep_samples);
   m.def("get_keep_samples", get_keep_samples);
-  m.def("params_ready_device", params_ready_device);
-  m.def("wait_params_ready", wait_params_ready);
+  m.def("take_params_ready_event", take_params_ready_event);
 }

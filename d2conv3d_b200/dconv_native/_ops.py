@@ -6,6 +6,7 @@ DeformConv3dFunction, csrc/ops/dconv3d.h:70-186, and DeformConv1dFunction,
 csrc/ops/dconv1d.h:69-156) are native too (csrc/torch_ops.cpp).
 """
 import ctypes
+import threading
 import types
 
 import torch
@@ -13,21 +14,21 @@ import torch
 from .. import _lib
 
 
+_ready_lock = threading.Lock()
+_ready = None
+
+
 def params_ready_event():
-    """A torch.cuda.Event that fires once the parameter gradients (grad_weight, grad_bias) of the most recent
-    `deform_conv3d` / `dyn_dilated_conv3d` backward of this process are final -- on the tensor-core tier before the
-    data-side gradients are computed.  A data-parallel trainer makes a side stream wait for it and all-reduces the
-    parameter gradients there (d2conv3d_b200.sharding.all_reduce_param_grads_overlapped), which hides the collective
-    under the rest of the backward.  None before the first backward."""
-    C = _lib.native()
-    device = C.params_ready_device()
-    if device < 0:
-        return None
-    # the backward records one event per device; what the caller gets follows it on a stream of its own, so a later
-    # backward does not move it
-    stream = torch.cuda.Stream(device)
-    C.wait_params_ready(device, stream.cuda_stream)
-    return stream.record_event()
+    """The torch.cuda.Event that the most recent `deform_conv3d` / `dyn_dilated_conv3d` backward of this process
+    recorded as soon as its parameter gradients (grad_weight, grad_bias) were final -- on the tensor-core tier
+    before the data-side gradients are computed.  A data-parallel trainer makes a side stream wait for it and
+    all-reduces the parameter gradients there (d2conv3d_b200.sharding.all_reduce_param_grads_overlapped), which
+    hides the collective under the rest of the backward.  No later backward records it again.  None before the first
+    backward."""
+    global _ready
+    with _ready_lock:
+        _ready = _lib.native().take_params_ready_event() or _ready
+        return _ready
 
 
 def _will_differentiate(*tensors):
