@@ -150,7 +150,10 @@ struct DeformNode : public Node {
 
   std::string name() const override { return "D2CDeformConvBackward"; }
 
+  // Two threads may run backward over a shared graph: what a node holds is unpacked and released under its mutex, as PyTorch's
+  // own nodes do; the pass itself works on its own references.
   void release_variables() override {
+    const std::lock_guard<std::mutex> lock(mutex_);
     x.reset_data(); geo.reset_data(); mask.reset_data(); weight.reset_data();
     cache_buf = Tensor();
     cache = d2c_sample_cache{};
@@ -160,7 +163,14 @@ struct DeformNode : public Node {
     const bool is_head = kind == Kind::head_offsets || kind == Kind::head_field;
     const size_t n_out = is_head ? 4 : 5;
     if (!grads[0].defined()) return variable_list(n_out);
-    const Tensor xv = x.unpack(), gv = geo.unpack(), mv = mask.unpack(), wv = weight.unpack();
+    Tensor xv, gv, mv, wv, kept_buf;
+    d2c_sample_cache kept;
+    {
+      const std::lock_guard<std::mutex> lock(mutex_);
+      xv = x.unpack(); gv = geo.unpack(); mv = mask.unpack(); wv = weight.unpack();
+      kept_buf = cache_buf;
+      kept = cache;
+    }
     Tensor gx, ggeo, gmask, gw, gbias;
     {
       at::AutoGradMode no_grad(false);
@@ -176,7 +186,7 @@ struct DeformNode : public Node {
       std::optional<at::cuda::CUDAEvent> ready;
       if (kind != Kind::conv1d) ready = ready_events().borrow(stream);
       cudaEvent_t ev = ready ? ready->event() : nullptr;
-      if (cache.format) check(d2c_bind_sample_cache(&cache), "bind_sample_cache");
+      if (kept.format) check(d2c_bind_sample_cache(&kept), "bind_sample_cache");
       int rc = 0;
       switch (kind) {
         case Kind::offsets:
@@ -427,11 +437,18 @@ struct DepthwiseNode : public Node {
   SavedVariable x, weight;
 
   std::string name() const override { return "D2CDepthwiseConv3dBackward"; }
-  void release_variables() override { x.reset_data(); weight.reset_data(); }
+  void release_variables() override {
+    const std::lock_guard<std::mutex> lock(mutex_);
+    x.reset_data(); weight.reset_data();
+  }
 
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return variable_list(3);
-    const Tensor xv = x.unpack(), wv = weight.unpack();
+    Tensor xv, wv;
+    {
+      const std::lock_guard<std::mutex> lock(mutex_);
+      xv = x.unpack(); wv = weight.unpack();
+    }
     Tensor gx, gw, gb;
     {
       at::AutoGradMode no_grad(false);
