@@ -13,7 +13,7 @@
 //     instead of five.  One thread for both would hold 108 registers of weights and sums and spilled.
 //   * planes arrive in two rings.  Every band of rows of a plane of one channel is one contiguous byte range; it is bulk
 //     copied from the 16-byte boundary below its start (any width, offset and pointer alignment: the remainder is added to
-//     the reader's address) into a raw stage.  Two warps turn the raw bands of a channel pair into one stage of fp32 pairs
+//     the reader's address; vectors that the tensor's first or last byte cuts are fetched by elements) into a raw stage.  Two warps turn the raw bands of a channel pair into one stage of fp32 pairs
 //     {c, c+1} with zeros around it, once per plane: a compute thread's plane is then 18 conflict-free 8-byte loads and 108
 //     packed FMA.  (Reading the channels' separate bands from the compute threads cost 36 loads, 24 selects and as many
 //     moves as FMA; pairing in the compute threads instead of two warps of their own gave 445 instructions per 108 FMA.)
@@ -131,6 +131,20 @@ struct DwpBand {
   }
   static __device__ __forceinline__ int shift(const T* start) {
     return (int)((reinterpret_cast<uintptr_t>(start) / sizeof(T)) % kVec);
+  }
+};
+
+// The 16-byte vectors that a bulk copy takes for the bytes [start, stop) of the tensor [base, end): those that hold any of them
+// and lie inside the tensor.  What remains of [start, stop) is part of a vector that the tensor's first or last byte cuts.
+struct DwpSpan {
+  uintptr_t lo, hi;
+  __host__ __device__ DwpSpan(uintptr_t start, uintptr_t stop, uintptr_t base, uintptr_t end) {
+    const uintptr_t first = (base + 15) & ~(uintptr_t)15, last = end & ~(uintptr_t)15;
+    lo = start & ~(uintptr_t)15;
+    hi = (stop + 15) & ~(uintptr_t)15;
+    if (lo < first) lo = first;
+    if (hi > last) hi = last;
+    if (hi < lo) hi = lo;
   }
 };
 
@@ -425,6 +439,8 @@ struct DwpCopier {
   int rows_n = 0;
   bool mine = false;
   const T* src = nullptr;
+  uintptr_t tensor_beg = reinterpret_cast<uintptr_t>(a.in);
+  uintptr_t tensor_end = tensor_beg + (uintptr_t)((long long)a.g.B * a.g.Cin * a.g.D * a.g.H * a.g.W * sizeof(T));
   uint32_t issued = 0;
   __device__ __forceinline__ bool done() const { return ch >= ch_end; }
   __device__ __forceinline__ void open() {
@@ -440,15 +456,24 @@ struct DwpCopier {
   }
   __device__ __forceinline__ void step() {
     if (p == 0) open();
-    constexpr int kVec = DwpBand<T>::kVec;
-    const int sh = DwpBand<T>::shift(src);
-    const uint32_t len = mine ? (uint32_t)((sh + rows_n + kVec - 1) / kVec * 16) : 0u;
+    const uint32_t slot = ring + (uint32_t)((stage * a.plan.groups * 2 + lane) * a.plan.raw * (int)sizeof(T));
+    const uintptr_t start = reinterpret_cast<uintptr_t>(src), stop = start + rows_n * sizeof(T), at0 = start & ~(uintptr_t)15;
+    const DwpSpan span(start, stop, tensor_beg, tensor_end);
+    const uint32_t len = mine ? (uint32_t)(span.hi - span.lo) : 0u;
+    if (mine && (span.lo > start || span.hi < stop)) {       // the tensor's first or last band, where it is not aligned
+      T* dst = reinterpret_cast<T*>(__cvta_shared_to_generic(slot + (uint32_t)(start - at0)));
+      for (int i = 0; i < rows_n; ++i) {
+        const uintptr_t e = start + i * sizeof(T);
+        if (e < span.lo || e >= span.hi) dst[i] = __ldg(src + i);
+        else i = (int)((span.hi - start) / sizeof(T)) - 1;
+      }
+      ptx::fence_proxy_async_smem();       // a bulk copy writes here the next time
+    }
+    __syncwarp();
     const uint32_t total = __reduce_add_sync(0xffffffffu, len);
     if (lane == 0) ptx::mbar_arrive_expect_tx(full0 + 8u * stage, total);
     __syncwarp();
-    if (mine)
-      ptx::bulk_g2s(ring + (uint32_t)((stage * a.plan.groups * 2 + lane) * a.plan.raw * (int)sizeof(T)), src - sh, len,
-                    full0 + 8u * stage);
+    if (len) ptx::bulk_g2s(slot + (uint32_t)(span.lo - at0), reinterpret_cast<const void*>(span.lo), len, full0 + 8u * stage);
     src += (long long)a.g.H * a.g.W;
     ++issued;
     if (++stage == kDwpRawStages) stage = 0;
