@@ -20,6 +20,7 @@ the reference does (which, like the reference, requires offset_groups == 1).
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 from torch.nn.modules.utils import _triple
 from torch.utils.checkpoint import checkpoint
 
@@ -189,12 +190,14 @@ class _DConvBase(nn.Module):
         """The predictor's output.  cuDNN pads the filter of a convolution whose output channels are not a multiple of
         eight (modulated field layers: 3 + 27 * groups) with a generic transform on every call, 92 us for 256 -> 219
         channels whatever the volume; copying it into padded rows costs 5 us.  Only where the extra channels cost
-        nothing afterwards: no autograd, one clip (the slice is then contiguous), and a plain convolution module."""
+        nothing afterwards: no autograd, one clip (the slice is then contiguous), and a plain convolution module that nobody
+        looks at (hooks of its own or of every module) or has replaced the forward of."""
         conv = self.deform_params
         pad = -self._deform_channels() % 8
         if (pad == 0 or type(conv) is not nn.Conv3d or torch.is_grad_enabled() or input.dim() != 5 or input.shape[0] != 1
                 or not input.is_cuda or conv.groups != 1 or conv.padding_mode != "zeros" or isinstance(conv.padding, str)
-                or conv.out_channels < 32 or conv._forward_hooks or conv._forward_pre_hooks):
+                or conv.out_channels < 32 or conv._forward_hooks or conv._forward_pre_hooks or _has_any_global_hook()
+                or "forward" in vars(conv)):
             return conv(input)
         # the extra rows are never looked at: an output channel depends on its own row only
         def padded(t):
