@@ -23,6 +23,7 @@ LIB = os.path.join(HERE, "libd2conv3d.so")
 TORCH_SRC = os.path.join(CSRC, "torch_ops.cpp")
 TORCH_LIB = os.path.join(HERE, "_C.so")
 OBJ_DIR = os.path.join(HERE, "build")
+TORCH_STAMP = os.path.join(OBJ_DIR, "torch_ops.stamp")
 
 SOURCES = ["d2c_api.cu", "depthwise.cu", "deform_sm100_fwd.cu", "deform_sm100_bwd.cu", "deform_sm100_dw.cu",
            "deform_exact_f32.cu", "deform_exact_f64.cu", "act_norm.cu"]
@@ -51,9 +52,18 @@ def needs_build():
     return any(os.path.getmtime(d) > t for d in _deps())
 
 
+def _torch_stamp():
+    """What the front-end was compiled against; it does not load, or misbehaves, with another one."""
+    import torch
+    return f"torch {torch.__version__}, python {sys.version_info.major}.{sys.version_info.minor}"
+
+
 def _torch_needs_build():
-    if not os.path.exists(TORCH_LIB):
+    if not os.path.exists(TORCH_LIB) or not os.path.exists(TORCH_STAMP):
         return True
+    with open(TORCH_STAMP) as f:
+        if f.read() != _torch_stamp():
+            return True
     t = os.path.getmtime(TORCH_LIB)
     return any(os.path.getmtime(d) > t for d in (TORCH_SRC, os.path.join(INCLUDE, "d2conv3d.h")))
 
@@ -63,6 +73,7 @@ def build_torch(force=False):
     finds beside itself)."""
     if not force and not _torch_needs_build():
         return TORCH_LIB
+    os.makedirs(OBJ_DIR, exist_ok=True)
     import sysconfig
 
     import torch
@@ -79,6 +90,8 @@ def build_torch(force=False):
     if p.returncode != 0:
         sys.stderr.write(p.stdout)
         raise RuntimeError("building the PyTorch front-end failed")
+    with open(TORCH_STAMP, "w") as f:
+        f.write(_torch_stamp())
     return TORCH_LIB
 
 
