@@ -236,7 +236,7 @@ TRAFFIC_PER_LAUNCH = {       # (phase, math mode) -> DRAM read + write bytes of 
 # (5.69 of 8 per sample on average at sigma = 2 voxels, D = 8) x 5.6 M samples x 256 B; rate = what
 # red.global.add.v4.f32 sustains on this part for exactly this access pattern (microbenchmark, 11.5 GB in 1.69 ms).
 SCATTER = {"payload_bytes": 5.687 * 2 * 8 * 27 * 12960 * 256, "rate_gbs": 6773.0,
-           "source": "d2conv3d_b200/csrc/microbench/l2_rates.cu on a B200 of this pool"}
+           "source": "profiles/b200_l2_scatter_gather_rates.md, stand-alone measurement on a B200"}
 
 PHASE_WORK = {
     # phase name -> (bound, key of the algorithmic work of one launch)

@@ -1,10 +1,6 @@
 """Builds libd2conv3d.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
 
-    python -m d2conv3d_b200.build [--force] [--verbose] [--microbench]
-
---microbench also builds the stand-alone programs of csrc/microbench into build/: l2_rates (the L2 scatter-add and
-gather rates that bound the sampling kernels) and mma_rate (clocks per tcgen05.mma of the kernels' shape).  They run
-on the GPU and are not part of the library.
+    python -m d2conv3d_b200.build [--force] [--verbose] [--unit-trace]
 
 The library links only the CUDA runtime (statically); it has no dependency on
 torch or Python.  _C.so, built beside it, is the PyTorch front-end (csrc/torch_ops.cpp:
@@ -40,7 +36,7 @@ def _nvcc():
 def _deps():
     out = [os.path.join(INCLUDE, "d2conv3d.h")]
     for f in os.listdir(CSRC):
-        if os.path.isfile(os.path.join(CSRC, f)) and not f.endswith(".cpp"):
+        if not f.endswith(".cpp"):
             out.append(os.path.join(CSRC, f))
     return out
 
@@ -146,19 +142,5 @@ def ptxas_report():
     return out
 
 
-def build_microbench():
-    os.makedirs(OBJ_DIR, exist_ok=True)
-    outs = []
-    for name in ("l2_rates", "mma_rate"):
-        out = os.path.join(OBJ_DIR, name)
-        cmd = [_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-o", out,
-               os.path.join(CSRC, "microbench", name + ".cu")]
-        subprocess.run(cmd, check=True)
-        outs.append(out)
-    return outs
-
-
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv, unit_trace="--unit-trace" in sys.argv))
-    if "--microbench" in sys.argv:
-        print(build_microbench())
