@@ -324,7 +324,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
 
 // ---- index arithmetic ----------------------------------------------------------------------------------
 
-// Division of 0 <= n < 2^31 by a divisor known on the host.
+// Division of 0 <= n < 2^31 by a divisor known on the host: multiply by its scaled reciprocal and shift (Granlund and Montgomery,
+// "Division by Invariant Integers using Multiplication", PLDI 1994).
 struct FastDiv {
   uint32_t d, mul, shift;
   static FastDiv of(int d) {
@@ -608,7 +609,8 @@ struct FwdOp {
 
   struct Producer {
     static constexpr int kDirW = kTK * TN / kProducers;     // weights a thread fetches per step when they are not staged
-    // two items in flight spill next to a 128-column tile (492 us with one, 545 with two)
+    // next to a 128-column tile one item in flight spills already (offsets, channels-last: 544 bytes stored, 548 loaded) and two
+    // spill twice that: 492 us with one, 545 with two
     static constexpr int kBuf = sizeof(T) == 8 || TN == 128 ? 1 : 2;
     const FwdOp& op;
     const int t, R;
@@ -1352,7 +1354,7 @@ inline long long units_grid(const Units& u, int sm_count) {
 // Whether some CTA of it ends inside a tile (then the output is accumulated).
 inline bool shares_tiles(const Units& u, int sm_count) { return u.tiles % units_grid(u, sm_count) != 0; }
 
-// Once per kernel and device: shared memory, register check, and how many clusters of each size fit.
+// Shared memory, and once per kernel and process (whose GPUs are alike) a register check and how many clusters of each size fit.
 struct GemmSetup {
   int rc;
   int clusters[9];     // [size]: resident clusters, 0 where the size is not used

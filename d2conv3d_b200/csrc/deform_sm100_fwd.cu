@@ -65,9 +65,10 @@ constexpr int kRowsPerThread = kBM / kRowStride;
 constexpr int kSmemLimit = 227 * 1024;
 // Shared memory is what the L1 cache does not get, and the gather lives off L1 (the two rows of corners of neighbouring
 // voxels and taps): the weight ring takes no more than leaves the 196 KB split (1 KB of it is the system's), 60 KB of L1.
-// 256 output channels, field layer, 2 x 8 x 60 x 107: 4 stages of 32 KB (28 KB of L1) 2.32 ms, 3 stages 2.15 ms, 2 stages
-// (92 KB of L1, but the ring runs dry) 2.16 ms.  512 output channels with 64 KB stages had no room for that: 1.55 ms at 2 x 8
-// x 30 x 54 where 32 KB stages take 1.31 ms.  Two A stages or two record stages instead cost more than the L1 gives back.
+// 256 output channels, field layer, 2 x 8 x 60 x 107, measured with 16-byte gathers (2.15 ms then, 1.85 now): 4 stages of 32 KB
+// (28 KB of L1) 2.32 ms, 3 stages 2.15 ms, 2 stages (92 KB of L1, but the ring runs dry) 2.16 ms.  512 output channels with 64
+// KB stages had no room for that: 1.55 ms at 2 x 8 x 30 x 54 where 32 KB stages took 1.31.  Two A stages or two record stages
+// instead cost more than the L1 gives back.
 constexpr int kSmemGather = 195 * 1024;
 // Fewest units a CTA is started for.  A unit takes 1.9-2.3 us in its CTA (the producers' gather latency), starting a CTA
 // and adding its partial tile to y about 5 us together: below four units per CTA more CTAs no longer shorten the call.
@@ -207,7 +208,11 @@ bool make_plan(const Geom& g, bool x3, Plan* pl, bool shared = false) {
   pl->dual = dual ? 1 : 0;
   pl->r_stage_bytes = kRStageBytesOf(pl->dual, shared ? 1 : 0);
   if (g.Cout % 64 != 0 || g.Cout > kMaxN) return false;
-  if (dual && g.Cout > 448) return false;      // layers this wide run the (more exact) split kernel
+  // The backward of such a layer is the split one above 256 output channels (deform_sm100_bwd.cu), and only a forward of the same
+  // arithmetic keeps its samples for it.  256 -> 512 channels in 8 groups, 2 x 8 x 30 x 54, forward + backward: split 0.78 + 2.12
+  // ms, single-pass 0.45 + 2.67 ms.  Inference alone would gain from the single pass (0.69 and 0.45 ms), at its precision (4e-4 of
+  // the result instead of 9e-7).
+  if (dual && g.Cout > 448) return false;
   if (g.Vin * g.Cin > 0x7fffffffLL) return false;                 // 32-bit element offsets within a clip
   if (g.K * 64 * (int)sizeof(float) > 48 * 1024) return false;    // weight staging kernel's smem
   pl->nh = dual ? 1 : g.cpg / (x3 ? 32 : kBK);

@@ -10,7 +10,8 @@
 //   * the backward needs only grad_out's neighbourhood: grad_x(q) and grad_w both multiply the SAME neighbour grad_out(q - k),
 //     by w(k) and by x(q).  Half of a block's compute warps form grad_x (the forward's code, weights reflected), the other
 //     half grad_w (x straight into registers), from the same staged planes: three tensors of traffic for the two gradients
-//     instead of five.  One thread for both would hold 108 registers of weights and sums and spilled.
+//     instead of five.  One thread for both would hold 108 registers of weights and sums; with two roles the kernel spills a
+//     little (fp16 backward: 64 bytes stored, 100 loaded).
 //   * planes arrive in two rings.  Every band of rows of a plane of one channel is one contiguous byte range; it is bulk
 //     copied from the 16-byte boundary below its start (any width, offset and pointer alignment: the remainder is added to
 //     the reader's address; vectors that the tensor's first or last byte cuts are fetched by elements) into a raw stage.  Two warps turn the raw bands of a channel pair into one stage of fp32 pairs

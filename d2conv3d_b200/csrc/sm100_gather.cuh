@@ -30,8 +30,9 @@
 // their contents from item to item, which spilled).  The forward, whose 32-byte gathers have a register file's worth in flight,
 // clears them only where the staged input holds a NaN (deform_sm100_fwd_kernel.cuh).
 // Corners of zero weight are those outside the volume and, for a dilation field, the upper neighbour along every axis on which
-// the tap sits at the kernel's centre: 4.6 corners a tap instead of 8 with 3 x 3 x 3 taps.  The forward of such a layer, 256
-// channels on 2 x 8 x 60 x 107, takes 2.27 ms instead of 2.71; with free offsets the corners outside the volume give 512 channels on 2 x 8 x 30 x 54 1.55 instead of 1.68.
+// the tap sits at the kernel's centre: 4.6 corners a tap instead of 8 with 3 x 3 x 3 taps.  Leaving them out took the forward of
+// such a layer, 256 channels on 2 x 8 x 60 x 107, from 2.71 to 2.27 ms (1.85 now) and, with free offsets, where they are the corners
+// outside the volume, 512 channels on 2 x 8 x 30 x 54 from 1.68 to 1.55 ms (1.32 now).
 #pragma once
 
 #include <cuda_fp16.h>
