@@ -222,7 +222,7 @@ bool make_plan(const Geom& g, bool x3, Plan* pl, bool shared = false) {
   if ((long long)pl->n_tiles * pl->S > 0x7fffffffLL) return false;   // the kernel counts units in 31 bits
   pl->w_slice_bytes = g.Cout * 128;
   pl->b_stage_bytes = (g.Cout < 256 ? g.Cout : 256) * 128;
-  // 256 bytes of barriers + 132 bytes of part ranges (rounded to 512) + 1 KB of alignment slack
+  // 256 bytes of barriers + 136 bytes of part ranges and flag (rounded to 512) + 1 KB of alignment slack
   const int other = 1024 + 768 + kAStages * kAStageBytes + kRStages * pl->r_stage_bytes;
   int nb = (kSmemGather - other) / pl->b_stage_bytes;
   if (nb > 4) nb = 4;

@@ -19,7 +19,7 @@
 
 constexpr int kThreadsFwd = 24 * 32;
 static_assert(128 * 56 + 128 * 40 + 512 * 96 <= kThreadsFwd * 80, "setmaxnreg budget exceeds the CTA's register allocation");
-constexpr int kMmaWarpFwd = 4, kLoadWarpFwd = 5, kRecWarpFwd = 6, kGatherWarp0Fwd = 8;
+constexpr int kMmaWarpFwd = 4, kLoadWarpFwd = 5, kRecWarpFwd = 6, kIdleWarpFwd = 7, kGatherWarp0Fwd = 8;
 
 // kX3 = 0: math mode bf16 (a unit is 64 channels of one tap, one bf16 operand pair).
 // kX3 = 1: math mode bf16x3, the fp32-parity mode: a unit is 32 channels; the A row holds [hi(32) | lo(32)] of
@@ -66,7 +66,7 @@ fwd_sm100_kernel(const FwdParams p) {
   // part.  Thread 0 puts the ranges into shared memory once, so that the roles (some of them left with 40 registers)
   // do no 64-bit division.
   // (unit indices fit 31 bits: checked by the host)
-  int* part_tab = reinterpret_cast<int*>(base_ptr + bar_off + 256);      // [part][beg, end], then the total
+  int* part_tab = reinterpret_cast<int*>(base_ptr + bar_off + 256);      // [part][beg, end], the total, whether x holds a NaN
   // Large volumes (FwdParams::rr): whole tiles dealt round-robin instead -- at any time the CTAs then work on
   // gridDim.x CONSECUTIVE tiles, whose sampling neighbourhoods overlap, so the part of the staged input they gather
   // from is a few planes and not a few planes around 148 places spread over the whole volume (which L2 cannot hold:
@@ -104,6 +104,8 @@ fwd_sm100_kernel(const FwdParams p) {
     *abort_flag = 0;
     ptx::fence_mbar_init();
   }
+  // by a warp without a role, beside the set-up (in the producers it would delay a call's first unit by up to 0.6 us)
+  if (threadIdx.x == kIdleWarpFwd * 32) part_tab[33] = __ldg(p.nan_flag);
   if (warp == 0) {
     __syncwarp();
     ptx::tmem_alloc(ptx::smem_u32((const void*)tmem_slot), (uint32_t)p.tmem_cols);
@@ -390,9 +392,9 @@ fwd_sm100_kernel(const FwdParams p) {
     // eight addresses serve 32 bytes of every corner and a row's 16-byte chunks of the A tile need no exchange between lanes.
     // The corners of unit k+1 are requested half by half (z floor, z ceil) as soon as the same half of unit k is blended:
     // 64 registers of corners are all in flight while the thread waits, half of them under each blend.
-    // Bound by the load pipe (73 % busy at 512 channels, 8 x 30 x 54).  With 16 bytes of two rows per thread and unit, twice the
-    // records, addresses and waits, it took 1.40 ms at 512 channels, 2 x 8 x 30 x 54, now 1.33; 256-channel field layer, 2 x 8 x
-    // 60 x 107: 2.20 ms, now 1.88.
+    // Bound by the load pipe (l1tex__data_pipe_lsu_wavefronts: 73 % of the elapsed cycles at 512 channels, 2 x 8 x 30 x 54,
+    // samples kept; profiles/forward_gather_kernels.md).  With 16 bytes of two rows per thread and unit, twice the records,
+    // addresses and waits, it took 1.40 ms there, now 1.33; 256-channel field layer, 2 x 8 x 60 x 107: 2.20 ms, now 1.86.
     const int t = threadIdx.x - kGatherWarp0Fwd * 32;
     const int j = t & 3;             // 32-byte quarter of the row
     // the two rows of a quarter warp (one shared-memory store phase) differ in the bit that keeps their chunks apart:
@@ -490,7 +492,7 @@ fwd_sm100_kernel(const FwdParams p) {
     // Corners that weigh nothing are not read, and blended with weight zero: their registers hold zero or a corner of an earlier
     // unit, of which only a NaN would show.  Where x holds a NaN they are cleared, in a loop of its own.  256 channels, field
     // layer of one group, 2 x 8 x 60 x 107, inference, without / with that / always cleared / cleared where a blended sample is
-    // NaN: 1.371 / 1.377 / 1.495 / 1.404 ms; as a branch in one loop 1.383.
+    // NaN: 1.371 / 1.376 / 1.495 / 1.404 ms; as a branch in one loop 1.383.
     auto work = [&](auto clear) {
     for (uint32_t k = 0; ok && k < n_my_units; ++k) {
       const int sr = k % kRStages, sa = k % kAStages;
@@ -575,7 +577,7 @@ fwd_sm100_kernel(const FwdParams p) {
       D2C_TG(7);
     }
     };
-    if (__ldg(p.nan_flag)) work(std::true_type{});
+    if (part_tab[33]) work(std::true_type{});
     else work(std::false_type{});
   }
 
