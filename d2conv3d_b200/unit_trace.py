@@ -14,8 +14,8 @@ STAMPS = [
     ["loop top", "stage free"],
     ["loop top", "stage free"],
     ["loop top", "A tile full", "weights full", "MMAs issued", "commits issued"],
-    ["loop top", "row 1 loads issued", "A stage free", "row 0 blended", "next records there", "next row 0 loads issued",
-     "row 1 blended", "arrived"],
+    ["unit begins", "z floor half blended", "next records there", "next z floor requested", "z ceil blended, requested",
+     "A stage free", "A tile stored", "arrived (copy kept)"],
 ]
 STAMPS.append(STAMPS[3])
 
