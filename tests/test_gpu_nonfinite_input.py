@@ -19,6 +19,7 @@ SHAPES = [
     dict(B=3, Cin=64, Cout=64, dims=(4, 9, 10), G=1),             # ragged last tile, several clips per CTA
     dict(B=2, Cin=256, Cout=64, dims=(3, 7, 9), G=8),             # 32 channels per group (bf16: two groups a unit)
     dict(B=2, Cin=128, Cout=320, dims=(2, 8, 9), G=1),            # two weight stages a unit
+    dict(B=2, Cin=128, Cout=64, dims=(3, 6, 8), G=2),             # 64 channels per group
     dict(B=2, Cin=24, Cout=40, dims=(3, 6, 7), G=2),              # CUDA-core tier
 ]
 
