@@ -4,9 +4,8 @@
 //                           as a tcgen05 GEMM (bf16 operands, fp32 accumulate in TMEM), voxel-major
 //                           rows so that the 64 channels of one (offset group, tap) slice are contiguous.
 //                           Replaces the reference's cuBLAS call at csrc/ops/dconv3d_gpu.cu:981-999.
-//   (b) sample_grad_kernel  one pass over dcol that produces grad_offset / grad_mask (8 corner dot-products
-//                           per (voxel, group, tap), reduced over channels by warp shuffles) AND scatters
-//                           grad_input with 16-byte vector reductions into a channels-last fp32 buffer.
+//   (b) sample_grad_taps_kernel  grad_offset / grad_mask and grad_input (channels-last fp32) from dcol; the contributions to an
+//                           input voxel are added up per block and leave it as one reduction (sm100_sample_grad.cuh).
 //                           Replaces deformable_col2im_coord_gpu_kernel (:756-864) and
 //                           deformable_col2im_gpu_kernel (:562-643).
 //   (c) unstage_grad_input_kernel  channels-last fp32 -> NCDHW.
@@ -19,6 +18,7 @@
 #include "deform_sm100.h"
 #include "sm100_gather.cuh"
 #include "sm100_ptx.cuh"
+#include "sm100_sample_grad.cuh"
 #include "sm100_stage.cuh"
 
 namespace d2c {
@@ -489,194 +489,6 @@ dcol_sm100_split_kernel(const DcolParams p) {
   }
 }
 
-// Tap positions per dim of the dilation-field variant, by value (a kernel parameter: no copy to the device).
-struct FieldAxes {
-  float pos[3][kMaxFieldKernelDim];
-};
-
-// ---- (b) sampling gradient + scatter ---------------------------------------------------------------
-
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  // volatile (must not be dropped) but no memory clobber: read-only loads may move across it
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d));
-}
-
-// Block = 32 voxels of one (clip, offset group) -- blockIdx.y -- times 8 threads per voxel; thread j owns
-// channels [8j, 8j+8) of each 64-channel slice.  The block walks the K taps; the record and the gradient
-// columns of tap t+1 are requested before tap t is processed, so the HBM stream of dcol (slice-major:
-// 8 KB contiguous per block and slice) stays in flight behind the L2 gathers and reductions.
-// kF32X: the channels-last staging of x is fp32 (fp32-parity mode) instead of fp16.
-// kNarrow: 32 channels per offset group.  The gradient columns keep their 64-channel
-// slices, each now holding two neighbouring groups; a block still serves one (clip, group) and its threads
-// own channels [4j, 4j+4) of the group's half of the slice.
-template <bool FieldOut, bool kF32X, bool kNarrow = false>
-__global__ void __launch_bounds__(256, kF32X ? 2 : 3)
-sample_grad_taps_kernel(Geom g, ClStrides cs, int b0, int nh, const float4* __restrict__ recs,
-                        const float* __restrict__ dcol, const void* __restrict__ x_cl_v, bool has_mask,
-                        float* __restrict__ grad_coord, float* __restrict__ grad_mask, float* __restrict__ gx_cl,
-                        int field_nch, int3 field_ch, const __grid_constant__ FieldAxes field_axes, int taps_per_block,
-                        HeadCfg head) {
-  const int j = threadIdx.x & 7;
-  const int v = blockIdx.x * 32 + (threadIdx.x >> 3);
-  const int grp = blockIdx.y % g.G, bl = blockIdx.y / g.G;
-  const int b = b0 + bl;
-  const bool active = v < g.V;
-  const int vc = active ? v : g.V - 1;                       // clamped: inactive threads load valid memory
-  const long long S = kNarrow ? (long long)(g.G / 2) * g.K : (long long)g.G * g.K * nh;
-  const float4* recp = recs + (((long long)b * g.G + grp) * g.K) * g.V + vc;
-  // thread j owns channels [4j, 4j+4) and [32+4j, 32+4j+4) of a slice: one warp-wide 16-byte access then
-  // covers whole 32-byte sectors (two lanes each), which halves the sector operations of the reductions
-  const float* dp = kNarrow
-      ? dcol + (((long long)bl * S + (long long)(grp >> 1) * g.K) * g.V + vc) * 64 + (grp & 1) * 32 + j * 4
-      : dcol + (((long long)bl * S + (long long)grp * g.K * nh) * g.V + vc) * 64 + j * 4;
-  const long long slice_stride = (long long)g.V * 64;
-  using XT = typename std::conditional<kF32X, float, __half>::type;
-  const XT* xb = reinterpret_cast<const XT*>(x_cl_v) + (long long)b * g.Vin * g.Cin;
-  float* gxb = gx_cl + (long long)b * g.Vin * g.Cin;
-  const int chbase = grp * g.cpg + j * 4;
-
-  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  float fsum[3] = {0.f, 0.f, 0.f};
-  auto ld_cols = [&](const float* q, float4& a, float4& b) {
-    a = __ldg(reinterpret_cast<const float4*>(q));
-    b = kNarrow ? zero4 : __ldg(reinterpret_cast<const float4*>(q + 32));
-  };
-  const int tap_beg = blockIdx.z * taps_per_block, tap_end = min(g.K, tap_beg + taps_per_block);
-  float4 rec_n = __ldg(recp + (long long)tap_beg * g.V);
-  float4 d0_n, d1_n;
-  ld_cols(dp + (long long)tap_beg * nh * slice_stride, d0_n, d1_n);
-  for (int tap = tap_beg; tap < tap_end; ++tap) {
-    const float4 rec = rec_n;
-    float4 d0 = d0_n, d1 = d1_n;
-    if (tap + 1 < tap_end) {
-      rec_n = __ldg(recp + (long long)(tap + 1) * g.V);
-      ld_cols(dp + (long long)(tap + 1) * nh * slice_stride, d0_n, d1_n);
-    }
-    const float m = rec.w;
-    const Sample<float> s = make_sample(g, rec.x, rec.y, rec.z);
-    // scatter weights of the reference's col2im: (1-|z-zp|)(1-|y-yp|)(1-|x-xp|), corners at distance
-    // exactly 1 excluded (dconv3d_gpu.cu:626-637)
-    const float wz[2] = {sub_rn(1.f, s.fz), sub_rn(1.f, s.gz)};
-    const float wy[2] = {sub_rn(1.f, s.fy), sub_rn(1.f, s.gy)};
-    const float wx[2] = {sub_rn(1.f, s.fx), sub_rn(1.f, s.gx)};
-    const bool okz[2] = {true, s.gz < 1.f}, oky[2] = {true, s.gy < 1.f}, okx[2] = {true, s.gx < 1.f};
-    unsigned valid = active ? s.valid : 0u;
-    if constexpr (FieldOut && (kF32X || !kNarrow)) {
-      // A tap at the kernel's centre on an axis does not move along it: the upper corners of that axis weigh nothing and the
-      // axis takes no gradient, so they are not read (4.6 corners a tap instead of 8 with 3 x 3 x 3 taps).  Not where a thread
-      // has 4 channels of fp16: it issues its loads either way (a corner left out reads the stand-in below), and finding out
-      // which to leave out costs it more than the cache hits give back and its registers spill.  256 channels, bf16 mode: 8
-      // groups on 8 x 120 x 214 9.13 ms with the skip, 8.15 without; one group (8 channels a thread) on 2 x 8 x 60 x 107 2.03 and 2.07.
-      const int k = tap % g.kw, jj = (tap / g.kw) % g.kh, i = tap / (g.kw * g.kh);
-      if (field_axes.pos[0][i] == 0.f && !okz[1]) valid &= 0x0fu;
-      if (field_axes.pos[1][jj] == 0.f && !oky[1]) valid &= 0x33u;
-      if (field_axes.pos[2][k] == 0.f && !okx[1]) valid &= 0x55u;
-    }
-    const int off0 = ((s.z0 * g.H + s.y0) * g.W + s.x0) * g.Cin + chbase;
-    float G[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) G[q] = 0.f;
-    for (int h = 0; h < nh; ++h) {
-      if (h > 0) {
-        ld_cols(dp + ((long long)tap * nh + h) * slice_stride, d0, d1);
-      }
-      // corner values of this thread's 8 channels ([4j, 4j+4) and [32+4j, 32+4j+4)), as loaded.  fp16 staging:
-      // the loads are unconditional -- a corner outside the volume reads the clip's first voxel instead and its
-      // dot product is discarded by a select after the slice loop (a select, so a non-finite stand-in cannot
-      // leak); measured 0.13 ms per step faster than predicated loads.  fp32 staging: predicated loads (twice
-      // the bytes per corner; fetching the stand-ins measured 0.08 ms slower).
-      uint4 c[8], chi[kF32X ? 8 : 1];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int off_in = off0 + h * 64 + (q >> 2) * cs.dz + ((q >> 1) & 1) * cs.dy + (q & 1) * cs.dx;
-        if constexpr (kF32X) {
-          if ((valid >> q) & 1u) {
-            c[q] = ptx::ldg_nc_v4(xb + off_in);
-            chi[q] = kNarrow ? make_uint4(0u, 0u, 0u, 0u) : ptx::ldg_nc_v4(xb + off_in + 32);
-          } else {
-            c[q] = chi[q] = make_uint4(0u, 0u, 0u, 0u);
-          }
-        } else {
-          const int off = ((valid >> q) & 1u) ? off_in : chbase + h * 64;
-          const uint2 lo = ptx::ldg_nc_v2(xb + off);
-          const uint2 hi = kNarrow ? make_uint2(0u, 0u) : ptx::ldg_nc_v2(xb + off + 32);
-          c[q] = make_uint4(lo.x, lo.y, hi.x, hi.y);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int dz = q >> 2, dy = (q >> 1) & 1, dx = q & 1;
-        if constexpr (kF32X) {
-          if constexpr (kNarrow)
-            G[q] += d0.x * __uint_as_float(c[q].x) + d0.y * __uint_as_float(c[q].y) +
-                    d0.z * __uint_as_float(c[q].z) + d0.w * __uint_as_float(c[q].w);
-          else
-            G[q] += d0.x * __uint_as_float(c[q].x) + d0.y * __uint_as_float(c[q].y) +
-                    d0.z * __uint_as_float(c[q].z) + d0.w * __uint_as_float(c[q].w) +
-                    d1.x * __uint_as_float(chi[q].x) + d1.y * __uint_as_float(chi[q].y) +
-                    d1.z * __uint_as_float(chi[q].z) + d1.w * __uint_as_float(chi[q].w);
-        } else {
-          const float2 x0 = __half22float2(bits_h2(c[q].x)), x1 = __half22float2(bits_h2(c[q].y));
-          const float2 x2 = __half22float2(bits_h2(c[q].z)), x3 = __half22float2(bits_h2(c[q].w));
-          if constexpr (kNarrow)
-            G[q] += d0.x * x0.x + d0.y * x0.y + d0.z * x1.x + d0.w * x1.y;
-          else
-            G[q] += d0.x * x0.x + d0.y * x0.y + d0.z * x1.x + d0.w * x1.y + d1.x * x2.x + d1.y * x2.y +
-                    d1.z * x3.x + d1.w * x3.y;
-        }
-        if (((valid >> q) & 1u) && okz[dz] && oky[dy] && okx[dx]) {
-          const float sw = mul_rn(mul_rn(wz[dz], wy[dy]), wx[dx]) * m;
-          float* dst = gxb + (off0 + h * 64 + dz * cs.dz + dy * cs.dy + dx * cs.dx);
-          red_add_v4(dst, sw * d0.x, sw * d0.y, sw * d0.z, sw * d0.w);
-          if (!kNarrow) red_add_v4(dst + 32, sw * d1.x, sw * d1.y, sw * d1.z, sw * d1.w);
-        }
-      }
-    }
-    // channel reduction of the 8 corner dot-products across the voxel's 8 threads (corners outside: zero)
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      if (!kF32X) G[q] = ((valid >> q) & 1u) ? G[q] : 0.f;
-      G[q] += __shfl_xor_sync(0xffffffffu, G[q], 1);
-      G[q] += __shfl_xor_sync(0xffffffffu, G[q], 2);
-      G[q] += __shfl_xor_sync(0xffffffffu, G[q], 4);
-    }
-    if (active && j == 0) {
-      float wts[3];
-      coord_weights(G, s, wts);    // linear in the corner values: applies to the channel-summed corners
-      // head.*_bstride != 0: the gradients go into the gradient of the predictor's raw output (clip stride = all of
-      // its channels), the mask's through the derivative of its activation (taken from the activated value m)
-      if (has_mask && grad_mask) {
-        float a[8];
-        sample_weights(s, a);
-        const long long ri = head.mask_bstride ? (long long)b * head.mask_bstride + ((long long)grp * g.K + tap) * g.V + v
-                                               : (((long long)b * g.G + grp) * g.K + tap) * g.V + v;
-        grad_mask[ri] = s.inside ? blend(G, a) * mask_act_slope(head.mask_act, m) : 0.f;
-      }
-      if constexpr (!FieldOut) {
-        float* go = grad_coord + (head.geo_bstride ? (long long)b * head.geo_bstride + ((long long)grp * 3 * g.K + 3 * tap) * g.V + v
-                                                   : (((long long)b * g.G + grp) * 3 * g.K + 3 * tap) * g.V + v);
-        go[0] = m * wts[0];
-        go[g.V] = m * wts[1];
-        go[2 * (long long)g.V] = m * wts[2];
-      } else {
-        // the field's gradient sums over taps (and groups): taps are summed here, one atomic per group after
-        const int k = tap % g.kw, jj = (tap / g.kw) % g.kh, i = tap / (g.kw * g.kh);
-        fsum[0] += field_axes.pos[0][i] * (m * wts[0]);
-        fsum[1] += field_axes.pos[1][jj] * (m * wts[1]);
-        fsum[2] += field_axes.pos[2][k] * (m * wts[2]);
-      }
-    }
-  }
-  if constexpr (FieldOut) {
-    if (active && j == 0) {
-      float* gs = grad_coord + (long long)b * (head.geo_bstride ? head.geo_bstride : (long long)field_nch * g.V) + v;
-      if (field_ch.x >= 0) atomicAdd(gs + (long long)field_ch.x * g.V, fsum[0]);
-      if (field_ch.y >= 0) atomicAdd(gs + (long long)field_ch.y * g.V, fsum[1]);
-      if (field_ch.z >= 0) atomicAdd(gs + (long long)field_ch.z * g.V, fsum[2]);
-    }
-  }
-}
-
 // ---- (c) channels-last fp32 -> NCDHW ----------------------------------------------------------------
 // The staging of x the other way round, with the same reasons: 16-byte loads, all requested before the first is stored.
 // 512 channels, 2 x 8 x 30 x 54: 37 us with 32 x 32 tiles and 4-byte loads, now 18.
@@ -864,31 +676,34 @@ int run_bwd(const Geom& g, bool x3, const Coords& coords, unsigned long long cap
       dcol_sm100_kernel<0><<<(unsigned)grid, kDcolThreads, pl.smem_bytes, st>>>(p);
     D2C_LAUNCH_CHECK();
     prof_mark(st, "bwd_sample_grad");
-    // A block walks the taps of its 32 voxels one after the other (about 1.7 us per tap while the GPU is not full: two
-    // dependent L2 round trips); small volumes share them out over up to nine blocks so that every multiprocessor has
-    // its two or three blocks.  1024-voxel layer, 27 taps: 46.9 us with one block per 32 voxels, 10.6 us with nine.
-    const long long vblocks = (long long)((g.V + 31) / 32) * nbc * g.G;
+    // A block lists and adds up the contributions of 32 voxels; the more taps it has, the more of them meet.  Small volumes share
+    // the taps out over up to nine blocks, so that every multiprocessor has its three (256 channels on 8 x 15 x 27: 107 us with
+    // three, six or twelve a multiprocessor asked for; 64 channels on 4 x 16 x 16: 17.6 us with nine blocks, 19.5 with 14).
+    const long long vblocks = (long long)((g.V + kSgVox - 1) / kSgVox) * nbc * g.G;
     int tap_split = (int)((3LL * sm_count + vblocks - 1) / vblocks);
     if (tap_split > 9) tap_split = 9;
+    if (tap_split < (g.K + kSgMaxTaps - 1) / kSgMaxTaps) tap_split = (g.K + kSgMaxTaps - 1) / kSgMaxTaps;
     if (tap_split > g.K) tap_split = g.K;
     const int taps_per_block = (g.K + tap_split - 1) / tap_split;
-    dim3 sgrid((unsigned)((g.V + 31) / 32), (unsigned)(nbc * g.G), (unsigned)((g.K + taps_per_block - 1) / taps_per_block));
-    if (pl.pairg && x3)
-      sample_grad_taps_kernel<FieldOut, true, true><<<sgrid, 256, 0, st>>>(g, cs, b0, pl.nh, recs, dcol, x_cl,
-                                                                           mask != nullptr, grad_coord, grad_mask,
-                                                                           gx_cl, field_nch, field_ch, axes, taps_per_block, head);
-    else if (pl.pairg)
-      sample_grad_taps_kernel<FieldOut, false, true><<<sgrid, 256, 0, st>>>(g, cs, b0, pl.nh, recs, dcol, x_cl,
-                                                                            mask != nullptr, grad_coord, grad_mask,
-                                                                            gx_cl, field_nch, field_ch, axes, taps_per_block, head);
-    else if (x3)
-      sample_grad_taps_kernel<FieldOut, true><<<sgrid, 256, 0, st>>>(g, cs, b0, pl.nh, recs, dcol, x_cl,
-                                                                     mask != nullptr, grad_coord, grad_mask, gx_cl,
-                                                                     field_nch, field_ch, axes, taps_per_block, head);
+    dim3 sgrid((unsigned)((g.V + kSgVox - 1) / kSgVox), (unsigned)(nbc * g.G), (unsigned)((g.K + taps_per_block - 1) / taps_per_block));
+    const size_t smem = sample_grad_smem(taps_per_block, pl.nh);
+    auto launch = [&](auto f32x, auto narrow, auto multi) -> int {
+      constexpr auto kernel = sample_grad_taps_kernel<FieldOut, decltype(f32x)::value, decltype(narrow)::value, decltype(multi)::value>;
+      const int rc = allow_dynamic_smem<kernel>((int)smem);
+      if (rc) return rc;
+      kernel<<<sgrid, kSgThreads, smem, st>>>(g, voxel_order(g), cs, b0, pl.nh, recs, dcol, x_cl, mask != nullptr, grad_coord, grad_mask,
+                                              gx_cl, field_nch, field_ch, axes, taps_per_block, head);
+      return D2C_OK;
+    };
+    const std::true_type yes;
+    const std::false_type no;
+    if (pl.pairg)
+      rc = x3 ? launch(yes, yes, no) : launch(no, yes, no);
+    else if (pl.nh > 1)
+      rc = x3 ? launch(yes, no, yes) : launch(no, no, yes);
     else
-      sample_grad_taps_kernel<FieldOut, false><<<sgrid, 256, 0, st>>>(g, cs, b0, pl.nh, recs, dcol, x_cl,
-                                                                      mask != nullptr, grad_coord, grad_mask, gx_cl,
-                                                                      field_nch, field_ch, axes, taps_per_block, head);
+      rc = x3 ? launch(yes, no, no) : launch(no, no, no);
+    if (rc) return rc;
     D2C_LAUNCH_CHECK();
   }
   if constexpr (FieldOut) {
