@@ -330,13 +330,12 @@ dw_sm100_kernel(const DwParams p) {
           if constexpr (kX3) {
             float w[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // rows past the clip end: stage bytes are stale
             if (r < rows) {
-              const uint2 w01 = *reinterpret_cast<const uint2*>(rec_stage + r * 48 + 8);
-              const uint4 w25 = *reinterpret_cast<const uint4*>(rec_stage + r * 48 + 16);
-              const uint2 w67 = *reinterpret_cast<const uint2*>(rec_stage + r * 48 + 32);
-              w[0] = __uint_as_float(w01.x); w[1] = __uint_as_float(w01.y);
-              w[2] = __uint_as_float(w25.x); w[3] = __uint_as_float(w25.y);
-              w[4] = __uint_as_float(w25.z); w[5] = __uint_as_float(w25.w);
-              w[6] = __uint_as_float(w67.x); w[7] = __uint_as_float(w67.y);
+              const uint4 w03 = *reinterpret_cast<const uint4*>(rec_stage + r * 48 + 16);
+              const uint4 w47 = *reinterpret_cast<const uint4*>(rec_stage + r * 48 + 32);
+              w[0] = __uint_as_float(w03.x); w[1] = __uint_as_float(w03.y);
+              w[2] = __uint_as_float(w03.z); w[3] = __uint_as_float(w03.w);
+              w[4] = __uint_as_float(w47.x); w[5] = __uint_as_float(w47.y);
+              w[6] = __uint_as_float(w47.z); w[7] = __uint_as_float(w47.w);
             }
             // channels 32 sl + 4j .. + 3 of the slice: 16-byte chunk 4 sl + j/2, half j&1; hi tile, lo tile
             const uint32_t in_tile = (uint32_t)((r >> 3) * 1024 + (r & 7) * 128) +

@@ -19,16 +19,15 @@
 // dealt round-robin instead: the CTAs then work on consecutive tiles, whose sampling neighbourhoods
 // overlap.
 //
-// Per CTA, 24 warps in warpgroup-aligned roles (deform_sm100_fwd_kernel.cuh):
+// Per CTA, 32 warps (deform_sm100_fwd_kernel.cuh):
 //   warps 0-3   epilogue: tcgen05.ld the 128 x N accumulator, add bias, store / reduce NCDHW
 //   warp  4     one thread issues tcgen05.mma and the commits that free the stages
 //   warp  5     one thread streams pre-swizzled weight slices with cp.async.bulk
 //   warp  6     one thread bulk-copies each unit's gather records into the record ring and writes the unit
 //               header (staging offset of the slice, valid rows), so the producers do no index arithmetic
-//   warp  7     idle (completes the warpgroup)
-//   warps 8-23  gather producers: unit header + gather record from the shared-memory record ring, 32 bytes of every corner
-//               that weighs anything, the next unit's loads issued half by half as the current unit's corners are blended
-//               (setmaxnreg moves registers from warps 0-7 to these), blend, bf16 pack, swizzled st.shared of the A tile
+//   warp  7     looks up whether x holds a NaN
+//   warps 8-31  gather producers, 8 rows at a time: unit header + gather record from the shared-memory record ring, 32 bytes of
+//               every corner that weighs anything, blend, bf16 pack, swizzled st.shared of the A tile
 // Stage hand-off is by mbarriers; every wait in the kernel's own code is bounded (sm100_ptx.cuh).
 //
 // Two math modes share the kernel (template parameter): single-pass bf16 (64-channel units, fp16 staging) and

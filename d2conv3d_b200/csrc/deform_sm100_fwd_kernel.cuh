@@ -1,7 +1,5 @@
 // The single-CTA forward kernel (included by deform_sm100_fwd.cu, whose constants, FwdParams and gather helpers it
-// uses).  Warp roles are aligned to warpgroups (4 epilogue warps | MMA, weight loader, record loader, one idle warp
-// | 16 gather warps) so that `setmaxnreg` can move registers from the light roles to the gather warps, whose loop
-// is software-pipelined at row granularity (see the producer branch).
+// uses).  Warps: 4 epilogue | MMA, weight loader, record loader, one idle | 24 gather, of 64 registers a thread each.
 // Optional instrumentation (compiled in with -DD2C_UNIT_TRACE, `python -m d2conv3d_b200.build --unit-trace`): every
 // role of ONE CTA stamps clock64() at fixed points of its per-unit loop for a window of 64 units, and every CTA
 // records its start / end (globaltimer), its SM and its unit count.  Read with `python -m d2conv3d_b200.unit_trace`.
@@ -17,8 +15,9 @@
 #define D2C_TR(role, k, e) ((void)0)
 #endif
 
-constexpr int kThreadsFwd = 24 * 32;
-static_assert(128 * 56 + 128 * 40 + 512 * 96 <= kThreadsFwd * 80, "setmaxnreg budget exceeds the CTA's register allocation");
+constexpr int kThreadsFwd = 32 * 32;
+constexpr int kGatherWarpsFwd = 24;
+constexpr int kUnitItems = kBM / 8;               // a gather warp's item: 8 rows of a unit
 constexpr int kMmaWarpFwd = 4, kLoadWarpFwd = 5, kRecWarpFwd = 6, kIdleWarpFwd = 7, kGatherWarp0Fwd = 8;
 
 // kX3 = 0: math mode bf16 (a unit is 64 channels of one tap, one bf16 operand pair).
@@ -63,8 +62,7 @@ fwd_sm100_kernel(const FwdParams p) {
   const Geom& g = p.g;
   // A CTA's work is n_parts (<= 16) contiguous unit ranges, one inside every clip (cta_part_range in
   // deform_sm100_fwd.cu); ring slots, phases and segment counters run on across the parts, positions restart at every
-  // part.  Thread 0 puts the ranges into shared memory once, so that the roles (some of them left with 40 registers)
-  // do no 64-bit division.
+  // part.  Thread 0 puts the ranges into shared memory once, so that the roles do no 64-bit division.
   // (unit indices fit 31 bits: checked by the host)
   int* part_tab = reinterpret_cast<int*>(base_ptr + bar_off + 256);      // [part][beg, end], the total, whether x holds a NaN
   // Large volumes (FwdParams::rr): whole tiles dealt round-robin instead -- at any time the CTAs then work on
@@ -96,9 +94,9 @@ fwd_sm100_kernel(const FwdParams p) {
       }
     }
     part_tab[32] = total;
-    for (int s = 0; s < kAStages; ++s) { ptx::mbar_init(a_full(s), kGatherWarps); ptx::mbar_init(a_empty(s), 1); }
+    for (int s = 0; s < kAStages; ++s) { ptx::mbar_init(a_full(s), kUnitItems); ptx::mbar_init(a_empty(s), 1); }
     for (int s = 0; s < p.b_stages; ++s) { ptx::mbar_init(b_full(s), 1); ptx::mbar_init(b_empty(s), 1); }
-    for (int s = 0; s < kRStages; ++s) { ptx::mbar_init(r_full(s), 1); ptx::mbar_init(r_empty(s), kGatherWarps); }
+    for (int s = 0; s < kRStages; ++s) { ptx::mbar_init(r_full(s), 1); ptx::mbar_init(r_empty(s), kUnitItems); }
     ptx::mbar_init(acc_full, 1);
     ptx::mbar_init(acc_empty, kEpiWarps);
     *abort_flag = 0;
@@ -116,14 +114,8 @@ fwd_sm100_kernel(const FwdParams p) {
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  // Register re-balancing between the roles (warpgroup-wide, first statement of each role's branch): the epilogue
-  // and service warps give registers back, the gather warps take them, so that a gather thread can hold the corner
-  // loads of TWO rows in flight while it blends.  The increase is served from what the CTA itself gave back: the CTA
-  // is launched with 768 x 80 = 61440 registers and 128*56 + 128*40 + 512*96 = 61440 (asking for more would make
-  // the increase wait for registers that never come).
   if (warp < kEpiWarps) {
     // ===================== epilogue: one pass per tile segment =====================
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     int seg = 0;
     for (int part = 0; part < p.n_parts; ++part) {
     if (*abort_flag) break;
@@ -203,7 +195,6 @@ fwd_sm100_kernel(const FwdParams p) {
     }
     }
   } else if (warp < kGatherWarp0Fwd) {
-   asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
    if (warp == kMmaWarpFwd) {
     // ===================== MMA issuer =====================
     if (lane == 0) {
@@ -325,6 +316,9 @@ fwd_sm100_kernel(const FwdParams p) {
         const int sr = k & (kRStages - 1);
         D2C_TR(0, k, 0);
         if (!ptx::mbar_wait(r_empty(sr), ((k / kRStages) & 1) ^ 1, abort_flag, 200)) break;
+        // A gather warp leaves out one unit at most between two items, so that it may wait for unit k when it has seen k - 2.  The
+        // parity it waits for is that of k only if the stage's last copy, k - 4, is there: copies are started in that order.
+        if (k >= 2 && !ptx::mbar_wait(r_full((k - 2) % kRStages), ((k - 2) / kRStages) & 1, abort_flag)) break;
         D2C_TR(0, k, 1);
         const int rows = min(kBM, g.V - v0);
         // unit header for the gather warps (no index arithmetic there); ordered before their reads by the
@@ -386,142 +380,106 @@ fwd_sm100_kernel(const FwdParams p) {
     }
    }
   } else {
-    // ===================== gather producers (software-pipelined) =====================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
-    // A thread owns 32 bytes (a quarter) of one row's 128: 8 fp32 or 16 fp16 channels, so that one record, one header and
-    // eight addresses serve 32 bytes of every corner and a row's 16-byte chunks of the A tile need no exchange between lanes.
-    // The corners of unit k+1 are requested half by half (z floor, z ceil) as soon as the same half of unit k is blended:
-    // 64 registers of corners are all in flight while the thread waits, half of them under each blend.
-    // Bound by the load pipe (l1tex__data_pipe_lsu_wavefronts: 73 % of the elapsed cycles at 512 channels, 2 x 8 x 30 x 54,
-    // samples kept; profiles/forward_gather_kernels.md).  With 16 bytes of two rows per thread and unit, twice the records,
-    // addresses and waits, it took 1.40 ms there, now 1.33; 256-channel field layer, 2 x 8 x 60 x 107: 2.20 ms, now 1.86.
-    const int t = threadIdx.x - kGatherWarp0Fwd * 32;
-    const int j = t & 3;             // 32-byte quarter of the row
+    // ===================== gather producers =====================
+    // An item is 8 rows of a unit; a warp takes every 24th.  A thread owns 32 bytes (a quarter) of one row's 128: 8 fp32 or 16 fp16
+    // channels, so that one record, one header and eight addresses serve 32 bytes of every corner and a row's 16-byte chunks of the
+    // A tile need no exchange between lanes.  The corners of the z ceil half are requested as those of the z floor half are blended.
+    // Bound by the latency of an item's chain (record, corners, corners, tile) over the warps there are: 24 warps that hold four
+    // corners beat 16 that hold eight and look a unit ahead, whose instructions between loads added up instead of overlapping
+    // (without its loads that kernel took half its time, with them half as much again).  Measured, 16 / 24 warps: 256-channel
+    // field layer of one group on 2 x 8 x 60 x 107 1.36 / 1.27 ms, of eight groups on 8 x 120 x 214 2.99 / 2.55, 1024 -> 256
+    // channels in 8 groups on 8 x 30 x 54 single pass 404 / 368 us, 512 channels in 8 groups on 2 x 8 x 30 x 54 1.06 / 1.04 ms, single
+    // pass 0.50 / 0.48.  The last 3 % of it is one 8-byte read of the record that does not wait for the header.  Not faster:
+    // corners of the next item requested under the blend (+6 %), the hand-over put off under the next item's loads, two slices
+    // of one record an item (spills), the voxels of a tile in bricks (half the requests hit L1, but a request with one miss runs
+    // at the rate of a miss).
+    const int j = lane & 3;          // 32-byte quarter of the row
     // the two rows of a quarter warp (one shared-memory store phase) differ in the bit that keeps their chunks apart:
     // fp32-parity stores chunk j, then 4 + j (rows r and r + 4); single pass stores chunks 2j and 2j + 1 (rows r and r + 1)
-    const int rr = (t >> 2) & 7;
-    const int r = (t >> 5) * 8 + (kX3 ? (rr >> 1) | ((rr & 1) << 2) : rr);
-    const uint32_t n_my_units = (uint32_t)part_tab[32];
-    const uint32_t row_off = (uint32_t)((r >> 3) * 1024 + (r & 7) * 128);
-    const uint32_t chunk0 = (uint32_t)(((kX3 ? j : 2 * j) ^ (r & 7)) << 4), chunk1 = (uint32_t)(((kX3 ? 4 + j : 2 * j + 1) ^ (r & 7)) << 4);
+    const int r8 = kX3 ? ((lane >> 3) & 3) | ((lane & 4)) : lane >> 2;
+    const uint32_t chunk0 = (uint32_t)(((kX3 ? j : 2 * j) ^ r8) << 4), chunk1 = (uint32_t)(((kX3 ? 4 + j : 2 * j + 1) ^ r8) << 4);
     const uint64_t pol_stream = ptx::l2_evict_first();
     using XT = typename std::conditional<kX3 != 0, float, __half>::type;
-    // dual: the second half of a row (channels 32-63 of the unit) belongs to the second offset group
-    const int rec_row = r * 48 + ((kDual && !kShared && j >= 2) ? kRecBytes : 0);
+    const uint32_t n_items = (uint32_t)part_tab[32] * kUnitItems;
 
-    // unit k + 1: base address of the thread's corners, steps along the axes, corner bits, whether the row exists, image word
-    const XT* p0 = reinterpret_cast<const XT*>(p.x_cl);
-    int dx = 0, dy = 0, dz = 0, word_n = 0;
-    uint32_t bits = 0;
-    bool live_n = false;
-    auto locate = [&](uint32_t k) {
-      const uint8_t* st = base_ptr + rec_off + (k % kRStages) * kRStage;
-      const uint4 hdr = *reinterpret_cast<const uint4*>(st + hdr_off);         // {staging offset, rows, image word}
-      live_n = r < (int)hdr.z;
-      word_n = (int)hdr.w;
-      uint2 head = make_uint2(0u, 0u);
-      if (live_n) head = *reinterpret_cast<const uint2*>(st + rec_row);
-      bits = head.y;
-      dx = (bits & 1u) ? p.cs.dx : 0; dy = (bits & 2u) ? p.cs.dy : 0; dz = (bits & 4u) ? p.cs.dz : 0;
-      p0 = reinterpret_cast<const XT*>(p.x_cl) + (long long)(((uint64_t)hdr.y << 32) | hdr.x) + j * (kX3 ? 8 : 16) + head.x;
-    };
-    auto issue_half = [&](int z, uint32_t (&c)[4][8]) {
-      const XT* q = z ? p0 + dz : p0;
-      ptx::ldg_nc_v8_if(c[0], q, bits & (z ? 128u : 8u));
-      ptx::ldg_nc_v8_if(c[1], q + dx, bits & (z ? 256u : 16u));
-      ptx::ldg_nc_v8_if(c[2], q + dy, bits & (z ? 512u : 32u));
-      ptx::ldg_nc_v8_if(c[3], q + dy + dx, bits & (z ? 1024u : 64u));
-    };
-    // corner order 000..111, as the reference's interpolation chain; rows past the clip end have weight zero (their records
-    // are stale bytes)
-    uint64_t acc2[4];                // fp32-parity: 8 channels
-    __half2 acch[8];                 // single pass: 16 channels
-    auto blend_half = [&](int z, const uint8_t* rec, bool live, const uint32_t (&c)[4][8]) {
-      if constexpr (kX3) {
-        float w[4] = {0.f, 0.f, 0.f, 0.f};
-        if (live) {
-          const float2 a = *reinterpret_cast<const float2*>(rec + (z ? 24 : 8)), b = *reinterpret_cast<const float2*>(rec + (z ? 32 : 16));
-          w[0] = a.x; w[1] = a.y; w[2] = b.x; w[3] = b.y;
-        }
+    uint32_t c[4][8];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          uint64_t w2;
-          asm("mov.b64 %0, {%1, %1};" : "=l"(w2) : "f"(w[q]));
+    for (int q = 0; q < 4; ++q)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            uint64_t c2;
-            asm("mov.b64 %0, {%1, %2};" : "=l"(c2) : "r"(c[q][2 * e]), "r"(c[q][2 * e + 1]));
-            if (z == 0 && q == 0) acc2[e] = 0ull;
-            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc2[e]) : "l"(c2), "l"(w2));
-          }
-        }
-      } else {
-        uint4 w = make_uint4(0u, 0u, 0u, 0u);
-        if (live) w = *reinterpret_cast<const uint4*>(rec + (z ? 32 : 16));
-        const uint32_t wq[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            if (z == 0 && q == 0) acch[e] = __float2half2_rn(0.f);
-            acch[e] = __hfma2(bits_h2(c[q][e]), bits_h2(wq[q]), acch[e]);
-          }
-      }
-    };
+      for (int e = 0; e < 8; ++e) c[q][e] = 0u;
 #ifdef D2C_UNIT_TRACE
-    const int trole = lane != 0 ? -1 : (warp == kGatherWarp0Fwd ? 3 : (warp == kGatherWarp0Fwd + 15 ? 4 : -1));
+    const int trole = lane != 0 ? -1 : (warp == kGatherWarp0Fwd ? 3 : (warp == kGatherWarp0Fwd + kGatherWarpsFwd - 1 ? 4 : -1));
 #define D2C_TG(e) do { if (trole >= 0) D2C_TR(trole, k, e); } while (0)
 #else
 #define D2C_TG(e) ((void)0)
 #endif
-
-    uint32_t c0[4][8], c1[4][8];
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) c0[q][e] = c1[q][e] = 0u;
-    bool ok = true;
-    if (n_my_units > 0) {
-      ok = ptx::mbar_wait(r_full(0), 0, abort_flag);
-      if (ok) {
-        locate(0);
-        issue_half(0, c0);
-        issue_half(1, c1);
-      }
-    }
     // Corners that weigh nothing are not read, and blended with weight zero: their registers hold zero or a corner of an earlier
-    // unit, of which only a NaN would show.  Where x holds a NaN they are cleared, in a loop of its own.  256 channels, field
-    // layer of one group, 2 x 8 x 60 x 107, inference, without / with that / always cleared / cleared where a blended sample is
-    // NaN: 1.371 / 1.376 / 1.495 / 1.404 ms; as a branch in one loop 1.383.
+    // item, of which only a NaN would show.  Where x holds a NaN they are cleared, in a loop of its own (in one loop, or always, it
+    // cost 1 to 9 % of the kernel).
     auto work = [&](auto clear) {
-    for (uint32_t k = 0; ok && k < n_my_units; ++k) {
+    for (uint32_t i = (uint32_t)(warp - kGatherWarp0Fwd); i < n_items; i += kGatherWarpsFwd) {
+      const uint32_t k = i / kUnitItems;
       const int sr = k % kRStages, sa = k % kAStages;
-      const uint8_t* st = base_ptr + rec_off + sr * kRStage;
-      const uint8_t* rec = st + rec_row;
-      const bool live = live_n, more = k + 1 < n_my_units;
-      [[maybe_unused]] const int word = word_n;
+      const int r = (int)(i % kUnitItems) * 8 + r8;
       D2C_TG(0);
-      blend_half(0, rec, live, c0);
+      if (!ptx::mbar_wait(r_full(sr), (k / kRStages) & 1, abort_flag)) break;
       D2C_TG(1);
-      if (more) {
-        if (!ptx::mbar_wait(r_full((k + 1) % kRStages), ((k + 1) / kRStages) & 1, abort_flag)) break;
-        D2C_TG(2);
-        locate(k + 1);
-        issue_half(0, c0);
-      }
-      D2C_TG(3);
-      blend_half(1, rec, live, c1);
-      if (more) issue_half(1, c1);
-      D2C_TG(4);
-      if constexpr (clear) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (!(bits & (8u << q))) ptx::clear_v8(c0[q]);
-          if (!(bits & (128u << q))) ptx::clear_v8(c1[q]);
+      const uint8_t* st = base_ptr + rec_off + sr * kRStage;
+      const uint8_t* rec = st + r * 48 + ((kDual && !kShared && j >= 2) ? kRecBytes : 0);
+      const uint4 hdr = *reinterpret_cast<const uint4*>(st + hdr_off);         // {staging offset, rows, image word}
+      const uint2 head = *reinterpret_cast<const uint2*>(rec);
+      const bool live = r < (int)hdr.z;
+      const uint32_t bits = live ? head.y : 0u;      // rows past the clip end have stale records: nothing is read for them
+      const int dx = (bits & 1u) ? p.cs.dx : 0, dy = (bits & 2u) ? p.cs.dy : 0, dz = (bits & 4u) ? p.cs.dz : 0;
+      const XT* p0 = reinterpret_cast<const XT*>(p.x_cl) + (long long)(((uint64_t)hdr.y << 32) | hdr.x) + j * (kX3 ? 8 : 16) + head.x;
+      auto load = [&](int z, int q) {
+        if constexpr (clear) {
+          if (!(bits & (8u << (4 * z + q)))) ptx::clear_v8(c[q]);
         }
-      }
+        ptx::ldg_nc_v8_if(c[q], p0 + (z ? dz : 0) + ((q & 2) ? dy : 0) + ((q & 1) ? dx : 0), bits & (8u << (4 * z + q)));
+      };
+#pragma unroll
+      for (int q = 0; q < 4; ++q) load(0, q);
+      D2C_TG(2);
+      auto weights = [&](int z) {
+        uint4 w = make_uint4(0u, 0u, 0u, 0u);
+        if (live) w = *reinterpret_cast<const uint4*>(rec + (z ? 32 : 16));
+        return w;
+      };
+      // corner order 000..111, as the reference's interpolation chain; rows past the clip end have weight zero (their records
+      // are stale bytes)
+      uint64_t acc2[4];                // fp32-parity: 8 channels
+      __half2 acch[8];                 // single pass: 16 channels
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc2[e] = 0ull;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acch[e] = __float2half2_rn(0.f);
+      auto blend = [&](uint32_t w, const uint32_t (&cc)[8]) {
+        if constexpr (kX3) {
+          uint64_t w2;
+          asm("mov.b64 %0, {%1, %1};" : "=l"(w2) : "r"(w));
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            uint64_t c2;
+            asm("mov.b64 %0, {%1, %2};" : "=l"(c2) : "r"(cc[2 * e]), "r"(cc[2 * e + 1]));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc2[e]) : "l"(c2), "l"(w2));
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acch[e] = __hfma2(bits_h2(cc[e]), bits_h2(w), acch[e]);
+        }
+      };
+      uint4 w = weights(0);
+      blend(w.x, c[0]); load(1, 0);
+      blend(w.y, c[1]); load(1, 1);
+      blend(w.z, c[2]); load(1, 2);
+      blend(w.w, c[3]); load(1, 3);
+      D2C_TG(3);
+      w = weights(1);
       float m = 1.f;
       if constexpr (kShared) m = live ? *reinterpret_cast<const float*>(st + kRecBytes + ((kDual && j >= 2) ? kMaskBytes : 0) + r * 4) : 0.f;
+      blend(w.x, c[0]); blend(w.y, c[1]); blend(w.z, c[2]); blend(w.w, c[3]);
+      D2C_TG(4);
       uint4 o0, o1;                  // chunk0, chunk1
       if constexpr (kX3) {
         uint32_t h[4], l[4];
@@ -548,6 +506,7 @@ fwd_sm100_kernel(const FwdParams p) {
       }
       if (!ptx::mbar_wait(a_empty(sa), ((k / kAStages) & 1) ^ 1, abort_flag)) break;
       D2C_TG(5);
+      const uint32_t row_off = (uint32_t)(r * 128);
       const uint32_t row = a_base + sa * kAStageBytes + row_off;
       ptx::sts_v4(row + chunk0, o0);
       ptx::sts_v4(row + chunk1, o1);
@@ -562,10 +521,11 @@ fwd_sm100_kernel(const FwdParams p) {
         // where the thread's bytes go in the kept image: block = (tile, 64-voxel block, slice) in the single-pass mode;
         // (tile, 64-voxel block, slice pair, {hi, lo}, slice of the pair) in the hi/lo mode, where a 64-channel row holds this
         // unit's 32 channels in its half `word & 1`, and the lo block lies two blocks further
+        const int word = (int)hdr.w;
         const uint32_t in_blk = row_off & 8191u;
         if constexpr (kX3) {
           uint8_t* sd = p.sav + ((long long)((word >> 1) + (r >> 6) * p.sav_np * 4) << 13) + in_blk +
-                        (uint32_t)(((4 * (word & 1) + j) ^ (r & 7)) << 4);
+                        (uint32_t)(((4 * (word & 1) + j) ^ r8) << 4);
           ptx::stg_v4_hint(sd, o0, pol_stream);
           ptx::stg_v4_hint(sd + (2 << 13), o1, pol_stream);
         } else {

@@ -19,8 +19,8 @@
 //                the same (readable) voxel;
 //                bit 3 + j set when corner j has a weight other than zero
 //        wj    = half2 {a_j*mask, a_j*mask}: trilinear weight x modulation, rounded to fp16, duplicated; ZERO
-//                for every corner that does not contribute to the forward sample.  In the fp32-parity mode
-//                the same 48 bytes hold {voff, steps, w0, w1}, w2..w5, {w6, w7, -, -} with fp32 weights.
+//                for every corner that does not contribute to the forward sample.  fp32 a_j*mask in
+//                the fp32-parity mode
 // A dilation field gives all offset groups the same positions: with more than one group its forward takes the record once per
 // (clip, tap, voxel), with the plain weights, and the activated modulation separately (fp32 [B][G][K][V padded to 4]), which the
 // producer multiplies the blended sample by.  Eight groups: 80 instead of 384 bytes written and read per tap and voxel.
@@ -101,9 +101,9 @@ sample_records_kernel(Geom g, Coords coords, const float* __restrict__ mask, lon
         uint32_t weighs = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) weighs |= (f[j] << 1) ? 8u << j : 0u;      // +-0 alike
-        o[0] = make_uint4((uint32_t)voff, steps | weighs, f[0], f[1]);
-        o[1] = make_uint4(f[2], f[3], f[4], f[5]);
-        o[2] = make_uint4(f[6], f[7], 0u, 0u);
+        o[0] = make_uint4((uint32_t)voff, steps | weighs, 0u, 0u);
+        o[1] = make_uint4(f[0], f[1], f[2], f[3]);
+        o[2] = make_uint4(f[4], f[5], f[6], f[7]);
       } else {
         uint32_t w[8];
 #pragma unroll

@@ -9,12 +9,12 @@ import sys
 
 import numpy as np
 
-ROLES = ["record loader", "weight loader", "MMA issuer", "gather warp 0", "gather warp 15"]
+ROLES = ["record loader", "weight loader", "MMA issuer", "first gather warp", "last gather warp"]
 STAMPS = [
     ["loop top", "stage free"],
     ["loop top", "stage free"],
     ["loop top", "A tile full", "weights full", "MMAs issued", "commits issued"],
-    ["unit begins", "z floor half blended", "next records there", "next z floor requested", "z ceil blended, requested",
+    ["item begins", "records there", "z floor requested", "z floor blended, z ceil requested", "z ceil blended",
      "A stage free", "A tile stored", "arrived (copy kept)"],
 ]
 STAMPS.append(STAMPS[3])
