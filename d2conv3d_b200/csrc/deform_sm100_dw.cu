@@ -382,8 +382,8 @@ dw_sm100_kernel(const DwParams p) {
 constexpr int kSvThreads = 7 * 32;        // 4 epilogue warps, MMA issuer, grad_out loader, sample loader
 constexpr int kSvLoadWarp = 5, kSvSampleWarp = 6;
 constexpr int kSvBlkBytes = 8192;         // one 64-channel slice x 64 voxels
-constexpr int kSvBStages = 5;
-constexpr int kSvARingBytes = 64 * 1024;  // 4 stages of 16 KB (bf16) or 2 stages of 32 KB (bf16x3)
+constexpr int kSvBStagesOf(int two) { return two ? 3 : 5; }
+constexpr int kSvARingOf(int two) { return (two ? 128 : 64) * 1024; }   // 4 stages (bf16) or 2 stages (bf16x3) of one or two pairs
 
 struct DwSavedParams {
   const uint8_t* sav;        // sample image, see FwdParams::sav
@@ -392,10 +392,15 @@ struct DwSavedParams {
   int N, S, NCH, n_pairs, n_tiles, tiles_per_split, tmem_cols;
 };
 
-template <int kX3>
+// kTwo = 1 (at most 256 output channels): a CTA takes two slice pairs, whose accumulators share tensor memory.  What streams into
+// shared memory per MMA is what bounds a CTA with one pair of 256 outputs -- per 64 voxels 96 KB for 12 MMAs in the fp32-parity mode,
+// 48 KB for 4 in the single-pass mode, at 70 to 90 bytes a clock -- and its MMAs all go into the same columns; two pairs share
+// grad_out (128 KB for 24, 64 KB for 8) and alternate.  256 -> 256 channels, one group, 2 x 8 x 60 x 107: 1.11 ms with one pair, 0.86 with two; single pass 0.47, 0.33.
+template <int kX3, int kTwo>
 __global__ void __launch_bounds__(kSvThreads, 1)
 dw_saved_sm100_kernel(const DwSavedParams p) {
-  constexpr int kAStage = (kX3 ? 4 : 2) * kSvBlkBytes;
+  constexpr int kPairBytes = (kX3 ? 4 : 2) * kSvBlkBytes, kAStage = (1 + kTwo) * kPairBytes;
+  constexpr int kSvARingBytes = kSvARingOf(kTwo), kSvBStages = kSvBStagesOf(kTwo);
   constexpr int kASt = kSvARingBytes / kAStage;
   constexpr int kParts = kX3 ? 2 : 1;                 // grad_out image groups per block: hi, lo
   extern __shared__ uint8_t smem_raw[];
@@ -414,7 +419,8 @@ dw_saved_sm100_kernel(const DwSavedParams p) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + bar_off + 8 * (9 + 2 * kSvBStages) + 4);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pair = blockIdx.x % p.n_pairs, split = blockIdx.x / p.n_pairs;
+  const int items = (p.n_pairs + kTwo) / (1 + kTwo), split = blockIdx.x / items;
+  const int pair = (blockIdx.x - split * items) * (1 + kTwo), my_pairs = min(1 + kTwo, p.n_pairs - pair);
   const int tile_beg = split * p.tiles_per_split;
   const int tile_end = min(p.n_tiles, tile_beg + p.tiles_per_split);
   const int n_blocks = 2 * (tile_end - tile_beg);      // 64-voxel blocks; may be <= 0 for a trailing split
@@ -442,25 +448,30 @@ dw_saved_sm100_kernel(const DwSavedParams p) {
       if (ptx::mbar_wait(acc_full, 0, abort_flag, 1000)) {
         ptx::tc_fence_after();
         const int m = warp * 32 + lane;
-        const int s = 2 * pair + (m >> 6);
-        float* row = p.dws + ((long long)s * 64 + (m & 63)) * p.N;
-        for (int c0 = 0; c0 < p.N; c0 += 32) {
-          uint32_t r[32];
-          ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
-          ptx::tmem_ld_wait();
-          if (s < p.S) {
+        for (int pr = 0; pr < my_pairs; ++pr) {
+          const int s = 2 * (pair + pr) + (m >> 6);
+          float* row = p.dws + ((long long)s * 64 + (m & 63)) * p.N;
+          for (int c0 = 0; c0 < p.N; c0 += 32) {
+            uint32_t r[32];
+            ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(pr * (p.tmem_cols >> 1) + c0), r);
+            ptx::tmem_ld_wait();
+            if (s < p.S) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(row + c0 + 4 * i),
-                           "f"(__uint_as_float(r[4 * i])), "f"(__uint_as_float(r[4 * i + 1])),
-                           "f"(__uint_as_float(r[4 * i + 2])), "f"(__uint_as_float(r[4 * i + 3]))
-                           : "memory");
+              for (int i = 0; i < 8; ++i)
+                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(row + c0 + 4 * i),
+                             "f"(__uint_as_float(r[4 * i])), "f"(__uint_as_float(r[4 * i + 1])),
+                             "f"(__uint_as_float(r[4 * i + 2])), "f"(__uint_as_float(r[4 * i + 3]))
+                             : "memory");
+            }
           }
         }
         ptx::tc_fence_before();
       }
     } else if (warp == kMmaWarp) {
       if (lane == 0) {
+        // accumulators that consecutive MMAs alternate between: 256-column ranges of the outputs, or the two pairs
+        const int n_acc = kTwo ? my_pairs : p.NCH;
+        const uint32_t acc_step = kTwo ? (uint32_t)(p.tmem_cols >> 1) : 256u;
         int sb = 0;
         uint32_t phb = 0;
         bool ok = true;
@@ -491,25 +502,30 @@ dw_saved_sm100_kernel(const DwSavedParams p) {
             for (int k4 = 0; k4 < 4; ++k4) {
               // A: 16 voxels from voxel k4*16 of the block = two 8-row groups of 1024 bytes (SBO); the second
               // slice of the pair (rows 64..127 of M) lies one 8 KB image further (LBO)
-              const uint64_t a_hi = ptx::umma_desc_mnmajor_sw128(a_stage + k4 * 2048, kSvBlkBytes, 1024);
-              const uint64_t a_lo = ptx::umma_desc_mnmajor_sw128(a_stage + 2 * kSvBlkBytes + k4 * 2048, kSvBlkBytes, 1024);
+              uint64_t a_hi[2], a_lo[2];
+#pragma unroll
+              for (int c = 0; c < 2; ++c) {
+                const uint32_t at = a_stage + k4 * 2048 + (kTwo ? c * kPairBytes : 0);
+                a_hi[c] = ptx::umma_desc_mnmajor_sw128(at, kSvBlkBytes, 1024);
+                a_lo[c] = ptx::umma_desc_mnmajor_sw128(at + 2 * kSvBlkBytes, kSvBlkBytes, 1024);
+              }
               const uint32_t acc = (kb > 0 || k4 > 0) ? 1u : 0u;
               if (!kX3 || part == 0) {
 #pragma unroll
                 for (int c = 0; c < 2; ++c)                                                  // a (a_hi) * g (g_hi)
-                  if (c < p.NCH)
-                    ptx::umma_bf16(tmem_base + (uint32_t)(256 * c), a_hi, bdesc0[c] + (uint64_t)(2 * k4), idesc[c], acc);
+                  if (c < n_acc)
+                    ptx::umma_bf16(tmem_base + acc_step * (uint32_t)c, a_hi[c], bdesc0[kTwo ? 0 : c] + (uint64_t)(2 * k4), idesc[kTwo ? 0 : c], acc);
                 if (kX3) {
 #pragma unroll
                   for (int c = 0; c < 2; ++c)                                                // a_lo * g_hi
-                    if (c < p.NCH)
-                      ptx::umma_bf16(tmem_base + (uint32_t)(256 * c), a_lo, bdesc0[c] + (uint64_t)(2 * k4), idesc[c], 1u);
+                    if (c < n_acc)
+                      ptx::umma_bf16(tmem_base + acc_step * (uint32_t)c, a_lo[c], bdesc0[kTwo ? 0 : c] + (uint64_t)(2 * k4), idesc[kTwo ? 0 : c], 1u);
                 }
               } else {
 #pragma unroll
                 for (int c = 0; c < 2; ++c)                                                  // a_hi * g_lo
-                  if (c < p.NCH)
-                    ptx::umma_bf16(tmem_base + (uint32_t)(256 * c), a_hi, bdesc0[c] + (uint64_t)(2 * k4), idesc[c], 1u);
+                  if (c < n_acc)
+                    ptx::umma_bf16(tmem_base + acc_step * (uint32_t)c, a_hi[c], bdesc0[kTwo ? 0 : c] + (uint64_t)(2 * k4), idesc[kTwo ? 0 : c], 1u);
               }
             }
 #pragma unroll
@@ -548,15 +564,16 @@ dw_saved_sm100_kernel(const DwSavedParams p) {
     } else if (warp == kSvSampleWarp) {
       // ---- kept samples: the slice pair's images of every 64-voxel block of the range
       if (lane == 0) {
-        const long long blk_stride = (long long)p.n_pairs * kAStage;   // bytes between consecutive blocks
-        const uint8_t* src = p.sav + (long long)tile_beg * 2 * blk_stride + (long long)pair * kAStage;
+        const long long blk_stride = (long long)p.n_pairs * kPairBytes;   // bytes between consecutive blocks
+        const uint8_t* src = p.sav + (long long)tile_beg * 2 * blk_stride + (long long)pair * kPairBytes;
+        const uint32_t bytes = (uint32_t)(my_pairs * kPairBytes);
         int kb = 0;
         const uint64_t pol_stream = ptx::l2_evict_first();    // every byte of the image is read exactly once
         for (; kb < n_blocks; ++kb) {
           const int sa = kb % kASt;
           if (!ptx::mbar_wait(a_empty(sa), ((kb / kASt) & 1) ^ 1, abort_flag, 100)) break;
-          ptx::mbar_arrive_expect_tx(a_full(sa), (uint32_t)kAStage);
-          ptx::bulk_g2s_hint(a_base + sa * kAStage, src, (uint32_t)kAStage, a_full(sa), pol_stream);
+          ptx::mbar_arrive_expect_tx(a_full(sa), bytes);
+          ptx::bulk_g2s_hint(a_base + sa * kAStage, src, bytes, a_full(sa), pol_stream);
           src += blk_stride;
         }
         for (int w = (kb > kASt ? kb - kASt : 0); w < kb; ++w) {
@@ -644,12 +661,11 @@ bool make_dw_plan(const Geom& g, int sm_count, bool x3, DwPlan* dp) {
   return true;
 }
 
-// Work split of the saved-samples kernel: (slice pair, voxel range) items, at least two waves of them, ranges of at
+// Work split of the saved-samples kernel: (slice pair, or two of them, voxel range) items, at least two waves of them, ranges of at
 // least 8 tiles (fewer where there would not be an item for every multiprocessor), the smallest count whose last wave is at
 // least 95 % full (else the fullest); the fp32-parity mode ends an accumulation chain after 27 tiles (24 accumulating MMAs
 // per tile and column range -> 648, see make_dw_plan).
-void split_saved(const DwPlan& dp, int sm_count, bool x3, int* tiles_per_split, int* nsplit_out) {
-  const int n_pairs = (dp.S + 1) / 2;
+void split_saved(const DwPlan& dp, int n_pairs, int sm_count, bool x3, int* tiles_per_split, int* nsplit_out) {
   const int chain_min = x3 ? (dp.n_tiles + 26) / 27 : 1;              // fewest ranges the chain cap allows
   // most ranges: of at least 8 tiles, or one item per multiprocessor
   const int size_max = std::max(std::max(1, dp.n_tiles / 8), std::min(dp.n_tiles, sm_count / n_pairs));
@@ -669,8 +685,8 @@ void split_saved(const DwPlan& dp, int sm_count, bool x3, int* tiles_per_split, 
   *nsplit_out = (dp.n_tiles + *tiles_per_split - 1) / *tiles_per_split;
 }
 
-constexpr int kSvSmemBytes = kSvARingBytes + kSvBStages * kChunkBytes + 256 + 1024;
-static_assert(kSvSmemBytes <= kSmemLimit, "saved-samples kernel: shared memory");
+constexpr int kSvSmemOf(int two) { return kSvARingOf(two) + kSvBStagesOf(two) * kChunkBytes + 256 + 1024; }
+static_assert(kSvSmemOf(0) <= kSmemLimit && kSvSmemOf(1) <= kSmemLimit, "saved-samples kernel: shared memory");
 
 }  // namespace
 
@@ -733,13 +749,18 @@ int sm100_dw(const Geom& g, bool x3, const float* gy, const void* x_cl, const vo
     sp.N = g.Cout; sp.S = dp.S; sp.NCH = dp.NCH; sp.n_pairs = (dp.S + 1) / 2; sp.n_tiles = dp.n_tiles;
     sp.tmem_cols = dp.tmem_cols;
     int nsplit = 1;
-    split_saved(dp, sm_count, x3, &sp.tiles_per_split, &nsplit);
+    // two pairs a CTA where every multiprocessor still gets two of them with eight tiles each
+    const bool two = g.Cout <= 256 && (long long)((sp.n_pairs + 1) / 2) * (dp.n_tiles / 8) >= 2LL * sm_count;
+    const int items = two ? (sp.n_pairs + 1) / 2 : sp.n_pairs, smem = kSvSmemOf(two);
+    if (two) sp.tmem_cols *= 2;
+    split_saved(dp, items, sm_count, x3, &sp.tiles_per_split, &nsplit);
     prof_mark(st, "bwd_dw_sm100_saved");
-    const int rc = x3 ? allow_dynamic_smem<dw_saved_sm100_kernel<1>>(kSvSmemBytes)
-                      : allow_dynamic_smem<dw_saved_sm100_kernel<0>>(kSvSmemBytes);
+    const int rc = x3 ? (two ? allow_dynamic_smem<dw_saved_sm100_kernel<1, 1>>(smem) : allow_dynamic_smem<dw_saved_sm100_kernel<1, 0>>(smem))
+                      : (two ? allow_dynamic_smem<dw_saved_sm100_kernel<0, 1>>(smem) : allow_dynamic_smem<dw_saved_sm100_kernel<0, 0>>(smem));
     if (rc) return rc;
-    auto kern = x3 ? dw_saved_sm100_kernel<1> : dw_saved_sm100_kernel<0>;
-    kern<<<sp.n_pairs * nsplit, kSvThreads, kSvSmemBytes, st>>>(sp);
+    auto kern = x3 ? (two ? dw_saved_sm100_kernel<1, 1> : dw_saved_sm100_kernel<1, 0>)
+                   : (two ? dw_saved_sm100_kernel<0, 1> : dw_saved_sm100_kernel<0, 0>);
+    kern<<<items * nsplit, kSvThreads, smem, st>>>(sp);
     D2C_LAUNCH_CHECK();
   } else {
     prof_mark(st, "bwd_dw_sm100");
