@@ -329,6 +329,22 @@ inline int allow_dynamic_smem(int bytes) {
   return D2C_OK;
 }
 
+// Kernels of one call that do not need one another's results may run at the same time: each lets the next one start as soon as all
+// its blocks have (launch_dependents), waits for the one before at its END, so that the end of the last means the end of all, and
+// the kernel that needs them waits before its first read.  The first of a call is launched the ordinary way.
+__device__ __forceinline__ void next_kernel_may_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void wait_for_kernels_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... Params, typename... Args>
+inline cudaError_t launch_beside(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // A buffer of 4-byte words that a staging kernel clears on the side, for a later kernel that accumulates into it (one
 // launch less than a memset of its own).  `block` of `blocks` clears its share.
 struct ZeroFill {

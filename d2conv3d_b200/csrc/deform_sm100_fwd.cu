@@ -139,6 +139,7 @@ __device__ __forceinline__ void cta_part_range(const FwdParams& p, int part, lon
 __global__ void __launch_bounds__(64)
 stage_weight_sw128_kernel(int Cout, int Cin, int K, int cpg, int nh, const float* __restrict__ w,
                           uint8_t* __restrict__ w_sw) {
+  next_kernel_may_start();
   extern __shared__ float wrow[];   // [64 channels][K]
   const int co = blockIdx.x, cblk = blockIdx.y;      // cblk: 64-channel block of Cin
   const int c0 = cblk * 64;
@@ -159,6 +160,7 @@ stage_weight_sw128_kernel(int Cout, int Cin, int K, int cpg, int nh, const float
                    ((jj ^ (co & 7)) << 4);
     *reinterpret_cast<uint4*>(dst) = out;
   }
+  if (threadIdx.x == 0) wait_for_kernels_before();
 }
 
 // bf16x3 mode: slice s = (grp*nh + h)*K + tap with nh = cpg/32 holds 32 channels; each row is
@@ -166,6 +168,7 @@ stage_weight_sw128_kernel(int Cout, int Cin, int K, int cpg, int nh, const float
 __global__ void __launch_bounds__(64)
 stage_weight_sw128_x3_kernel(int Cout, int Cin, int K, int cpg, int nh, const float* __restrict__ w,
                              uint8_t* __restrict__ w_sw) {
+  next_kernel_may_start();
   extern __shared__ float wrow[];   // [32 channels][K]
   const int co = blockIdx.x, cblk = blockIdx.y;      // cblk: 32-channel block of Cin
   const int c0 = cblk * 32;
@@ -191,6 +194,7 @@ stage_weight_sw128_x3_kernel(int Cout, int Cin, int K, int cpg, int nh, const fl
                    ((jj ^ (co & 7)) << 4);
     *reinterpret_cast<uint4*>(dst) = out;
   }
+  if (threadIdx.x == 0) wait_for_kernels_before();
 }
 
 struct Plan {
@@ -248,22 +252,30 @@ bool pick_variant(const Geom& g, int math_mode, bool* x3, Plan* pl, bool shared 
   return false;
 }
 
+// Calls of at most this many units per CTA start the kernel beside the last staging kernel, its set-up under that one's end: 256
+// channels on 8 x 15 x 27 (38 units) 84.7 us a call, 88.4 started after it (93.6 with all four kernels one after the other).  A
+// kernel started that way runs 3 % slower (1024 -> 256 channels on 8 x 30 x 54, 298 units, 505 instead of 494 us a call), more than
+// the start where it runs for long.
+constexpr int kMaxUnitsBeside = 64;
+
 template <int kX3, int kDual, int kSave, bool kMayShare>
 int launch_fwd(const FwdParams& p, unsigned grid, int smem_bytes, cudaStream_t st) {
+  auto start = [&](auto kernel) -> int {
+    if (p.n_units <= (long long)kMaxUnitsBeside * grid)
+      D2C_CUDA_TRY(launch_beside(kernel, grid, kThreadsFwd, smem_bytes, st, p));
+    else
+      kernel<<<grid, kThreadsFwd, smem_bytes, st>>>(p);
+    D2C_LAUNCH_CHECK();
+    return D2C_OK;
+  };
   if constexpr (kMayShare) {
     if (p.masks) {
       const int rc = allow_dynamic_smem<fwd_sm100_kernel<kX3, kDual, kSave, 1>>(smem_bytes);
-      if (rc) return rc;
-      fwd_sm100_kernel<kX3, kDual, kSave, 1><<<grid, kThreadsFwd, smem_bytes, st>>>(p);
-      D2C_LAUNCH_CHECK();
-      return D2C_OK;
+      return rc ? rc : start(fwd_sm100_kernel<kX3, kDual, kSave, 1>);
     }
   }
   const int rc = allow_dynamic_smem<fwd_sm100_kernel<kX3, kDual, kSave, 0>>(smem_bytes);
-  if (rc) return rc;
-  fwd_sm100_kernel<kX3, kDual, kSave, 0><<<grid, kThreadsFwd, smem_bytes, st>>>(p);
-  D2C_LAUNCH_CHECK();
-  return D2C_OK;
+  return rc ? rc : start(fwd_sm100_kernel<kX3, kDual, kSave, 0>);
 }
 
 template <typename Coords>
@@ -360,20 +372,19 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
   if (pair_clusters > 0) { sav = nullptr; pos = nullptr; x_cl = ws; }       // the CTA-pair kernel keeps nothing
   prof_mark(st, "fwd_stage_operands");
   {
-    if ((rc = launch_sample_records(g, coords, mask, head, pos, recs, st, x3, masks, nan_flag))) return rc;
+    // three kernels that need nothing of one another
+    if ((rc = launch_sample_records(g, coords, mask, head, pos, recs, st, x3, masks))) return rc;
     const ZeroFill zero_y{y, whole_tiles_only ? 0 : (long long)sizeof(float) * g.B * g.Cout * g.V};
     if (x3) {
-      if ((rc = launch_stage_input(g, x, reinterpret_cast<float*>(x_cl), zero_y, nan_flag, sm_count, st))) return rc;
-      dim3 wgrid((unsigned)g.Cout, (unsigned)(g.Cin / 32));
-      stage_weight_sw128_x3_kernel<<<wgrid, 64, 32 * g.K * sizeof(float), st>>>(g.Cout, g.Cin, g.K, g.cpg, pl.nh, w, w_sw);
-      D2C_LAUNCH_CHECK();
+      if ((rc = launch_stage_input(g, x, reinterpret_cast<float*>(x_cl), zero_y, nan_flag, sm_count, st, true))) return rc;
+      D2C_CUDA_TRY(launch_beside(stage_weight_sw128_x3_kernel, dim3((unsigned)g.Cout, (unsigned)(g.Cin / 32)), 64, 32 * g.K * sizeof(float),
+                                 st, g.Cout, g.Cin, g.K, g.cpg, pl.nh, w, w_sw));
     } else {
-      if ((rc = launch_stage_input(g, x, reinterpret_cast<__half*>(x_cl), zero_y, nan_flag, sm_count, st))) return rc;
-      dim3 wgrid((unsigned)g.Cout, (unsigned)(g.Cin / 64));
-      stage_weight_sw128_kernel<<<wgrid, 64, 64 * g.K * sizeof(float), st>>>(g.Cout, g.Cin, g.K,
-                                                                              pl.dual ? 64 : g.cpg, pl.nh, w, w_sw);
-      D2C_LAUNCH_CHECK();
+      if ((rc = launch_stage_input(g, x, reinterpret_cast<__half*>(x_cl), zero_y, nan_flag, sm_count, st, true))) return rc;
+      D2C_CUDA_TRY(launch_beside(stage_weight_sw128_kernel, dim3((unsigned)g.Cout, (unsigned)(g.Cin / 64)), 64, 64 * g.K * sizeof(float), st,
+                                 g.Cout, g.Cin, g.K, pl.dual ? 64 : g.cpg, pl.nh, w, w_sw));
     }
+    D2C_LAUNCH_CHECK();
   }
 
   FwdParams p;

@@ -103,12 +103,16 @@ fwd_sm100_kernel(const FwdParams p) {
     ptx::fence_mbar_init();
   }
   // by a warp without a role, beside the set-up (in the producers it would delay a call's first unit by up to 0.6 us)
-  if (threadIdx.x == kIdleWarpFwd * 32) part_tab[33] = __ldg(p.nan_flag);
+  if (threadIdx.x == kIdleWarpFwd * 32) {
+    wait_for_kernels_before();
+    part_tab[33] = __ldg(p.nan_flag) == kNanFound;
+  }
   if (warp == 0) {
     __syncwarp();
     ptx::tmem_alloc(ptx::smem_u32((const void*)tmem_slot), (uint32_t)p.tmem_cols);
     ptx::tmem_relinquish();
   }
+  wait_for_kernels_before();         // what was staged is there from here on
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();

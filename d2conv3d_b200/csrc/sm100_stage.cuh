@@ -18,15 +18,17 @@ __device__ __forceinline__ uint32_t pack_f16x2_sat(float lo, float hi) {
 
 // x [B][C][Vin] fp32 -> x_cl [B][Vin][C] channels-last: fp16 (saturating), or fp32 for the fp32-parity mode.  fp32: infinities are
 // replaced by the largest finite float (as the fp16 staging saturates).
-// `zero` is cleared on the side (the output that partial tiles are added to); nan_flag (nullable, zero before) is set where x
-// holds a NaN.
+// `zero` is cleared on the side (the output that partial tiles are added to); nan_flag (nullable) is set to kNanFound where x
+// holds a NaN; nothing clears it: a word that says so without cause only costs the forward its faster loop.
 // Bound by HBM.  Block: 64 channels x kVox voxels; all of a thread's loads are requested before the first is stored, and it
 // writes 16 bytes.  (8 loads and 4- or 8-byte writes a thread: fp32, 512 channels on 2 x 8 x 30 x 54 with the output cleared, 46 us,
 // now 26; fp16, 1024 channels on 8 x 30 x 54, 35 us, now 17.)
+constexpr int kNanFound = 0x4e614e21;
 template <typename T, int kVox>
 static __global__ void __launch_bounds__(256)
 stage_input_cl_kernel(int C, long long Vin, const float* __restrict__ x, T* __restrict__ x_cl, ZeroFill zero,
                       int* __restrict__ nan_flag) {
+  next_kernel_may_start();
   constexpr int kPer = 16 / sizeof(T);             // channels a thread writes
   constexpr int kLanes = 64 / kPer;                // threads per voxel
   __shared__ float tile[64][kVox + 1];
@@ -52,7 +54,7 @@ stage_input_cl_kernel(int C, long long Vin, const float* __restrict__ x, T* __re
       if (sizeof(T) == 4 && isinf(f[i])) f[i] = copysignf(3.402823466e+38f, f[i]);
       tile[ty + kRowsPass * i][tx] = f[i];
     }
-    if (nan && nan_flag) *nan_flag = 1;
+    if (nan && nan_flag) *nan_flag = kNanFound;
   }
   __syncthreads();
   const int q = threadIdx.x % kLanes, c = q * kPer;
@@ -70,18 +72,23 @@ stage_input_cl_kernel(int C, long long Vin, const float* __restrict__ x, T* __re
       *reinterpret_cast<float4*>(dst) = make_float4(tile[c][vv], tile[c + 1][vv], tile[c + 2][vv], tile[c + 3][vv]);
     }
   }
+  if (threadIdx.x == 0) wait_for_kernels_before();
 }
 
-// Blocks of 64 voxels, of 32 where that leaves multiprocessors without one.
+// Blocks of 64 voxels, of 32 where that leaves multiprocessors without one.  beside: may run at the same time as the kernel before.
 template <typename T>
 static int launch_stage_input(const Geom& g, const float* x, T* x_cl, const ZeroFill& zero, int* nan_flag, int sm_count,
-                              cudaStream_t st) {
-  const dim3 grid((unsigned)((g.Vin + 63) / 64), (unsigned)((g.Cin + 63) / 64), (unsigned)g.B);
-  if ((long long)grid.x * grid.y * grid.z >= 2LL * sm_count)
-    stage_input_cl_kernel<T, 64><<<grid, 256, 0, st>>>(g.Cin, g.Vin, x, x_cl, zero, nan_flag);
+                              cudaStream_t st, bool beside = false) {
+  dim3 grid((unsigned)((g.Vin + 63) / 64), (unsigned)((g.Cin + 63) / 64), (unsigned)g.B);
+  auto kernel = stage_input_cl_kernel<T, 64>;
+  if ((long long)grid.x * grid.y * grid.z < 2LL * sm_count) {
+    grid.x = (unsigned)((g.Vin + 31) / 32);
+    kernel = stage_input_cl_kernel<T, 32>;
+  }
+  if (beside)
+    D2C_CUDA_TRY(launch_beside(kernel, grid, 256, 0, st, g.Cin, g.Vin, x, x_cl, zero, nan_flag));
   else
-    stage_input_cl_kernel<T, 32><<<dim3((unsigned)((g.Vin + 31) / 32), grid.y, grid.z), 256, 0, st>>>(g.Cin, g.Vin, x, x_cl, zero,
-                                                                                                     nan_flag);
+    kernel<<<grid, 256, 0, st>>>(g.Cin, g.Vin, x, x_cl, zero, nan_flag);
   D2C_LAUNCH_CHECK();
   return D2C_OK;
 }

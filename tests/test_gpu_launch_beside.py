@@ -1,0 +1,61 @@
+"""The kernels of a tensor-core forward that run beside one another: calls one after the other on the same buffers, a call on each of
+two streams, capture into a graph and its replays on new inputs, a NaN in one call and none in the next (whose workspace may be the
+same memory).  Small calls, whose last kernel starts beside the staging too, and larger ones."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(64, 64, (4, 16, 16)), (256, 256, (8, 15, 27)), (256, 128, (8, 60, 70))]
+
+
+def problem(cin, cout, dims, seed):
+    gen = torch.Generator("cuda").manual_seed(seed)
+    rand = lambda *s: torch.randn(s, generator=gen, device="cuda")  # noqa: E731
+    return [rand(1, cin, *dims), 2 * rand(1, 81, *dims), torch.sigmoid(rand(1, 27, *dims)), rand(cout, cin, 3, 3, 3) * (27 * cin) ** -0.5,
+            rand(cout)]
+
+
+def close(a, b):
+    # the same kernels on the same inputs: partial tiles meet in another order
+    return float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
+
+
+@pytest.mark.parametrize("cin,cout,dims", SIZES)
+def test_calls_streams_and_graphs(cin, cout, dims):
+    from d2conv3d_b200 import _lib, dconv_native
+    call = lambda p: dconv_native.deform_conv3d(*p, 1, 1, 1, 1, 1)  # noqa: E731
+    p, q = problem(cin, cout, dims, 1), problem(cin, cout, dims, 2)
+    with torch.no_grad():
+        want = []
+        for s in (p, q):
+            want.append(call(s))
+            torch.cuda.synchronize()
+        for y, w in zip([call(s) for s in (p, q, p, q)], want + want):
+            assert close(y, w)
+        bad = [p[0].clone()] + p[1:]
+        bad[0][0, 0, 0, 0, 0] = float("nan")
+        y = call(bad)
+        assert torch.isnan(y).any()
+        del y
+        assert close(call(q), want[1])
+        side = [torch.cuda.Stream(), torch.cuda.Stream()]
+        got = [[], []]
+        torch.cuda.synchronize()
+        for _ in range(4):
+            for i, s in enumerate((p, q)):
+                with torch.cuda.stream(side[i]):
+                    got[i].append(call(s))
+        torch.cuda.synchronize()
+        for i in range(2):
+            assert all(close(y, want[i]) for y in got[i])
+        graph, into = torch.cuda.CUDAGraph(), [t.clone() for t in p]
+        with torch.cuda.graph(graph):
+            y = call(into)
+        for s, w in ((p, want[0]), (q, want[1]), (p, want[0])):
+            for a, b in zip(into, s):
+                a.copy_(b)
+            graph.replay()
+            torch.cuda.synchronize()
+            assert close(y, w)
+    _lib.device_status()
