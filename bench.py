@@ -219,10 +219,10 @@ def run_reference_arm(args):
 TRAFFIC_SOURCE = "ncu capture of this bench's C2 step, one launch per kernel, both math modes"
 TRAFFIC_PER_LAUNCH = {       # (phase, math mode) -> DRAM read + write bytes of one launch
     # the forward keeps its operand tiles for the weight gradient (sample cache): + 0.72 / 1.44 GB written
-    ("fwd_sm100_fused", "bf16"): 0.415e9 + 0.762e9, ("fwd_sm100_fused", "auto"): 2.198e9 + 1.657e9,
-    ("fwd_sm100_fused", "bf16x3"): 2.198e9 + 1.657e9,
-    ("bwd_sample_grad", "bf16"): 1.603e9 + 0.137e9, ("bwd_sample_grad", "auto"): 1.629e9 + 0.138e9,
-    ("bwd_sample_grad", "bf16x3"): 1.629e9 + 0.138e9,
+    ("fwd_sm100_fused", "bf16"): 0.417e9 + 0.765e9, ("fwd_sm100_fused", "auto"): 2.224e9 + 1.656e9,
+    ("fwd_sm100_fused", "bf16x3"): 2.224e9 + 1.656e9,
+    ("bwd_sample_grad", "bf16"): 1.464e9 + 0.136e9, ("bwd_sample_grad", "auto"): 1.539e9 + 0.139e9,
+    ("bwd_sample_grad", "bf16x3"): 1.539e9 + 0.139e9,
     ("bwd_dcol_sm100", "bf16"): 0.089e9 + 1.383e9, ("bwd_dcol_sm100", "auto"): 0.636e9 + 1.394e9,
     ("bwd_dcol_sm100", "bf16x3"): 0.636e9 + 1.394e9,
     ("bwd_dw_sm100_saved", "bf16"): 0.781e9 + 0.005e9, ("bwd_dw_sm100_saved", "auto"): 1.530e9 + 0.004e9,
@@ -231,13 +231,6 @@ TRAFFIC_PER_LAUNCH = {       # (phase, math mode) -> DRAM read + write bytes of 
     ("bwd_dw_sm100", "bf16"): 0.430e9 + 0.073e9, ("bwd_dw_sm100", "auto"): 0.592e9 + 0.127e9,
     ("bwd_dw_sm100", "bf16x3"): 0.592e9 + 0.127e9,
 }
-# The sampling-gradient kernel's real limiter: every live corner of every sample adds 64 fp32 channels into the
-# L2-resident grad_input accumulator.  payload_bytes = corners inside the volume for the benchmark's offsets
-# (5.69 of 8 per sample on average at sigma = 2 voxels, D = 8) x 5.6 M samples x 256 B; rate = what
-# red.global.add.v4.f32 sustains on this part for exactly this access pattern (microbenchmark, 11.5 GB in 1.69 ms).
-SCATTER = {"payload_bytes": 5.687 * 2 * 8 * 27 * 12960 * 256, "rate_gbs": 6773.0,
-           "source": "profiles/b200_l2_scatter_gather_rates.md, stand-alone measurement on a B200"}
-
 PHASE_WORK = {
     # phase name -> (bound, key of the algorithmic work of one launch)
     "fwd_sm100_fused": ("tensor", "F"), "fwd_generic": ("tensor", "F"),
@@ -624,14 +617,6 @@ def run_gpu_arm(args, impl="ours"):
                  "traffic_source": TRAFFIC_SOURCE,
                  "ms_per_launch": avg_ms / launches_per_step, "launches_per_step": launches_per_step,
                  "peak_source": peaks["source"] + (" (bf16 dense, sustained)" if bound == "tensor" else " (copy)")}
-            if name == "bwd_sample_grad":
-                # what actually bounds this kernel: fp32 vector reductions into the L2-resident grad_input
-                # accumulator; the payload and the sustained rate of such reductions are measured, see SCATTER
-                r["second_bound"] = {"what": "fp32 red.global.add.v4 payload into L2", "payload_bytes": SCATTER["payload_bytes"],
-                                     "measured_rate_gbs": SCATTER["rate_gbs"],
-                                     "floor_ms": SCATTER["payload_bytes"] / SCATTER["rate_gbs"] / 1e6,
-                                     "frac": SCATTER["payload_bytes"] / SCATTER["rate_gbs"] / 1e6 / (avg_ms / launches_per_step),
-                                     "source": SCATTER["source"]}
             return r
 
         phase_summary = {}
