@@ -102,10 +102,11 @@ fwd_sm100_kernel(const FwdParams p) {
     *abort_flag = 0;
     ptx::fence_mbar_init();
   }
-  // by a warp without a role, beside the set-up (in the producers it would delay a call's first unit by up to 0.6 us)
+  // by a warp without a role, beside the set-up (in the producers it would delay a call's first unit by up to 0.6 us).  A volatile
+  // load: the staging kernel may write the word while this one already runs, so that it is not read-only for this kernel's life.
   if (threadIdx.x == kIdleWarpFwd * 32) {
     wait_for_kernels_before();
-    part_tab[33] = __ldg(p.nan_flag) == kNanFound;
+    part_tab[33] = *static_cast<const volatile int*>(p.nan_flag) == kNanFound;
   }
   if (warp == 0) {
     __syncwarp();
@@ -440,7 +441,7 @@ fwd_sm100_kernel(const FwdParams p) {
         if constexpr (clear) {
           if (!(bits & (8u << (4 * z + q)))) ptx::clear_v8(c[q]);
         }
-        ptx::ldg_nc_v8_if(c[q], p0 + (z ? dz : 0) + ((q & 2) ? dy : 0) + ((q & 1) ? dx : 0), bits & (8u << (4 * z + q)));
+        ptx::ldg_v8_if(c[q], p0 + (z ? dz : 0) + ((q & 2) ? dy : 0) + ((q & 1) ? dx : 0), bits & (8u << (4 * z + q)));
       };
 #pragma unroll
       for (int q = 0; q < 4; ++q) load(0, q);

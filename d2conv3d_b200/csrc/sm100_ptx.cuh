@@ -326,11 +326,13 @@ __device__ __forceinline__ void ldg_nc_v4_or_zero(uint4& r, const void* p, uint3
       "@q ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
       : "=&r"(r.x), "=&r"(r.y), "=&r"(r.z), "=&r"(r.w) : "l"(p), "r"(cond));
 }
-// 32 bytes (32-byte aligned) under a predicate: r keeps its contents where cond is 0.
-__device__ __forceinline__ void ldg_nc_v8_if(uint32_t (&r)[8], const void* p, uint32_t cond) {
-  asm("{\n\t.reg .pred q;\n\t"
+// 32 bytes (32-byte aligned) under a predicate: r keeps its contents where cond is 0.  An ordinary load, in the program's order with
+// the waits: what it reads may be written by a kernel that runs beside this one until that kernel is waited for, so that it is not
+// read-only for this kernel's life, as ld.global.nc would promise.
+__device__ __forceinline__ void ldg_v8_if(uint32_t (&r)[8], const void* p, uint32_t cond) {
+  asm volatile("{\n\t.reg .pred q;\n\t"
       "setp.ne.u32 q, %9, 0;\n\t"
-      "@q ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
+      "@q ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
       : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
       : "l"(p), "r"(cond));
 }

@@ -1,8 +1,11 @@
 """The kernels of a tensor-core forward that run beside one another: calls one after the other on the same buffers, a call on each of
 two streams, capture into a graph and its replays on new inputs, a NaN in one call and none in the next (whose workspace may be the
 same memory).  Small calls, whose last kernel starts beside the staging too, and larger ones."""
+import numpy as np
 import pytest
 import torch
+
+from oracle import oracle as orc
 
 pytestmark = pytest.mark.gpu
 
@@ -58,4 +61,40 @@ def test_calls_streams_and_graphs(cin, cout, dims):
             graph.replay()
             torch.cuda.synchronize()
             assert close(y, w)
+    _lib.device_status()
+
+
+@pytest.mark.parametrize("mode", ["auto", "bf16"])
+@pytest.mark.parametrize("cin,cout,dims", SIZES[:2])
+def test_which_outputs_are_nan(mode, cin, cout, dims):
+    """Calls with and without a NaN in turn: the outputs whose samples give the voxel a weight are NaN in the one, and none but those
+    that read it with weight zero at most; none at all in the other."""
+    import d2conv3d_b200
+    from d2conv3d_b200 import _lib, dconv_native
+    p = problem(cin, cout, dims, 3)
+    at = tuple(d // 2 for d in dims)
+    bad = [p[0].clone()] + p[1:]
+    bad[0][(0, cin // 2) + at] = float("nan")
+
+    def reached(corners):
+        ind = np.zeros((1, 1) + dims)
+        for c in corners:
+            ind[(0, 0) + tuple(c)] = 1.0
+        geo, mask = (t.double().cpu().numpy() for t in p[1:3])
+        y = orc.deform_conv3d_fwd(ind, geo, mask, np.ones((1, 1, 3, 3, 3)), None, padding=1)
+        return torch.from_numpy(y > 0).cuda().expand(1, cout, *dims)
+
+    touched, allowed = reached([at]), reached([np.subtract(at, d) for d in np.ndindex(2, 2, 2)])
+    assert touched.any() and not allowed.all()
+    d2conv3d_b200.set_math_mode(mode)
+    try:
+        with torch.no_grad():
+            want = dconv_native.deform_conv3d(*p, 1, 1, 1, 1, 1)
+            for _ in range(4):
+                y = dconv_native.deform_conv3d(*bad, 1, 1, 1, 1, 1)
+                assert y[touched].isnan().all() and not y[~allowed].isnan().any()
+                assert float((y - want)[~allowed].abs().max()) <= 1e-5 * float(want.abs().max())
+                assert close(dconv_native.deform_conv3d(*p, 1, 1, 1, 1, 1), want)
+    finally:
+        d2conv3d_b200.set_math_mode("auto")
     _lib.device_status()
