@@ -372,8 +372,9 @@ int run_fwd(const Geom& g, int math_mode, const Coords& coords, const HeadCfg& h
   if (pair_clusters > 0) { sav = nullptr; pos = nullptr; x_cl = ws; }       // the CTA-pair kernel keeps nothing
   prof_mark(st, "fwd_stage_operands");
   {
-    // three kernels that need nothing of one another
-    if ((rc = launch_sample_records(g, coords, mask, head, pos, recs, st, x3, masks))) return rc;
+    // three kernels that need nothing of one another, but for the NaN word: the first clears it, the second may set it when the
+    // first is done
+    if ((rc = launch_sample_records(g, coords, mask, head, pos, recs, st, x3, masks, nan_flag))) return rc;
     const ZeroFill zero_y{y, whole_tiles_only ? 0 : (long long)sizeof(float) * g.B * g.Cout * g.V};
     if (x3) {
       if ((rc = launch_stage_input(g, x, reinterpret_cast<float*>(x_cl), zero_y, nan_flag, sm_count, st, true))) return rc;

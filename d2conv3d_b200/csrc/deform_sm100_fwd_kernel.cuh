@@ -106,7 +106,7 @@ fwd_sm100_kernel(const FwdParams p) {
   // load: the staging kernel may write the word while this one already runs, so that it is not read-only for this kernel's life.
   if (threadIdx.x == kIdleWarpFwd * 32) {
     wait_for_kernels_before();
-    part_tab[33] = *static_cast<const volatile int*>(p.nan_flag) == kNanFound;
+    part_tab[33] = *static_cast<const volatile int*>(p.nan_flag);
   }
   if (warp == 0) {
     __syncwarp();

@@ -51,12 +51,15 @@ __host__ __device__ inline int mask_row(int V) { return (V + 3) / 4 * 4; }
 
 // kShared: the coordinates do not depend on the offset group (dilation field): a thread serves one (voxel, tap)
 // and all groups, computing the position, corners and weights once and applying each group's modulation.
+// nan_flag (nullable): cleared for the staging of x, which sets it when this kernel is done (stage_input_cl_kernel).
 template <typename Coords, bool kShared>
 static __global__ void __launch_bounds__(256)
 sample_records_kernel(Geom g, Coords coords, const float* __restrict__ mask, long long mask_bstride, int mask_act,
-                      float4* __restrict__ pos, uint4* __restrict__ gat, int f32_weights, float* __restrict__ masks) {
+                      float4* __restrict__ pos, uint4* __restrict__ gat, int f32_weights, float* __restrict__ masks,
+                      int* __restrict__ nan_flag) {
   next_kernel_may_start();
   const int v = blockIdx.x * 256 + threadIdx.x;
+  if (nan_flag && v == 0 && blockIdx.y == 0 && blockIdx.z == 0) *nan_flag = 0;
   if (v >= g.V) return;
   const int tap = kShared ? blockIdx.y : blockIdx.y % g.K, b = blockIdx.z;
   const int grp_beg = kShared ? 0 : blockIdx.y / g.K, grp_end = kShared ? g.G : grp_beg + 1;
@@ -124,12 +127,12 @@ struct CoordsSharedAcrossGroups<FieldCoords<T>> { static constexpr bool value = 
 
 template <typename Coords>
 static int launch_sample_records(const Geom& g, const Coords& coords, const float* mask, const HeadCfg& head, float4* pos,
-                                 uint4* gat, cudaStream_t st, bool f32_weights = false, float* masks = nullptr) {
+                                 uint4* gat, cudaStream_t st, bool f32_weights = false, float* masks = nullptr, int* nan_flag = nullptr) {
   constexpr bool kShared = CoordsSharedAcrossGroups<Coords>::value;
   dim3 grid((unsigned)((g.V + 255) / 256), (unsigned)(kShared ? g.K : g.G * g.K), (unsigned)g.B);
   if (grid.y > 65535 || grid.z > 65535) return D2C_ERR_TOO_LARGE;
   sample_records_kernel<Coords, kShared><<<grid, 256, 0, st>>>(g, coords, mask, head.mask_bstride, head.mask_act, pos, gat,
-                                                              f32_weights ? 1 : 0, masks);
+                                                              f32_weights ? 1 : 0, masks, nan_flag);
   D2C_LAUNCH_CHECK();
   return D2C_OK;
 }

@@ -18,12 +18,11 @@ __device__ __forceinline__ uint32_t pack_f16x2_sat(float lo, float hi) {
 
 // x [B][C][Vin] fp32 -> x_cl [B][Vin][C] channels-last: fp16 (saturating), or fp32 for the fp32-parity mode.  fp32: infinities are
 // replaced by the largest finite float (as the fp16 staging saturates).
-// `zero` is cleared on the side (the output that partial tiles are added to); nan_flag (nullable) is set to kNanFound where x
-// holds a NaN; nothing clears it: a word that says so without cause only costs the forward its faster loop.
+// `zero` is cleared on the side (the output that partial tiles are added to); nan_flag (nullable) is set to 1 where x holds a NaN:
+// the kernel before, which this one may run beside, clears it, so it is set after the wait.
 // Bound by HBM.  Block: 64 channels x kVox voxels; all of a thread's loads are requested before the first is stored, and it
 // writes 16 bytes.  (8 loads and 4- or 8-byte writes a thread: fp32, 512 channels on 2 x 8 x 30 x 54 with the output cleared, 46 us,
 // now 26; fp16, 1024 channels on 8 x 30 x 54, 35 us, now 17.)
-constexpr int kNanFound = 0x4e614e21;
 template <typename T, int kVox>
 static __global__ void __launch_bounds__(256)
 stage_input_cl_kernel(int C, long long Vin, const float* __restrict__ x, T* __restrict__ x_cl, ZeroFill zero,
@@ -34,6 +33,7 @@ stage_input_cl_kernel(int C, long long Vin, const float* __restrict__ x, T* __re
   __shared__ float tile[64][kVox + 1];
   const int b = blockIdx.z, c0 = blockIdx.y * 64;
   const long long v0 = (long long)blockIdx.x * kVox;
+  bool nan = false;
   {
     constexpr int kRowsPass = 256 / kVox, kLoads = 64 / kRowsPass;
     const int tx = threadIdx.x % kVox, ty = threadIdx.x / kVox;
@@ -47,16 +47,14 @@ stage_input_cl_kernel(int C, long long Vin, const float* __restrict__ x, T* __re
     }
     zero_fill(zero, blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z),
               (long long)gridDim.x * gridDim.y * gridDim.z);
-    bool nan = false;
 #pragma unroll
     for (int i = 0; i < kLoads; ++i) {
       nan |= isnan(f[i]);
       if (sizeof(T) == 4 && isinf(f[i])) f[i] = copysignf(3.402823466e+38f, f[i]);
       tile[ty + kRowsPass * i][tx] = f[i];
     }
-    if (nan && nan_flag) *nan_flag = kNanFound;
   }
-  __syncthreads();
+  nan = __syncthreads_or(nan);
   const int q = threadIdx.x % kLanes, c = q * kPer;
 #pragma unroll
   for (int vv = threadIdx.x / kLanes; vv < kVox; vv += 256 / kLanes) {
@@ -72,7 +70,10 @@ stage_input_cl_kernel(int C, long long Vin, const float* __restrict__ x, T* __re
       *reinterpret_cast<float4*>(dst) = make_float4(tile[c][vv], tile[c + 1][vv], tile[c + 2][vv], tile[c + 3][vv]);
     }
   }
-  if (threadIdx.x == 0) wait_for_kernels_before();
+  if (threadIdx.x == 0) {
+    wait_for_kernels_before();
+    if (nan && nan_flag) *nan_flag = 1;
+  }
 }
 
 // Blocks of 64 voxels, of 32 where that leaves multiprocessors without one.  beside: may run at the same time as the kernel before.

@@ -98,3 +98,40 @@ def test_which_outputs_are_nan(mode, cin, cout, dims):
     finally:
         d2conv3d_b200.set_math_mode("auto")
     _lib.device_status()
+
+
+def test_nan_word_is_this_calls_own():
+    """The word by which a forward chooses its loop, in a workspace of the caller's that holds anything: it tells of this call's input,
+    not of what the memory held or of an earlier call, in replays of a graph too."""
+    import ctypes
+    import d2conv3d_b200
+    from d2conv3d_b200 import _lib
+    cin, cout, dims = SIZES[0]
+    x, offset, mask, w, bias = problem(cin, cout, dims, 4)
+    d = _lib.ConvDesc(dtype=_lib.F32, batch=1, in_channels=cin, out_channels=cout, in_d=dims[0], in_h=dims[1], in_w=dims[2], kd=3, kh=3,
+                      kw=3, stride_d=1, stride_h=1, stride_w=1, pad_d=1, pad_h=1, pad_w=1, dil_d=1, dil_h=1, dil_w=1, groups=1,
+                      offset_groups=1)
+    L = _lib.lib()
+    d2conv3d_b200.set_math_mode("auto")
+    n = L.d2c_workspace_bytes(_lib.OP_DEFORM_FWD, ctypes.byref(d))
+    records = 27 * dims[0] * dims[1] * dims[2] * 48                    # the word's 256 bytes lie before them, at the end
+    ws, y = torch.full((n,), 255, dtype=torch.uint8, device="cuda"), torch.empty(1, cout, *dims, device="cuda")
+    word = ws[n - records - 256:][:4].view(torch.int32)
+    clean, into = x.clone(), x.clone()
+
+    def call():
+        st = L.d2c_deform_conv3d_fwd(ctypes.byref(d), into.data_ptr(), offset.data_ptr(), mask.data_ptr(), w.data_ptr(), bias.data_ptr(),
+                                     y.data_ptr(), ws.data_ptr(), n, torch.cuda.current_stream().cuda_stream)
+        assert st == 0
+
+    x[0, 5, 1, 2, 3] = float("nan")
+    graph = torch.cuda.CUDAGraph()
+    side = torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=side):
+        call()
+    for run in (call, graph.replay):
+        for src, found in ((clean, 0), (x, 1), (clean, 0)):
+            into.copy_(src)
+            run()
+            assert int(word) == found
+    _lib.device_status()
