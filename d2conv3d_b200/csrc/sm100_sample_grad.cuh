@@ -150,13 +150,15 @@ sample_grad_taps_kernel(Geom g, VoxelOrder order, ClStrides cs, int b0, int nh, 
       const Sample<float> s = make_sample(g, rec[k].x, rec[k].y, rec[k].z);
       unsigned valid = active && k * 8 + warp < n_tap ? s.valid : 0u;
       if constexpr (FieldOut) {
-        // A tap at the kernel's centre on an axis does not move along it: the upper corners of that axis weigh nothing and the
-        // axis takes no gradient (4.6 corners a tap instead of 8 with 3 x 3 x 3 taps).
+        // A tap at the kernel's centre on an axis does not move along it, and no tap does where the field has no channel for the
+        // axis: the upper corners of that axis weigh nothing and the axis takes no gradient (with 3 x 3 x 3 taps 4.6
+        // corners a tap instead of 8, and 2.8 where the field scales rows and columns alone; the latter, one group of 256 channels
+        // on 2 x 8 x 30 x 54: 531 us with the first of the two rules alone, 374 with both, 494 with every corner reduced by itself).
         const int kx = tap % g.kw, ky = (tap / g.kw) % g.kh, kz = tap / (g.kw * g.kh);
         if (valid) {
-          if (field_axes.pos[0][kz] == 0.f && !(s.gz < 1.f)) valid &= 0x0fu;
-          if (field_axes.pos[1][ky] == 0.f && !(s.gy < 1.f)) valid &= 0x33u;
-          if (field_axes.pos[2][kx] == 0.f && !(s.gx < 1.f)) valid &= 0x55u;
+          if ((field_ch.x < 0 || field_axes.pos[0][kz] == 0.f) && !(s.gz < 1.f)) valid &= 0x0fu;
+          if ((field_ch.y < 0 || field_axes.pos[1][ky] == 0.f) && !(s.gy < 1.f)) valid &= 0x33u;
+          if ((field_ch.z < 0 || field_axes.pos[2][kx] == 0.f) && !(s.gx < 1.f)) valid &= 0x55u;
         }
       }
       corners[k] = valid;

@@ -92,6 +92,32 @@ def test_nan_voxel_stays_where_it_is_sampled(mode, field, keep, shape):
         assert near(a[~allowed.expand_as(a)], b[~allowed.expand_as(a)])
 
 
+@pytest.mark.parametrize("mode", ["auto", "bf16"])
+@pytest.mark.parametrize("field", ["x", "xy"])
+@pytest.mark.parametrize("cin,dims", [(64, (3, 7, 9)), (256, (6, 15, 27))])
+def test_corners_that_a_field_cannot_reach(mode, field, cin, dims):
+    """An axis without a channel in the field: every sample lies on a voxel along it, and the next one up is no corner of it.  A NaN
+    there leaves the gradients of the field and of the modulation alone."""
+    import d2conv3d_b200
+    p = make_problem(77, B=1, Cin=cin, Cout=64, dims=dims, k=3, padding=1, dtype=np.float32, field_mode=field, G=1)
+    at = (0, 5) + tuple(d // 2 for d in dims)
+    ind = np.zeros_like(p["x"], dtype=np.float64)
+    for d in np.ndindex(2, 2):                              # rows and columns have a channel, frames have none
+        ind[(0, 5) + tuple(np.subtract(at[2:], (0,) + d))] = 1.0
+    reached = cu(orc.dyn_dilated_conv3d_fwd(ind, p["geo"].astype(np.float64), p["mask"].astype(np.float64), np.ones(p["weight"].shape),
+                                            None, field, padding=1, offset_groups=1)[:, :1] > 0)
+    assert reached.any() and not reached.all()
+    x = p["x"].copy()
+    x[at] = np.nan
+    d2conv3d_b200.set_math_mode(mode)
+    try:
+        want, got = (_run(p, a, field, 1, True)[2] for a in (p["x"], x))
+    finally:
+        d2conv3d_b200.set_math_mode("auto")
+    for a, b in ((got[1], want[1]), (got[2], want[2])):
+        assert ((a - b).abs() <= 1e-5 * b.abs().max())[~reached.expand_as(a)].all()
+
+
 @pytest.mark.skipif(os.environ.get("D2C_SM100_PAIR") == "1", reason="already inside")
 def test_the_same_with_cta_pairs():
     """The opt-in pair kernel is chosen by an environment variable that the library reads once per process."""
