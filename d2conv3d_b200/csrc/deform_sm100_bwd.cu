@@ -5,13 +5,15 @@
 //                           rows so that the 64 channels of one (offset group, tap) slice are contiguous.
 //                           Replaces the reference's cuBLAS call at csrc/ops/dconv3d_gpu.cu:981-999.
 //   (b) sample_grad_taps_kernel  grad_offset / grad_mask and grad_input (channels-last fp32) from dcol; the contributions to an
-//                           input voxel are added up per block and leave it as one reduction (sm100_sample_grad.cuh).
+//                           input voxel are added up per block and leave it as one reduction, or, where few would meet or
+//                           weigh anything, each by itself (sample_grad_direct_kernel; sm100_sample_grad.cuh).
 //                           Replaces deformable_col2im_coord_gpu_kernel (:756-864) and
 //                           deformable_col2im_gpu_kernel (:562-643).
 //   (c) unstage_grad_input_kernel  channels-last fp32 -> NCDHW.
 //
 // The weight gradient is in deform_sm100_dw.cu; sampling positions come from the records of
 // sm100_gather.cuh, computed once per backward call.
+#include <algorithm>
 #include <type_traits>
 
 #include "deform_exact.h"   // slice_clips
@@ -34,6 +36,7 @@ constexpr int kDcolEpiWarps = 8;              // warp w: TMEM lane quarter w%4, 
 constexpr int kDcolMmaWarp = 8, kDcolLoadWarp = 9;
 constexpr int kDcolThreads = 320;
 constexpr int kSmemLimit = 227 * 1024;
+constexpr size_t kWordBytes = 256;            // of the workspace: the answer of PositionAsk
 
 // ---- staging ------------------------------------------------------------------------------------
 
@@ -50,8 +53,9 @@ __device__ __forceinline__ float split_part(float f, bool lo) {
 
 __global__ void __launch_bounds__(256)
 stage_gy_img_kernel(int Cout, int V, int tiles_per_clip, int b0, int x3, const float* __restrict__ gy,
-                    uint8_t* __restrict__ img, long long lo_off) {
+                    uint8_t* __restrict__ img, long long lo_off, const __grid_constant__ PositionAsk ask) {
   __shared__ float tile[64][129];
+  if (ask.n_recs > 0 && blockIdx.x == 0 && blockIdx.y == 0) ask_positions(ask);
   const int tile_id = blockIdx.x, kb = blockIdx.y, KB = gridDim.y;
   const int bl = tile_id / tiles_per_clip, v0 = (tile_id % tiles_per_clip) * kBM;
   const int b = b0 + bl;
@@ -588,6 +592,7 @@ int run_bwd(const Geom& g, bool x3, const Coords& coords, unsigned long long cap
   uint8_t* wt_img = wsp; wsp += pl.wt_img_bytes;
   float* dcol = reinterpret_cast<float*>(wsp); wsp += pl.dcol_bytes;
   float* gx_cl = reinterpret_cast<float*>(wsp); wsp += pl.gx_cl_bytes;
+  int* direct_word = reinterpret_cast<int*>(wsp); wsp += kWordBytes;
   void* dw_ws = wsp;
 
   int sm_count = 0, rc;
@@ -651,9 +656,13 @@ int run_bwd(const Geom& g, bool x3, const Coords& coords, unsigned long long cap
   for (int b0 = 0; b0 < g.B; b0 += pl.clips_per_chunk) {
     const int nbc = (g.B - b0 < pl.clips_per_chunk) ? g.B - b0 : pl.clips_per_chunk;
     const int n_tiles = nbc * pl.tiles_per_clip;
+    const SampleGradPlan sp = sample_grad_plan(g, nbc, pl.nh, FieldOut, x3, pl.pairg, sm_count);
+    const long long n_clip_recs = (long long)g.G * g.K * g.V;
+    const PositionAsk ask{g, recs + b0 * n_clip_recs, sp.ask ? nbc * n_clip_recs : 0, voxel_order(g), sp.taps, FieldOut, field_ch, axes,
+                          direct_word};
     prof_mark(st, "bwd_stage_grad_out");
     stage_gy_img_kernel<<<dim3((unsigned)n_tiles, (unsigned)pl.KBT), 256, 0, st>>>(g.Cout, g.V, pl.tiles_per_clip, b0,
-                                                                                  img_mode, gy, gy_img, pl.gy_lo_off);
+                                                                                  img_mode, gy, gy_img, pl.gy_lo_off, ask);
     D2C_LAUNCH_CHECK();
     DcolParams p;
     p.gy_img = gy_img; p.wt_img = wt_img; p.dcol = dcol;
@@ -676,23 +685,33 @@ int run_bwd(const Geom& g, bool x3, const Coords& coords, unsigned long long cap
       dcol_sm100_kernel<0><<<(unsigned)grid, kDcolThreads, pl.smem_bytes, st>>>(p);
     D2C_LAUNCH_CHECK();
     prof_mark(st, "bwd_sample_grad");
-    // A block lists and adds up the contributions of 32 voxels; the more taps it has, the more of them meet.  Small volumes share
-    // the taps out over up to nine blocks, so that every multiprocessor has its three (256 channels on 8 x 15 x 27: 107 us with
-    // three, six or twelve a multiprocessor asked for; 64 channels on 4 x 16 x 16: 17.6 us with nine blocks, 19.5 with 14).
-    const long long vblocks = (long long)((g.V + kSgVox - 1) / kSgVox) * nbc * g.G;
-    int tap_split = (int)((3LL * sm_count + vblocks - 1) / vblocks);
-    if (tap_split > 9) tap_split = 9;
-    if (tap_split < (g.K + kSgMaxTaps - 1) / kSgMaxTaps) tap_split = (g.K + kSgMaxTaps - 1) / kSgMaxTaps;
-    if (tap_split > g.K) tap_split = g.K;
-    const int taps_per_block = (g.K + tap_split - 1) / tap_split;
-    dim3 sgrid((unsigned)((g.V + kSgVox - 1) / kSgVox), (unsigned)(nbc * g.G), (unsigned)((g.K + taps_per_block - 1) / taps_per_block));
-    const size_t smem = sample_grad_smem(taps_per_block, pl.nh);
+    const size_t smem = sample_grad_smem(sp.taps, pl.nh);
     auto launch = [&](auto f32x, auto narrow, auto multi) -> int {
-      constexpr auto kernel = sample_grad_taps_kernel<FieldOut, decltype(f32x)::value, decltype(narrow)::value, decltype(multi)::value>;
+      constexpr bool kF32X = decltype(f32x)::value, kNarrow = decltype(narrow)::value, kMulti = decltype(multi)::value;
+      constexpr bool kMayAsk = !FieldOut || kMulti;
+      const int3 blocks = make_int3((int)sp.grid.x, (int)sp.grid.y, (int)sp.grid.z);
+      auto direct = [&](auto kernel, const dim3& grid) -> int {
+        kernel<<<grid, kSgThreads, 0, st>>>(g, cs, b0, pl.nh, recs, dcol, x_cl, mask != nullptr, grad_coord, grad_mask, gx_cl,
+                                            field_nch, field_ch, axes, sp.taps, head, blocks, direct_word);
+        D2C_LAUNCH_CHECK();
+        return D2C_OK;
+      };
+      if (!sp.lists) return direct(sample_grad_direct_kernel<FieldOut, kF32X, kNarrow, false>, sp.grid);
+      if constexpr (kMayAsk) {
+        const int few = std::min((kF32X || !kNarrow ? 2 : 3) * sm_count, blocks.x * blocks.y * blocks.z);
+        if (sp.ask && (rc = direct(sample_grad_direct_kernel<FieldOut, kF32X, kNarrow, true>, (unsigned)few))) return rc;
+      }
+      constexpr auto kernel = sample_grad_taps_kernel<FieldOut, kF32X, kNarrow, kMulti>;
       const int rc = allow_dynamic_smem<kernel>((int)smem);
       if (rc) return rc;
-      kernel<<<sgrid, kSgThreads, smem, st>>>(g, voxel_order(g), cs, b0, pl.nh, recs, dcol, x_cl, mask != nullptr, grad_coord, grad_mask,
-                                              gx_cl, field_nch, field_ch, axes, taps_per_block, head);
+      if (sp.ask) {
+        D2C_CUDA_TRY(launch_beside(kernel, sp.grid, kSgThreads, smem, st, g, voxel_order(g), cs, b0, pl.nh, recs, dcol, x_cl, mask != nullptr,
+                                   grad_coord, grad_mask, gx_cl, field_nch, field_ch, axes, sp.taps, head, direct_word));
+      } else {
+        kernel<<<sp.grid, kSgThreads, smem, st>>>(g, voxel_order(g), cs, b0, pl.nh, recs, dcol, x_cl, mask != nullptr, grad_coord, grad_mask,
+                                                  gx_cl, field_nch, field_ch, axes, sp.taps, head, nullptr);
+      }
+      D2C_LAUNCH_CHECK();
       return D2C_OK;
     };
     const std::true_type yes;
@@ -704,7 +723,6 @@ int run_bwd(const Geom& g, bool x3, const Coords& coords, unsigned long long cap
     else
       rc = x3 ? launch(yes, no, no) : launch(no, no, no);
     if (rc) return rc;
-    D2C_LAUNCH_CHECK();
   }
   if constexpr (FieldOut) {
     if (head.size_act != 0 && raw_field) {      // chain rule through the size activation, on the summed gradient
@@ -756,7 +774,7 @@ size_t sm100_bwd_workspace(const Geom& g, int dtype, int math_mode, unsigned lon
   const bool x3 = bwd_use_x3(g, math_mode, cap);
   BwdPlan pl;
   make_bwd_plan(g, cap, x3, &pl);
-  return pl.x_cl_bytes + pl.rec_bytes + pl.gat_bytes + pl.gy_img_bytes + pl.wt_img_bytes + pl.dcol_bytes + pl.gx_cl_bytes +
+  return pl.x_cl_bytes + pl.rec_bytes + pl.gat_bytes + pl.gy_img_bytes + pl.wt_img_bytes + pl.dcol_bytes + pl.gx_cl_bytes + kWordBytes +
          sm100_dw_workspace(g, x3);
 }
 

@@ -59,6 +59,10 @@ inline size_t sample_grad_smem(int taps, int nh) {
   return n * (8 * 4 * (nh > 1 ? 2 : 1) + 8 + 8 * 2) + kSgCells * 2;
 }
 
+__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
+  // volatile (must not be dropped) but no memory clobber: read-only loads may move across it
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d));
+}
 // Loads under a predicate; the register keeps its contents otherwise.
 __device__ __forceinline__ void ldg_if(float4& r, const float* p, bool on) {
   asm("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
@@ -88,6 +92,138 @@ __device__ __forceinline__ float4 ldg_again(const float4* p) {
   return r;
 }
 
+// Corners of a sample that are inside the volume and can matter.  A tap at the kernel's centre on an axis does not move along it, and
+// no tap does where the field has no channel for the axis: the upper corners of that axis weigh nothing and the axis takes no
+// gradient (with 3 x 3 x 3 taps 4.6 corners a tap instead of 8, and 2.8 where the field scales rows and columns alone; the latter, one
+// group of 256 channels on 2 x 8 x 30 x 54: 531 us with the first of the two rules alone, 374 with both).
+template <bool FieldOut>
+__device__ __forceinline__ unsigned live_corners(const Geom& g, const Sample<float>& s, int tap, int3 field_ch, const FieldAxes& axes) {
+  unsigned valid = s.valid;
+  if constexpr (FieldOut) {
+    const int kx = tap % g.kw, ky = (tap / g.kw) % g.kh, kz = tap / (g.kw * g.kh);
+    if (valid) {
+      if ((field_ch.x < 0 || axes.pos[0][kz] == 0.f) && !(s.gz < 1.f)) valid &= 0x0fu;
+      if ((field_ch.y < 0 || axes.pos[1][ky] == 0.f) && !(s.gy < 1.f)) valid &= 0x33u;
+      if ((field_ch.z < 0 || axes.pos[2][kx] == 0.f) && !(s.gx < 1.f)) valid &= 0x55u;
+    }
+  }
+  return valid;
+}
+// Those that weigh something in the scatter (a corner at distance exactly 1 does not, dconv3d_gpu.cu:626-637).
+__device__ __forceinline__ unsigned weighing_corners(const Sample<float>& s, unsigned valid) {
+  return valid & (s.gz < 1.f ? 0xffu : 0x0fu) & (s.gy < 1.f ? 0xffu : 0x33u) & (s.gx < 1.f ? 0xffu : 0x55u);
+}
+
+// Which kernel takes a call's positions (below): asked of 256 records, evenly spread over the clips at hand, by one block of a kernel
+// that runs before both.
+struct PositionAsk {
+  Geom g;
+  const float4* recs;          // of the first clip at hand
+  long long n_recs;            // 0: not asked
+  VoxelOrder order;
+  int taps;                    // of a block
+  int field;
+  int3 field_ch;
+  FieldAxes field_axes;
+  int* direct;                 // the answer
+};
+// Sums win where contributions meet and weigh something.  (us, sums / direct, two clips of 8 x 60 x 107 and one group of 256 channels
+// unless it says otherwise; measured with each kernel taking all.)
+//   offsets    few corners weigh: the direct kernel sends fewer, the lists are as long as ever.  All offsets zero (one corner of
+//              eight) 2700 / 1620, whole along one axis (a half) 2980 / 2370, along none 2900 / 3470; single pass 2760 / 1390, 2860 /
+//              2170, 2830 / 3320.  The line lies a little above a half.
+//   fields     a field of ones over three axes (0.22 of the corners left) 2190 / 1740; over two (0.36) 1440 / 1680; so 0.3.  Groups of one
+//              slice are not asked: there the lists win at 0.22 too (two groups of 64: 1110 / 1230).
+//   scattered  contributions of a brick that rarely meet: two groups of 64 channels on 8 x 120 x 214, offsets of sigma 16 in the plane
+//              and 0.5 across (13 cells a contribution) 4310 / 3720, sigma 8 (4) 3850 / 3840, sigma 4 3590 / 3870; the line at 7.
+//   outside    the lists hold nothing for samples outside the volume, while the direct kernel reads every gradient column: 512
+//              channels on 2 x 8 x 30 x 54, sigma 64, 270 / 1070.  So the direct kernel needs three quarters of the samples inside.
+__device__ __forceinline__ bool direct_by_positions(const PositionAsk& q, const int* sums) {
+  const Geom& g = q.g;
+  const int n_in = sums[0], n = sums[1], n_weigh = sums[2];
+  if (4 * n_in < 3 * kSgThreads) return false;
+  if (q.field) return 10 * n_weigh <= 3 * n;
+  if (16 * n_weigh <= 9 * n) return true;
+  // cells of a brick's box (864 samples reach about 8 times their mean distance from end to end) against its contributions
+  auto cells = [&](int size, int brick, int stride, int k, int dil, int spread) {
+    const float ext = (float)((brick - 1) * stride + (k - 1) * dil + 2) + 8.f / (16.f * kSgThreads) * (float)spread;
+    return fminf(ext, (float)size);
+  };
+  const float box = cells(g.D, q.order.bz, g.sd, g.kd, g.dd, sums[3]) * cells(g.H, q.order.by, g.sh, g.kh, g.dh, sums[4]) *
+                    cells(g.W, 8, g.sw, g.kw, g.dw, sums[5]);
+  return box > 7.f * (float)n * ((float)(kSgVox * q.taps) / (float)kSgThreads);
+}
+__device__ __forceinline__ void ask_positions(const PositionAsk& q) {
+  __shared__ int sums[6];      // samples in the volume, their corners, those that weigh; |position - tap| in 1/16 voxel
+  const Geom& g = q.g;
+  if (threadIdx.x < 6) sums[threadIdx.x] = 0;
+  __syncthreads();
+  const long long i = (2 * (long long)threadIdx.x + 1) * q.n_recs / (2 * kSgThreads);
+  const int v = (int)(i % g.V), tap = (int)(i / g.V % g.K);
+  const float4 rec = __ldg(q.recs + i);
+  const Sample<float> s = make_sample(g, rec.x, rec.y, rec.z);
+  const unsigned valid = q.field ? live_corners<true>(g, s, tap, q.field_ch, q.field_axes) : s.valid;
+  int base[3];
+  voxel_tap_base(g, v, tap, base[0], base[1], base[2]);
+  const float at[3] = {rec.x, rec.y, rec.z};
+  int own[6] = {valid != 0, __popc(valid), __popc(weighing_corners(s, valid))};
+#pragma unroll
+  for (int d = 0; d < 3; ++d) own[3 + d] = (int)(16.f * fminf(fabsf(at[d] - (float)base[d]), 4096.f));
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const int t = __reduce_add_sync(0xffffffffu, own[k]);
+    if ((threadIdx.x & 31) == 0) atomicAdd(sums + k, t);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) *q.direct = direct_by_positions(q, sums);
+}
+
+// How a call's sampling gradient is split, and which kernel may take it.
+struct SampleGradPlan {
+  dim3 grid;                   // voxels / 32, clips x groups, tap ranges
+  int taps;                    // of a block
+  bool lists, ask;             // may be sample_grad_taps_kernel's; the positions decide
+};
+// Asking costs a call about 3 us (a launch that ends at once and the wait for it): from this many (32 voxels, tap, slice) on, about 300
+// us of kernel.
+constexpr long long kSgAskFrom = 32768;
+// A block lists and adds up the contributions of 32 voxels; the more taps it has, the more of them meet.  Small volumes share
+// the taps out over up to nine blocks, so that every multiprocessor has its three (256 channels on 8 x 15 x 27: 107 us with
+// three, six or twelve a multiprocessor asked for; 64 channels on 4 x 16 x 16: 17.6 us with nine blocks, 19.5 with 14).
+// Which kernel, by what the host knows (us, direct / sums; offsets of two voxels):
+//   few taps           the lists' fixed cost, and little meets.  256 channels in 4 groups on 2 x 8 x 30 x 54, 1 tap 54 / 87, 3 taps 115 /
+//                      133, 5 taps 179 / 182, 6 taps 215 / 209; fp16 staging, 6 taps 196 / 205, 7 taps 218 / 223, 8 taps 280 / 266.
+//                      One group, 5 taps 160 / 154.  A field has fewer corners a tap: 1 tap 43 / 75, 3 taps 90 / 94 (one group 64
+//                      / 61, groups of 32 channels 148 / 170), 5 taps 137 / 117 (groups of 32 channels 223 / 209).
+//   few taps a block   64 channels on 4 x 16 x 16, 3 taps a block 16 / 19; on 8 x 16 x 16, 4 taps 31 / 27; 2 groups of 32 there, 7 taps 33 / 37.
+//   strides            the voxels of a brick lie apart.  512 channels in 8 groups, 8 x 60 x 107 with stride 2 on every axis 970 / 1000 (fp16
+//                      836 / 892), with stride 3 in the plane 454 / 502 (4 groups of 64).  Groups of several slices win with sums all the
+//                      same (one of 256: 628 / 499).
+//   32 channels a group, offsets: half the sums' gain for the same lists.  256 channels on 8 x 60 x 107 2310 / 2230, 9 taps on 2 x 8 x
+//                      30 x 54 400 / 432, stride 2 there 625 / 681; fp16 staging 2110 / 2267, but 57 / 50 on 4 x 16 x 16, where the taps
+//                      are shared out.
+inline SampleGradPlan sample_grad_plan(const Geom& g, int nbc, int nh, bool field, bool f32x, bool narrow, int sm_count) {
+  const long long vblocks = (long long)((g.V + kSgVox - 1) / kSgVox) * nbc * g.G;
+  const int min_split = (g.K + kSgMaxTaps - 1) / kSgMaxTaps;
+  long long split = (3LL * sm_count + vblocks - 1) / vblocks;
+  const bool full = split == 1;
+  if (split > 9) split = 9;
+  if (split < min_split) split = min_split;
+  if (split > g.K) split = g.K;
+  SampleGradPlan p;
+  p.taps = (g.K + (int)split - 1) / (int)split;
+  p.grid = dim3((unsigned)((g.V + kSgVox - 1) / kSgVox), (unsigned)(nbc * g.G), (unsigned)((g.K + p.taps - 1) / p.taps));
+  if (field) {
+    p.lists = g.K >= (narrow ? 5 : 3);
+  } else {
+    p.lists = g.K >= (f32x || nh > 1 ? 5 : 8) && p.taps >= (narrow ? 8 : 4);
+    if (nh == 1 && g.sd * g.sh * g.sw >= (narrow ? 2 : 8)) p.lists = false;
+    if (narrow && (g.K < 16 || (!f32x && full))) p.lists = false;
+  }
+  p.ask = p.lists && (!field || nh > 1) && vblocks * g.K * nh >= kSgAskFrom;
+  return p;
+}
+
 // Block = 32 output voxels (a brick) and up to 27 taps of one (clip, offset group).  A sample is one (voxel, tap); each of its
 // corners inside the volume is a contribution: weight x gradient column is due to the input voxel there, and (gradient column .
 // input) is due to the sample's coordinate and modulation gradients.
@@ -112,9 +248,13 @@ sample_grad_taps_kernel(Geom g, VoxelOrder order, ClStrides cs, int b0, int nh, 
                          const float* __restrict__ dcol, const void* __restrict__ x_cl_v, bool has_mask,
                          float* __restrict__ grad_coord, float* __restrict__ grad_mask, float* __restrict__ gx_cl,
                          int field_nch, int3 field_ch, const __grid_constant__ FieldAxes field_axes, int taps_per_block,
-                         HeadCfg head) {
+                         HeadCfg head, const int* __restrict__ direct) {
   extern __shared__ __align__(16) uint8_t sg_smem[];
   __shared__ int s_box[6], s_total, s_single, s_delta[8];
+  if (direct) {                        // started beside sample_grad_direct_kernel, which is the other answer's
+    wait_for_kernels_before();
+    if (*direct) return;
+  }
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int grp = blockIdx.y % g.G, bl = blockIdx.y / g.G, b = b0 + bl;
   const int tap_beg = blockIdx.z * taps_per_block, n_tap = min(g.K - tap_beg, taps_per_block);
@@ -149,11 +289,7 @@ sample_grad_taps_kernel(Geom g, VoxelOrder order, ClStrides cs, int b0, int nh, 
       const int tap = tap_beg + k * 8 + warp;
       const Sample<float> s = make_sample(g, rec[k].x, rec[k].y, rec[k].z);
       unsigned valid = active && k * 8 + warp < n_tap ? s.valid : 0u;
-      if constexpr (FieldOut) {
-        // A tap at the kernel's centre on an axis does not move along it, and no tap does where the field has no channel for the
-        // axis: the upper corners of that axis weigh nothing and the axis takes no gradient (with 3 x 3 x 3 taps 4.6
-        // corners a tap instead of 8, and 2.8 where the field scales rows and columns alone; the latter, one group of 256 channels
-        // on 2 x 8 x 30 x 54: 531 us with the first of the two rules alone, 374 with both, 494 with every corner reduced by itself).
+      if constexpr (FieldOut) {          // live_corners, written out: as a call this kernel's code comes out up to 12 % slower
         const int kx = tap % g.kw, ky = (tap / g.kw) % g.kh, kz = tap / (g.kw * g.kh);
         if (valid) {
           if ((field_ch.x < 0 || field_axes.pos[0][kz] == 0.f) && !(s.gz < 1.f)) valid &= 0x0fu;
@@ -416,6 +552,191 @@ sample_grad_taps_kernel(Geom g, VoxelOrder order, ClStrides cs, int b0, int nh, 
       if (ch >= 0)
         atomicAdd(grad_coord + (long long)b * (head.geo_bstride ? head.geo_bstride : (long long)field_nch * g.V) + (long long)ch * g.V + v, sum);
     }
+  }
+}
+
+// The same without lists: every corner of every sample is read, and reduced into L2, by itself.  Eight threads a voxel, thread j with
+// channels [4j, 4j + 4) and [32 + 4j, 32 + 4j + 4) of a slice (two lanes cover a 32-byte sector); the block walks its taps, the record
+// and the gradient columns of the next tap requested before the present one is worked on.  Bound by L2's rate of fp32 additions where
+// all corners weigh.  Voxels in storage order: in bricks, whose threads add to the same voxels at the same time, it is up to 15 % slower.
+// Small volumes share the taps out as there (1024 voxels, 27 taps: 46.9 us with one block per 32 voxels, 10.6 with nine).
+template <bool FieldOut, bool kF32X, bool kNarrow>
+__device__ __forceinline__ void
+sample_grad_direct(Geom g, ClStrides cs, int b0, int nh, const float4* __restrict__ recs,
+                   const float* __restrict__ dcol, const void* __restrict__ x_cl_v, bool has_mask,
+                   float* __restrict__ grad_coord, float* __restrict__ grad_mask, float* __restrict__ gx_cl,
+                   int field_nch, int3 field_ch, const FieldAxes& field_axes, int taps_per_block,
+                   HeadCfg head, unsigned blk_x, unsigned blk_y, unsigned blk_z) {
+  const int j = threadIdx.x & 7;
+  const int v = blk_x * kSgVox + (threadIdx.x >> 3);
+  const int grp = blk_y % g.G, bl = blk_y / g.G;
+  const int b = b0 + bl;
+  const bool active = v < g.V;
+  const int vc = active ? v : g.V - 1;                       // clamped: inactive threads load valid memory
+  const long long S = kNarrow ? (long long)(g.G / 2) * g.K : (long long)g.G * g.K * nh;
+  const float4* recp = recs + (((long long)b * g.G + grp) * g.K) * g.V + vc;
+  // thread j owns channels [4j, 4j+4) and [32+4j, 32+4j+4) of a slice: one warp-wide 16-byte access then
+  // covers whole 32-byte sectors (two lanes each), which halves the sector operations of the reductions
+  const float* dp = kNarrow
+      ? dcol + (((long long)bl * S + (long long)(grp >> 1) * g.K) * g.V + vc) * 64 + (grp & 1) * 32 + j * 4
+      : dcol + (((long long)bl * S + (long long)grp * g.K * nh) * g.V + vc) * 64 + j * 4;
+  const long long slice_stride = (long long)g.V * 64;
+  using XT = typename std::conditional<kF32X, float, __half>::type;
+  const XT* xb = reinterpret_cast<const XT*>(x_cl_v) + (long long)b * g.Vin * g.Cin;
+  float* gxb = gx_cl + (long long)b * g.Vin * g.Cin;
+  const int chbase = grp * g.cpg + j * 4;
+
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  float fsum[3] = {0.f, 0.f, 0.f};
+  auto ld_cols = [&](const float* q, float4& a, float4& b) {
+    a = __ldg(reinterpret_cast<const float4*>(q));
+    b = kNarrow ? zero4 : __ldg(reinterpret_cast<const float4*>(q + 32));
+  };
+  const int tap_beg = blk_z * taps_per_block, tap_end = min(g.K, tap_beg + taps_per_block);
+  float4 rec_n = __ldg(recp + (long long)tap_beg * g.V);
+  float4 d0_n, d1_n;
+  ld_cols(dp + (long long)tap_beg * nh * slice_stride, d0_n, d1_n);
+  for (int tap = tap_beg; tap < tap_end; ++tap) {
+    const float4 rec = rec_n;
+    float4 d0 = d0_n, d1 = d1_n;
+    if (tap + 1 < tap_end) {
+      rec_n = __ldg(recp + (long long)(tap + 1) * g.V);
+      ld_cols(dp + (long long)(tap + 1) * nh * slice_stride, d0_n, d1_n);
+    }
+    const float m = rec.w;
+    const Sample<float> s = make_sample(g, rec.x, rec.y, rec.z);
+    // scatter weights of the reference's col2im: (1-|z-zp|)(1-|y-yp|)(1-|x-xp|), corners at distance
+    // exactly 1 excluded (dconv3d_gpu.cu:626-637)
+    const float wz[2] = {sub_rn(1.f, s.fz), sub_rn(1.f, s.gz)};
+    const float wy[2] = {sub_rn(1.f, s.fy), sub_rn(1.f, s.gy)};
+    const float wx[2] = {sub_rn(1.f, s.fx), sub_rn(1.f, s.gx)};
+    const bool okz[2] = {true, s.gz < 1.f}, oky[2] = {true, s.gy < 1.f}, okx[2] = {true, s.gx < 1.f};
+    // (Not the field's dead corners where a thread has 4 channels of fp16: it issues its loads either way, a corner left out
+    // reads the stand-in below, and finding out which to leave out costs it more than the cache hits give back.)
+    const unsigned valid = active ? live_corners<FieldOut && (kF32X || !kNarrow)>(g, s, tap, field_ch, field_axes) : 0u;
+    const int off0 = ((s.z0 * g.H + s.y0) * g.W + s.x0) * g.Cin + chbase;
+    float G[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) G[q] = 0.f;
+    for (int h = 0; h < nh; ++h) {
+      if (h > 0) {
+        ld_cols(dp + ((long long)tap * nh + h) * slice_stride, d0, d1);
+      }
+      // corner values of this thread's 8 channels ([4j, 4j+4) and [32+4j, 32+4j+4)), as loaded.  fp16 staging:
+      // the loads are unconditional -- a corner outside the volume reads the clip's first voxel instead and its
+      // dot product is discarded by a select after the slice loop (a select, so a non-finite stand-in cannot
+      // leak); measured 0.13 ms per step faster than predicated loads.  fp32 staging: predicated loads (twice
+      // the bytes per corner; fetching the stand-ins measured 0.08 ms slower).
+      uint4 c[8], chi[kF32X ? 8 : 1];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int off_in = off0 + h * 64 + (q >> 2) * cs.dz + ((q >> 1) & 1) * cs.dy + (q & 1) * cs.dx;
+        if constexpr (kF32X) {
+          if ((valid >> q) & 1u) {
+            c[q] = ptx::ldg_nc_v4(xb + off_in);
+            chi[q] = kNarrow ? make_uint4(0u, 0u, 0u, 0u) : ptx::ldg_nc_v4(xb + off_in + 32);
+          } else {
+            c[q] = chi[q] = make_uint4(0u, 0u, 0u, 0u);
+          }
+        } else {
+          const int off = ((valid >> q) & 1u) ? off_in : chbase + h * 64;
+          const uint2 lo = ptx::ldg_nc_v2(xb + off);
+          const uint2 hi = kNarrow ? make_uint2(0u, 0u) : ptx::ldg_nc_v2(xb + off + 32);
+          c[q] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int dz = q >> 2, dy = (q >> 1) & 1, dx = q & 1;
+        if constexpr (kF32X) {
+          if constexpr (kNarrow)
+            G[q] += d0.x * __uint_as_float(c[q].x) + d0.y * __uint_as_float(c[q].y) +
+                    d0.z * __uint_as_float(c[q].z) + d0.w * __uint_as_float(c[q].w);
+          else
+            G[q] += d0.x * __uint_as_float(c[q].x) + d0.y * __uint_as_float(c[q].y) +
+                    d0.z * __uint_as_float(c[q].z) + d0.w * __uint_as_float(c[q].w) +
+                    d1.x * __uint_as_float(chi[q].x) + d1.y * __uint_as_float(chi[q].y) +
+                    d1.z * __uint_as_float(chi[q].z) + d1.w * __uint_as_float(chi[q].w);
+        } else {
+          const float2 x0 = __half22float2(bits_h2(c[q].x)), x1 = __half22float2(bits_h2(c[q].y));
+          const float2 x2 = __half22float2(bits_h2(c[q].z)), x3 = __half22float2(bits_h2(c[q].w));
+          if constexpr (kNarrow)
+            G[q] += d0.x * x0.x + d0.y * x0.y + d0.z * x1.x + d0.w * x1.y;
+          else
+            G[q] += d0.x * x0.x + d0.y * x0.y + d0.z * x1.x + d0.w * x1.y + d1.x * x2.x + d1.y * x2.y +
+                    d1.z * x3.x + d1.w * x3.y;
+        }
+        if (((valid >> q) & 1u) && okz[dz] && oky[dy] && okx[dx]) {
+          const float sw = mul_rn(mul_rn(wz[dz], wy[dy]), wx[dx]) * m;
+          float* dst = gxb + (off0 + h * 64 + dz * cs.dz + dy * cs.dy + dx * cs.dx);
+          red_add_v4(dst, sw * d0.x, sw * d0.y, sw * d0.z, sw * d0.w);
+          if (!kNarrow) red_add_v4(dst + 32, sw * d1.x, sw * d1.y, sw * d1.z, sw * d1.w);
+        }
+      }
+    }
+    // channel reduction of the 8 corner dot-products across the voxel's 8 threads (corners outside: zero)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      if (!kF32X) G[q] = ((valid >> q) & 1u) ? G[q] : 0.f;
+      G[q] += __shfl_xor_sync(0xffffffffu, G[q], 1);
+      G[q] += __shfl_xor_sync(0xffffffffu, G[q], 2);
+      G[q] += __shfl_xor_sync(0xffffffffu, G[q], 4);
+    }
+    if (active && j == 0) {
+      float wts[3];
+      coord_weights(G, s, wts);    // linear in the corner values: applies to the channel-summed corners
+      // head.*_bstride != 0: the gradients go into the gradient of the predictor's raw output (clip stride = all of
+      // its channels), the mask's through the derivative of its activation (taken from the activated value m)
+      if (has_mask && grad_mask) {
+        float a[8];
+        sample_weights(s, a);
+        const long long ri = head.mask_bstride ? (long long)b * head.mask_bstride + ((long long)grp * g.K + tap) * g.V + v
+                                               : (((long long)b * g.G + grp) * g.K + tap) * g.V + v;
+        grad_mask[ri] = s.inside ? blend(G, a) * mask_act_slope(head.mask_act, m) : 0.f;
+      }
+      if constexpr (!FieldOut) {
+        float* go = grad_coord + (head.geo_bstride ? (long long)b * head.geo_bstride + ((long long)grp * 3 * g.K + 3 * tap) * g.V + v
+                                                   : (((long long)b * g.G + grp) * 3 * g.K + 3 * tap) * g.V + v);
+        go[0] = m * wts[0];
+        go[g.V] = m * wts[1];
+        go[2 * (long long)g.V] = m * wts[2];
+      } else {
+        // the field's gradient sums over taps (and groups): taps are summed here, one atomic per group after
+        const int k = tap % g.kw, jj = (tap / g.kw) % g.kh, i = tap / (g.kw * g.kh);
+        fsum[0] += field_axes.pos[0][i] * (m * wts[0]);
+        fsum[1] += field_axes.pos[1][jj] * (m * wts[1]);
+        fsum[2] += field_axes.pos[2][k] * (m * wts[2]);
+      }
+    }
+  }
+  if constexpr (FieldOut) {
+    if (active && j == 0) {
+      float* gs = grad_coord + (long long)b * (head.geo_bstride ? head.geo_bstride : (long long)field_nch * g.V) + v;
+      if (field_ch.x >= 0) atomicAdd(gs + (long long)field_ch.x * g.V, fsum[0]);
+      if (field_ch.y >= 0) atomicAdd(gs + (long long)field_ch.y * g.V, fsum[1]);
+      if (field_ch.z >= 0) atomicAdd(gs + (long long)field_ch.z * g.V, fsum[2]);
+    }
+  }
+}
+// kAsk: only where the positions were asked and this is the answer; a few blocks that take turns, so that it costs little where not
+// (in turns it takes 3 to 8 % longer; fp16, 8 channels a thread, spills at three blocks a multiprocessor then).
+template <bool FieldOut, bool kF32X, bool kNarrow, bool kAsk>
+__global__ void __launch_bounds__(kSgThreads, kF32X || (kAsk && !kNarrow) ? 2 : 3)
+sample_grad_direct_kernel(Geom g, ClStrides cs, int b0, int nh, const float4* __restrict__ recs,
+                          const float* __restrict__ dcol, const void* __restrict__ x_cl_v, bool has_mask,
+                          float* __restrict__ grad_coord, float* __restrict__ grad_mask, float* __restrict__ gx_cl,
+                          int field_nch, int3 field_ch, const __grid_constant__ FieldAxes field_axes, int taps_per_block,
+                          HeadCfg head, int3 blocks, const int* __restrict__ direct) {
+  auto block = [&](int x, int y, int z) {
+    sample_grad_direct<FieldOut, kF32X, kNarrow>(g, cs, b0, nh, recs, dcol, x_cl_v, has_mask, grad_coord, grad_mask, gx_cl, field_nch,
+                                                 field_ch, field_axes, taps_per_block, head, x, y, z);
+  };
+  if constexpr (kAsk) {
+    if (!*direct) return;
+    const int n_blocks = blocks.x * blocks.y * blocks.z;
+    for (int i = blockIdx.x; i < n_blocks; i += gridDim.x) block(i % blocks.x, i / blocks.x % blocks.y, i / (blocks.x * blocks.y));
+  } else {
+    block(blockIdx.x, blockIdx.y, blockIdx.z);
   }
 }
 
