@@ -252,16 +252,21 @@ bool pick_variant(const Geom& g, int math_mode, bool* x3, Plan* pl, bool shared 
   return false;
 }
 
-// Calls of at most this many units per CTA start the kernel beside the last staging kernel, its set-up under that one's end: 256
-// channels on 8 x 15 x 27 (38 units) 84.7 us a call, 88.4 started after it (93.6 with all four kernels one after the other).  A
-// kernel started that way runs 3 % slower (1024 -> 256 channels on 8 x 30 x 54, 298 units, 505 instead of 494 us a call), more than
-// the start where it runs for long.
-constexpr int kMaxUnitsBeside = 64;
+// Short calls start the kernel beside the last staging kernel, its set-up under that one's end.  That saves 1 to 3 us, and a kernel
+// started that way runs slower by 1 to 4 %, the more the more outputs it has, so that it is worth it up to a length.  us a call
+// (back to back in a graph), started after / beside:
+//   single pass, 512 outputs   22 units a CTA 98.2 / 97.1, 38: 124.5 / 125.2, 60: 167.2 / 171.3, 83: 206.5 / 214.4
+//                320           15: 64.8 / 63.2, 38: 103.6 / 103.2, 44: 114.8 / 116.2
+//                256           44: 108.0 / 106.9, 55: 107.6 / 107.3, 60: 133.7 / 135.0, 74: 156.8 / 160.1
+//                128           37: 80.1 / 78.0, 55: 134.6 / 134.1, 74: 172.7 / 172.2
+// so units x outputs decide there.  The fp32-parity mode has units half as long and loses less: 512 outputs, 76 units 186.3 / 184.5,
+// 256 outputs, 38: 84.1 / 82.0, 58: 122.8 / 121.1, 149: 225 / 224; but 128 outputs, 74: 124.2 / 127.1, 149: 255.5 / 261.9.
+constexpr int kMaxUnitsBeside = 64, kMaxOutputUnitsBeside = 12288;
 
 template <int kX3, int kDual, int kSave, bool kMayShare>
 int launch_fwd(const FwdParams& p, unsigned grid, int smem_bytes, cudaStream_t st) {
   auto start = [&](auto kernel) -> int {
-    if (p.n_units <= (long long)kMaxUnitsBeside * grid)
+    if (p.n_units <= (long long)kMaxUnitsBeside * grid && (kX3 || p.n_units * p.N <= (long long)kMaxOutputUnitsBeside * grid))
       D2C_CUDA_TRY(launch_beside(kernel, grid, kThreadsFwd, smem_bytes, st, p));
     else
       kernel<<<grid, kThreadsFwd, smem_bytes, st>>>(p);

@@ -100,6 +100,24 @@ def test_which_outputs_are_nan(mode, cin, cout, dims):
     _lib.device_status()
 
 
+@pytest.mark.parametrize("dims", [(8, 12, 20), (8, 15, 27)])
+def test_both_sides_of_the_line_for_many_outputs(dims):
+    """Single pass, 512 outputs: 22 units a CTA start beside the staging, 38 do not.  New inputs in every call."""
+    import d2conv3d_b200
+    from d2conv3d_b200 import _lib, dconv_native
+    ps = [problem(512, 512, dims, seed) for seed in range(3)]
+    try:
+        with torch.no_grad():
+            d2conv3d_b200.set_math_mode("fp32")
+            want = [dconv_native.deform_conv3d(*p, 1, 1, 1, 1, 1) for p in ps]
+            d2conv3d_b200.set_math_mode("bf16")
+            for y, w in zip([dconv_native.deform_conv3d(*p, 1, 1, 1, 1, 1) for p in ps * 3], want * 3):
+                assert float((y - w).abs().max()) <= 2e-2 * float(w.abs().max())      # the mode's bound
+    finally:
+        d2conv3d_b200.set_math_mode("auto")
+    _lib.device_status()
+
+
 def test_nan_word_is_this_calls_own():
     """The word by which a forward chooses its loop, in a workspace of the caller's that holds anything: it tells of this call's input,
     not of what the memory held or of an earlier call, in replays of a graph too."""
