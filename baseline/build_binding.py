@@ -1,7 +1,7 @@
 """Builds the C++ drop-in binding: the reference's UNMODIFIED pybind / autograd layer (csrc/ops/dconv.cpp with
 dconv3d.h and dconv1d.h, read where they lie in the reference checkout) linked against libd2conv3d.so through
 baseline/binding/d2c_dconv_binding.cpp, which supplies the four `*_cuda` functions that the reference implements
-in its two .cu files.  Output: baseline/_ref/_binding/dconv_d2c_ops.so (git-ignored; travels to the GPU box).
+in its two .cu files.  Output: baseline/_ref/_binding/dconv_d2c_ops.so (git-ignored; it goes where the tests run).
 
     python baseline/build_binding.py <path of the reference checkout>
 

@@ -69,9 +69,10 @@ constexpr int kSmemLimit = 227 * 1024;
 // KB stages had no room for that: 1.55 ms at 2 x 8 x 30 x 54 where 32 KB stages took 1.31.  Two A stages or two record stages
 // instead cost more than the L1 gives back.
 constexpr int kSmemGather = 195 * 1024;
-// Fewest units a CTA is started for.  A unit takes 1.9-2.3 us in its CTA (the producers' gather latency), starting a CTA
-// and adding its partial tile to y about 5 us together: below four units per CTA more CTAs no longer shorten the call.
-// Small layer (432 units): 27 CTAs of 16 units 36.2 us, 108 CTAs of 4 units 17.7 us.
+// Fewest units a CTA is started for.  A unit takes 1.1-1.6 us in its CTA, starting a CTA and adding its partial tile to y about 5 us
+// together: below four units per CTA more CTAs no longer shorten the call by much.  us a call (back to back in a graph) with at least
+// 2 / 4 / 8 / 16 units a CTA: 64 -> 64 on 4 x 16 x 16 18.1 / 18.6 / 23.1 / 30.0, 128 -> 128 on 4 x 12 x 12 25.4 / 21.2 / 30.1 / 37.0, 256 -> 64
+// on 2 x 15 x 15 16.9 / 16.9 / 20.0 / 27.4; single pass 16.3 / 18.3 / 22.8 / 29.8, 18.7 / 24.7 / 29.2 / 36.6, 13.9 / 15.1 / 20.1 / 26.8.
 constexpr int kMinUnitsPerCta = 4;
 // ... and for which the units of a call are cut clip by clip (cta_part_range): every part ends in a partial tile.
 constexpr int kMinUnitsPerPart = 64;

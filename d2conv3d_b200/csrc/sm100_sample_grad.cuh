@@ -236,8 +236,8 @@ inline SampleGradPlan sample_grad_plan(const Geom& g, int nbc, int nh, bool fiel
 // taps meets the same input voxel 4.2 times, so that 1.9 GB of sums leave it and 2 GB of input are read instead of 8.15; what bounds
 // it now are the instructions of step 2 (about 110 a warp for four entries) and the steps' barriers.  Measured there: fp32 staging
 // 1.68 -> 1.38 ms, fp16 staging 1.55 -> 1.35; field layer of one group of 256 channels on 2 x 8 x 60 x 107 2.16 -> 1.90; 32 channels
-// a group, one clip of 8 x 120 x 214, 9.1 -> 7.7.  The smallest layers pay for the lists: 64 channels, 4 x 16 x 16, 15.7 -> 17.6 us,
-// 256 channels in 4 groups 39.6 -> 37.1.  Not faster: a warp per entry with two channels a lane (35 instructions an entry),
+// a group there, one clip of 8 x 120 x 214, 9.1 -> 7.7; 256 channels in 4 groups, 4 x 16 x 16, 39.6 -> 37.1 us.  Where it is slower,
+// sample_grad_plan and direct_by_positions send the call to sample_grad_direct_kernel.  Not faster: a warp per entry with two channels a lane (35 instructions an entry),
 // entries filled up so that none is out of range, the input read with every entry, three entries ahead, packed FMAs.
 // Three blocks a multiprocessor with one entry ahead (80 registers) beat two blocks with two ahead, 1.38 to 1.43 ms; where a group has
 // several slices shared memory allows two blocks, and the field's kernels would spill.
