@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <mutex>
 
 #include "../../include/d2conv3d.h"
 
@@ -317,15 +318,20 @@ void prof_mark(cudaStream_t st, const char* name);
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Raises a kernel's dynamic shared-memory limit, once per kernel, device and size: the attribute call costs about as
-// much host time as a launch, and a small layer makes a dozen launches per pass.
+// much host time as a launch, and a small layer makes a dozen launches per pass.  The limit never goes down: threads that ask
+// for different sizes at the same time raise it one after the other.
 template <auto kKernel>
 inline int allow_dynamic_smem(int bytes) {
   static std::atomic<int> allowed[64];
+  static std::mutex raise;
   int dev = -1;
   D2C_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < 64 && allowed[dev].load(std::memory_order_relaxed) >= bytes) return D2C_OK;
+  const bool known = dev >= 0 && dev < 64;
+  if (known && allowed[dev].load(std::memory_order_acquire) >= bytes) return D2C_OK;
+  const std::lock_guard<std::mutex> lk(raise);
+  if (known && allowed[dev].load(std::memory_order_relaxed) >= bytes) return D2C_OK;
   D2C_CUDA_TRY(cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  if (dev >= 0 && dev < 64) allowed[dev].store(bytes, std::memory_order_relaxed);
+  if (known) allowed[dev].store(bytes, std::memory_order_release);
   return D2C_OK;
 }
 
