@@ -299,8 +299,8 @@ fwd_sm100_kernel(const FwdParams p) {
     }
   } else if (warp == kRecWarpFwd) {
     // ===================== gather-record loader =====================
-    // The records of a unit's rows are one contiguous run of the [B][G][K][V] stream: one bulk copy per unit,
-    // kRStages units ahead of the gather warps, so the producers read them from shared memory.
+    // The records of a unit's rows are one contiguous run of the [B][G][K][V] stream: one bulk copy per unit, into a ring from which the
+    // producers read them.  The ring has kRStages units; a copy starts once the one two units before it is there.
     if (lane == 0) {
       uint32_t k = 0;
       // position of the first unit, once per CTA; then everything advances by counters (this single thread's

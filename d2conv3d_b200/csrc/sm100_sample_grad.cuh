@@ -188,8 +188,9 @@ struct SampleGradPlan {
 // us of kernel.
 constexpr long long kSgAskFrom = 32768;
 // A block lists and adds up the contributions of 32 voxels; the more taps it has, the more of them meet.  Small volumes share
-// the taps out over up to nine blocks, so that every multiprocessor has its three (256 channels on 8 x 15 x 27: 107 us with
-// three, six or twelve a multiprocessor asked for; 64 channels on 4 x 16 x 16: 17.6 us with nine blocks, 19.5 with 14).
+// the taps out over up to nine blocks, so that there are three for every multiprocessor, also for the kernels of which two fit on one
+// (256 channels on 8 x 15 x 27: 107 us with three, six or twelve a multiprocessor; 64 channels on 4 x 16 x 16: 17.6 us with nine
+// blocks, 19.5 with 14).
 // Which kernel, by what the host knows (us, direct / sums; offsets of two voxels):
 //   few taps           the lists' fixed cost, and little meets.  256 channels in 4 groups on 2 x 8 x 30 x 54, 1 tap 54 / 87, 3 taps 115 /
 //                      133, 5 taps 179 / 182, 6 taps 215 / 209; fp16 staging, 6 taps 196 / 205, 7 taps 218 / 223, 8 taps 280 / 266.
@@ -231,14 +232,15 @@ inline SampleGradPlan sample_grad_plan(const Geom& g, int nbc, int nh, bool fiel
 //   2  groups of 8 lanes walk equal shares of the lists, a lane with 8 channels: the gradient columns of every entry are read, the
 //      input only when the cell changes, the sum over a cell stays in registers and leaves as one reduction;
 //   3  a thread per sample turns the eight corner sums into the gradients of offset (field) and modulation.
-// Reducing every contribution into L2 by itself is bound by L2's rate of fp32 additions (6.8 TB/s): 512 channels in 8 groups on
-// 2 x 8 x 30 x 54, offsets of two voxels, sends 8.15 GB, 1.68 ms with 16-byte reductions per corner.  A brick of 32 voxels and 27
-// taps meets the same input voxel 4.2 times, so that 1.9 GB of sums leave it and 2 GB of input are read instead of 8.15; what bounds
-// it now are the instructions of step 2 (about 110 a warp for four entries) and the steps' barriers.  Measured there: fp32 staging
-// 1.68 -> 1.38 ms, fp16 staging 1.55 -> 1.35; field layer of one group of 256 channels on 2 x 8 x 60 x 107 2.16 -> 1.90; 32 channels
-// a group there, one clip of 8 x 120 x 214, 9.1 -> 7.7; 256 channels in 4 groups, 4 x 16 x 16, 39.6 -> 37.1 us.  Where it is slower,
-// sample_grad_plan and direct_by_positions send the call to sample_grad_direct_kernel.  Not faster: a warp per entry with two channels a lane (35 instructions an entry),
-// entries filled up so that none is out of range, the input read with every entry, three entries ahead, packed FMAs.
+// Reducing every contribution into L2 by itself sends 8.15 GB for 512 channels in 8 groups on 2 x 8 x 30 x 54, offsets of two voxels:
+// 1.20 ms at L2's rate of fp32 additions (6.8 TB/s, measured alone), 1.68 ms with the corners' loads and the products beside it.  A
+// brick of 32 voxels and 27 taps meets the same input voxel 4.2 times, so that 1.9 GB of sums leave it and 2 GB of input are read
+// instead of 8.15; what bounds it now are the instructions of step 2 (about 110 a warp for four entries) and the steps' barriers.
+// Measured there: fp32 staging 1.68 -> 1.38 ms, fp16 staging 1.55 -> 1.35; field layer of one group of 256 channels on 2 x 8 x 60 x 107
+// 2.16 -> 1.90; 32 channels a group there, one clip of 8 x 120 x 214, 9.1 -> 7.7; 256 channels in 4 groups, 4 x 16 x 16, 39.6 -> 37.1
+// us.  Where it is slower, sample_grad_plan and direct_by_positions send the call to sample_grad_direct_kernel.  Not faster: a warp per
+// entry with two channels a lane (35 instructions an entry), entries filled up so that none is out of range, the input read with every
+// entry, three entries ahead, packed FMAs.
 // Three blocks a multiprocessor with one entry ahead (80 registers) beat two blocks with two ahead, 1.38 to 1.43 ms; where a group has
 // several slices shared memory allows two blocks, and the field's kernels would spill.
 // kMulti: the offset group has several slices of 64 channels (nh > 1).
