@@ -55,8 +55,12 @@ __global__ void __launch_bounds__(256)
 stage_gy_img_kernel(int Cout, int V, int tiles_per_clip, int b0, int x3, const float* __restrict__ gy,
                     uint8_t* __restrict__ img, long long lo_off, const __grid_constant__ PositionAsk ask) {
   __shared__ float tile[64][129];
-  if (ask.n_recs > 0 && blockIdx.x == 0 && blockIdx.y == 0) ask_positions(ask);
-  const int tile_id = blockIdx.x, kb = blockIdx.y, KB = gridDim.y;
+  const int asks = ask.n_recs > 0;               // then a column of blocks more, of which one asks, beside the others
+  if (asks && blockIdx.x == 0) {
+    if (blockIdx.y == 0) ask_positions(ask);
+    return;
+  }
+  const int tile_id = blockIdx.x - asks, kb = blockIdx.y, KB = gridDim.y;
   const int bl = tile_id / tiles_per_clip, v0 = (tile_id % tiles_per_clip) * kBM;
   const int b = b0 + bl;
   const int nco = x3 == 1 ? 32 : 64;
@@ -661,8 +665,8 @@ int run_bwd(const Geom& g, bool x3, const Coords& coords, unsigned long long cap
     const PositionAsk ask{g, recs + b0 * n_clip_recs, sp.ask ? nbc * n_clip_recs : 0, voxel_order(g), sp.taps, FieldOut, field_ch, axes,
                           direct_word};
     prof_mark(st, "bwd_stage_grad_out");
-    stage_gy_img_kernel<<<dim3((unsigned)n_tiles, (unsigned)pl.KBT), 256, 0, st>>>(g.Cout, g.V, pl.tiles_per_clip, b0,
-                                                                                  img_mode, gy, gy_img, pl.gy_lo_off, ask);
+    stage_gy_img_kernel<<<dim3((unsigned)(n_tiles + (sp.ask ? 1 : 0)), (unsigned)pl.KBT), 256, 0, st>>>(
+        g.Cout, g.V, pl.tiles_per_clip, b0, img_mode, gy, gy_img, pl.gy_lo_off, ask);
     D2C_LAUNCH_CHECK();
     DcolParams p;
     p.gy_img = gy_img; p.wt_img = wt_img; p.dcol = dcol;

@@ -184,9 +184,13 @@ struct SampleGradPlan {
   int taps;                    // of a block
   bool lists, ask;             // may be sample_grad_taps_kernel's; the positions decide
 };
-// Asking costs a call about 3 us (a launch that ends at once and the wait for it): from this many (32 voxels, tap, slice) on, about 300
-// us of kernel.
-constexpr long long kSgAskFrom = 32768;
+// Asking costs a call 1 to 2 us (a launch that ends at once and the wait for it): from this many (32 voxels, tap, slice) on, about 30 us
+// of kernel.  us of forward and backward kernels, not asked / asked (single pass):
+//   offsets of two voxels   64 channels, 4 x 4 x 16 x 16 175 / 174 (155 / 155); 128, 8 x 15 x 27 240 / 242 (207 / 207); 256 in 4 groups
+//                           there 388 / 390 (313 / 316); 128, 8 x 30 x 54 571 / 571 (455 / 456)
+//   all offsets zero        180 / 168 (161 / 150); 233 / 216 (205 / 186); 374 / 352 (310 / 292), in one group 383 / 332 (322 / 264);
+//                           546 / 495 (453 / 403)
+constexpr long long kSgAskFrom = 2048;
 // A block lists and adds up the contributions of 32 voxels; the more taps it has, the more of them meet.  Small volumes share
 // the taps out over up to nine blocks, so that there are three for every multiprocessor, also for the kernels of which two fit on one
 // (256 channels on 8 x 15 x 27: 107 us with three, six or twelve a multiprocessor; 64 channels on 4 x 16 x 16: 17.6 us with nine

@@ -101,23 +101,26 @@ def gradients(dn, ts, geo, gy, g, k=(3, 3, 3), stride=(1, 1, 1), field=None):
     return torch.autograd.grad(y, ts, gy)
 
 
-# lists of contributions or every corner by itself, by what the host knows
+# lists of contributions or every corner by itself, by what the host knows; "both": the positions decide, where it would be lists, from
+# 2048 (32 voxels, tap, slice) on
 ROUTES = [
     ("direct", "auto", dict(cin=64, dims=(4, 16, 16), g=1)),                          # three taps a block
     ("lists", "auto", dict(cin=64, dims=(8, 16, 16), g=1)),                           # four
     ("direct", "bf16", dict(cin=64, dims=(8, 16, 16), g=2)),                          # seven, 32 channels a group
     ("direct", "auto", dict(cin=128, dims=(8, 30, 54), g=2, k=(1, 1, 3))),
-    ("lists", "auto", dict(cin=128, dims=(8, 30, 54), g=2, k=(1, 1, 5))),
+    ("both", "auto", dict(cin=128, dims=(8, 30, 54), g=2, k=(1, 1, 5))),
     ("direct", "bf16", dict(cin=128, dims=(8, 30, 54), g=2, k=(1, 1, 7))),
-    ("lists", "bf16", dict(cin=128, dims=(8, 30, 54), g=2, k=(2, 2, 2))),
+    ("both", "bf16", dict(cin=128, dims=(8, 30, 54), g=2, k=(2, 2, 2))),
     ("direct", "auto", dict(cin=64, dims=(16, 60, 60), g=1, stride=(2, 2, 2))),
-    ("lists", "auto", dict(cin=64, dims=(8, 60, 60), g=1, stride=(1, 2, 2))),
-    ("lists", "auto", dict(cin=128, dims=(16, 60, 60), g=1, stride=(2, 2, 2))),       # two slices
+    ("both", "auto", dict(cin=64, dims=(8, 60, 60), g=1, stride=(1, 2, 2))),
+    ("both", "auto", dict(cin=128, dims=(16, 60, 60), g=1, stride=(2, 2, 2))),        # two slices
     ("direct", "auto", dict(cin=64, dims=(8, 60, 60), g=2, stride=(1, 2, 2))),
     ("direct", "auto", dict(cin=64, dims=(8, 30, 54), g=2, k=(1, 3, 5))),
-    ("lists", "auto", dict(cin=64, dims=(8, 40, 40), g=2)),
+    ("both", "auto", dict(cin=64, dims=(8, 40, 40), g=2)),
     ("direct", "bf16", dict(cin=64, dims=(8, 60, 60), g=2)),                          # 32 channels a group, fp16
-    ("both", "auto", dict(cin=64, dims=(8, 60, 107), g=1)),                           # the positions decide
+    ("lists", "bf16", dict(cin=64, dims=(8, 15, 20), g=1)),                           # 75 x 27
+    ("both", "bf16", dict(cin=64, dims=(8, 19, 16), g=1)),                            # 76 x 27
+    ("both", "auto", dict(cin=64, dims=(8, 60, 107), g=1)),
 ]
 
 
@@ -159,7 +162,8 @@ POSITIONS = {"zero": (0, 0, 0), "whole frames": (0, 2, 0), "ordinary": (2, 2, 0)
 
 
 @pytest.mark.parametrize("mode", REL)
-@pytest.mark.parametrize("cin,g,dims", [(64, 1, (8, 60, 107)), (128, 1, (8, 48, 64)), (64, 2, (8, 60, 107))])
+@pytest.mark.parametrize("cin,g,dims", [(64, 1, (8, 60, 107)), (128, 1, (8, 48, 64)), (64, 2, (8, 60, 107)), (256, 4, (7, 9, 13)),
+                                        (64, 1, (5, 23, 29))])
 @pytest.mark.parametrize("name", POSITIONS)
 def test_asked(dn, mode, cin, g, dims, name):
     import d2conv3d_b200
